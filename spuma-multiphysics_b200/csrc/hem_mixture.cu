@@ -1,6 +1,8 @@
 // Multi-species HEM UV flash on the device: a Peng-Robinson gas mixture of up
 // to four species with up to two pure condensed liquids (the air / N2O /
-// isopropanol model of the reference's production case), one thread per cell.
+// isopropanol model of the reference's production case). The independent
+// evaluations of a cell's search (the two sides of every Jacobian column, a line
+// search's trial fractions, the seeds) run on different lanes of a warp.
 //
 // The search restates the reference device flash
 // (src/reactiveThermo/reactiveDeviceFlash.h) for models without solids, with its
@@ -329,58 +331,10 @@ __device__ __noinline__ bool scalarGas(MixCell& c, MixEval& result) {
     return result.s.volumeResidual <= m.vtol && result.s.energyResidual <= m.etol;
 }
 
-// A frozen partition (fixed liquid masses): Newton in (ln p, ln T) with the
-// (0.7, 0.2) limiter and a halving line search; stallLimit > 0 ends the solve as
-// a failure after that many consecutive steps accepted below a fraction of 1/32.
-__device__ __noinline__ bool frozen(MixCell& c, const double* mass, MixEval& value, int stallLimit) {
-    const ReactiveB200HemModel& m = c.m;
-    if (!fin(c.energy)) return false;
-    if (m.scalarRecovery && mass[0] == 0 && mass[1] == 0 && scalarGas(c, value)) return true;
-    double p = clampd(c.guess.p, m.pmin, m.pmax), T = clampd(c.guess.T, m.Tmin, m.Tmax);
-    if (!evaluate(c, mass, p, T, value, false, nullptr)) return false;
-    int stalled = 0;
-    for (int it = 0; it < 70; ++it) {
-        const double scale = energyScale(value), rv = value.volume - 1, re = (value.energy - c.energy) / scale;
-        value.s.volumeResidual = fabs(rv);
-        value.s.energyResidual = fabs(re);
-        value.s.iterations = it;
-        if (fabs(rv) <= m.vtol && fabs(re) <= m.etol) return true;
-        double jac[4][4] = {}, rhs[4] = {-rv, -re, 0, 0}, step[4] = {};
-        jac[0][0] = value.Vp * p; jac[0][1] = value.VT * T;
-        jac[1][0] = value.Ep * p / scale; jac[1][1] = value.ET * T / scale;
-        if (!solveDense(jac, rhs, 2, step)) return false;
-        const double limit = fmax(1., fmax(fabs(step[0]) / .7, fabs(step[1]) / .2));
-        step[0] /= limit;
-        step[1] /= limit;
-        const double previous = fmax(fabs(rv), fabs(re));
-        bool accepted = false;
-        for (double fraction = 1; fraction > 1e-9; fraction *= .5) {
-            const double pp = p * exp(fraction * step[0]), tt = T * exp(fraction * step[1]);
-            MixEval trial;
-            if (evaluate(c, mass, pp, tt, trial, false, nullptr)) {
-                const double next = fmax(fabs(trial.volume - 1), fabs(trial.energy - c.energy) / scale);
-                if (next < previous * (1 - 1e-4 * fraction) || next < fmin(m.vtol, m.etol)) {
-                    value = trial;
-                    p = pp;
-                    T = tt;
-                    accepted = true;
-                    stalled = fraction < 1. / 32 ? stalled + 1 : 0;
-                    break;
-                }
-            }
-        }
-        if (!accepted) return false;
-        if (stallLimit > 0 && stalled >= stallLimit
-            && !(fabs(value.volume - 1) <= m.vtol && fabs(value.energy - c.energy) / energyScale(value) <= m.etol))
-            return false;
-    }
-    return false;
-}
-
 // Residual of an active set at x = (ln p, ln T, fractions): liquid fractions in
 // [0, 1) or, in the boundary recovery, log vapour fractions <= 0.
 __device__ __noinline__ bool activeResidual(MixCell& c, const int* active, int n, const double* x, double scale,
-                                            double* f, MixEval* out) {
+                                            double* f, MixEval& v) {
     ++c.n.residuals;
     const ReactiveB200HemModel& m = c.m;
     double mass[kLiq] = {0, 0}, vapor[kLiq] = {0, 0};
@@ -398,7 +352,6 @@ __device__ __noinline__ bool activeResidual(MixCell& c, const int* active, int n
             mass[i] = x[j + 2] * q;
         }
     }
-    MixEval v;
     if (!evaluate(c, mass, exp(x[0]), exp(x[1]), v, true, c.adaptive ? vapor : nullptr) || !(v.s.gasMass > 0))
         return false;
     f[0] = v.volume - 1;
@@ -407,154 +360,11 @@ __device__ __noinline__ bool activeResidual(MixCell& c, const int* active, int n
         f[2 + j] = v.muLiq[active[j]] - v.muGas[active[j]];
         if (!fin(f[2 + j])) return false;
     }
-    if (out) *out = v;
-    return true;
-}
-
-// Bounded central differences (h = 2e-6 in ln p and ln T, 2e-5 in the
-// fractions, halved up to 12 times when neither side evaluates; one-sided when
-// only one does; the boundary recovery's coordinates step at least one ulp and
-// weight the two sides by their actual steps).
-__device__ __noinline__ bool jacobianFD(MixCell& c, const int* active, int n, const double* x, double scale,
-                                        const double* f, double jac[4][4]) {
-    ++c.n.fd;
-    const int size = n + 2;
-    for (int j = 0; j < size; ++j) {
-        double h = j < 2 ? 2e-6 : 2e-5;
-        bool success = false;
-        for (int attempt = 0; attempt < 12 && !success; ++attempt, h *= .5) {
-            double xp[4] = {}, xm[4] = {}, fp[4] = {}, fm[4] = {};
-            for (int i = 0; i < size; ++i) xp[i] = xm[i] = x[i];
-            xp[j] += h;
-            xm[j] -= h;
-            if (c.adaptive) {
-                if (xp[j] == x[j]) xp[j] = nextafter(x[j], HUGE_VAL);
-                if (xm[j] == x[j]) xm[j] = nextafter(x[j], -HUGE_VAL);
-            }
-            const bool plus = activeResidual(c, active, n, xp, scale, fp, nullptr);
-            const bool minus = activeResidual(c, active, n, xm, scale, fm, nullptr);
-            if (!plus && !minus) continue;
-            const double hp = xp[j] - x[j], hm = x[j] - xm[j];
-            double maximum = 0;
-            success = true;
-            for (int i = 0; i < size; ++i) {
-                double d;
-                if (c.adaptive)
-                    d = plus && minus ? (hm / (hp + hm)) * ((fp[i] - f[i]) / hp) + (hp / (hp + hm)) * ((f[i] - fm[i]) / hm)
-                                      : plus ? (fp[i] - f[i]) / hp : (f[i] - fm[i]) / hm;
-                else
-                    d = plus && minus ? (fp[i] - fm[i]) / (2 * h) : plus ? (fp[i] - f[i]) / h : (f[i] - fm[i]) / h;
-                jac[i][j] = d;
-                maximum = fmax(maximum, fabs(d));
-                success = success && fin(d);
-            }
-            if (c.adaptive) success = success && maximum > 0;
-        }
-        if (!success) return false;
-    }
     return true;
 }
 
 __device__ __forceinline__ bool rejectedCoordinate(bool adaptive, double y) {
     return adaptive ? (!fin(y) || y > 0) : !(y >= 0 && y < 1);
-}
-
-// Newton on an active set of liquids from a fraction seed (seed < 0: the seed
-// state's liquid fraction; -3 in the boundary recovery: a vapour fraction from
-// the non-condensable inventory); secondSeed (when not -2) seeds the second
-// liquid; restart (optional) replaces the seed state.
-__device__ __noinline__ bool activeFlash(MixCell& c, const int* active, int n, double seed, MixEval& value,
-                                         double secondSeed, const ReactiveThermoState* restart) {
-    ++c.n.candidates;
-    const ReactiveB200HemModel& m = c.m;
-    const int size = n + 2;
-    const double rho = density(c);
-    const ReactiveThermoState& g = restart ? *restart : c.guess;
-    const double scale = fmax(1e5 * rho, fmax(fabs(c.energy), rho * 2000 * fmax(g.T, m.Tmin)));
-    double x[4] = {log(clampd(g.p, m.pmin, m.pmax)), log(clampd(g.T, m.Tmin, m.Tmax)), 0, 0};
-    for (int j = 0; j < n; ++j) {
-        const int i = active[j];
-        const double selected = j == 1 && secondSeed != -2 ? secondSeed : seed;
-        const double previous = g.liquidMass[i] / c.q[m.condensable[i]];
-        x[j + 2] = selected < 0 ? clampd(previous, 1e-8, 1 - 1e-8) : selected;
-        if (c.adaptive) {
-            double vapor = selected < 0 ? 1 - previous : 1 - selected;
-            if (selected == -3 || (selected < 0 && vapor < 1e-6)) {
-                double other = 0;
-                for (int k = 0; k < m.ns; ++k) {
-                    bool chosen = false;
-                    for (int a = 0; a < n; ++a) chosen |= k == m.condensable[active[a]];
-                    if (!chosen) other += c.q[k];
-                }
-                vapor = other > 0 ? fmin(1e-6, .01 * (other / c.q[m.condensable[i]])) : 1e-8;
-            }
-            if (!(vapor > 0 && fin(vapor))) return false;
-            x[j + 2] = log(fmin(1., vapor));
-        }
-    }
-    double f[4] = {};
-    if (!activeResidual(c, active, n, x, scale, f, &value)) return false;
-    for (int it = 0; it < 90; ++it) {
-        const double chemical = maxAbs(f + 2, n);
-        double jac[4][4] = {};
-        if (fabs(f[0]) <= m.vtol && fabs(f[1]) <= m.etol && chemical <= m.mutol) {
-            value.s.volumeResidual = fabs(f[0]);
-            value.s.energyResidual = fabs(f[1]);
-            value.s.chemicalResidual = chemical;
-            value.s.iterations = it;
-            if (!jacobianFD(c, active, n, x, scale, f, jac)) return false;
-            const double rhs[4] = {-1 / rho, value.s.p / (rho * scale), 0, 0};
-            double response[4] = {};
-            if (!solveDense(jac, rhs, size, response)) return false;
-            const double squared = value.s.p * response[0];
-            if (!fin(squared) || squared <= 0) return false;
-            value.s.soundEquilibrium = sqrt(squared);
-            return value.s.soundEquilibrium <= value.s.soundFrozen * (1 + 2e-3);
-        }
-        if (!jacobianFD(c, active, n, x, scale, f, jac)) return false;
-        double rhs[4] = {}, step[4] = {};
-        for (int j = 0; j < size; ++j) rhs[j] = -f[j];
-        if (!solveDense(jac, rhs, size, step)) return false;
-        double limiter = fmax(1., fmax(fabs(step[0]) / .7, fabs(step[1]) / .18));
-        for (int j = 2; j < size; ++j) limiter = fmax(limiter, fabs(step[j]) / (c.adaptive ? 2. : .3));
-        for (int j = 0; j < size; ++j) step[j] /= limiter;
-        bool accepted = false;
-        const double previous = maxAbs(f, size);
-        double fraction = 1;
-        for (int k = 0; k < 30; ++k, fraction *= .5) {
-            double tx[4] = {}, tf[4] = {};
-            for (int j = 0; j < size; ++j) tx[j] = x[j] + fraction * step[j];
-            bool rejected = false;
-            for (int j = 0; j < n; ++j) rejected |= rejectedCoordinate(c.adaptive, tx[j + 2]);
-            if (rejected) {
-                // the rejected fractions form a prefix (each coordinate moves back
-                // toward the valid x as the fraction halves): its end by bisection
-                // on the same expression and predicate, 30 standing for none
-                int lower = k, upper = 30;
-                while (upper - lower > 1) {
-                    const int mid = (lower + upper) / 2;
-                    const double fm = ldexp(1.0, -mid);
-                    bool bad = false;
-                    for (int j = 0; j < n; ++j) bad |= rejectedCoordinate(c.adaptive, x[j + 2] + fm * step[j + 2]);
-                    if (bad) lower = mid; else upper = mid;
-                }
-                c.n.residuals += unsigned(upper - k);
-                if (upper == 30) break;
-                k = upper;
-                fraction = ldexp(1.0, -upper);
-                for (int j = 0; j < size; ++j) tx[j] = x[j] + fraction * step[j];
-            }
-            MixEval trial;
-            if (activeResidual(c, active, n, tx, scale, tf, &trial) && maxAbs(tf, size) < previous * (1 - 1e-4 * fraction)) {
-                for (int j = 0; j < size; ++j) { x[j] = tx[j]; f[j] = tf[j]; }
-                value = trial;
-                accepted = true;
-                break;
-            }
-        }
-        if (!accepted) return false;
-    }
-    return false;
 }
 
 // Gibbs energy of the gas mixture of the present liquids' species at mole
@@ -622,135 +432,57 @@ __device__ __noinline__ bool stableCandidate(MixCell& c, const MixEval& v) {
     return best >= -m.mutol;
 }
 
-// A converged candidate enters the selection when stable; the first maximum of
-// the entropy density wins. Returns whether it was stable.
-__device__ bool consider(MixCell& c, const MixEval& cand, MixEval& best, bool& have) {
-    if (!stableCandidate(c, cand)) { ++c.n.failures; return false; }
-    ++c.n.stable;
-    if (!have || cand.entropyD > best.entropyD) { best = cand; have = true; }
-    return true;
-}
-
-__device__ __noinline__ bool temperatureSearch(MixCell& c, MixEval& best) {
-    const ReactiveB200HemModel& m = c.m;
-    constexpr double seeds[5] = {-1, .5, .95, .1, .9999};
-    constexpr double fractions[4] = {.02, .25, .5, .75};
-    bool have = false;
-    MixEval cand;
-    for (int mask = 1; mask < (1 << m.nl); ++mask) {
-        int active[kLiq] = {0, 0}, n = 0;
-        bool possible = true;
-        double lower = m.Tmin, upper = m.Tmax;
-        for (int i = 0; i < m.nl; ++i)
-            if (mask & (1 << i)) {
-                if (c.q[m.condensable[i]] <= 0) possible = false;
-                else {
-                    active[n++] = i;
-                    lower = fmax(lower, m.liquidTmin[i]);
-                    upper = fmin(upper, m.liquidTc[i] * (1 - 1e-10));
-                }
-            }
-        if (!possible || !(upper > lower)) continue;
-        for (int t = 0; t < 4; ++t) {
-            ReactiveThermoState restart = c.guess;
-            restart.T = lower + (upper - lower) * fractions[t];
-            for (int j = 0; j < 5; ++j) {
-                if (activeFlash(c, active, n, seeds[j], cand, -2, &restart)) consider(c, cand, best, have);
-                else ++c.n.failures;
-            }
-        }
-    }
-    return have;
-}
-
 __device__ __forceinline__ bool prunable(const ReactiveB200HemModel& m) {
     return m.nl == 1 && m.condensedKind[0] == 0 && m.condensedKind[1] == 0;
 }
 
-__device__ __noinline__ bool searchCandidates(MixCell& c, MixEval& best) {
-    const ReactiveB200HemModel& m = c.m;
-    constexpr double seeds[5] = {-1, .5, .95, .1, .9999};
-    constexpr double pairs[4] = {.1, .5, .95, .9999};
-    bool have = false, gasStable = false;
-    MixEval cand;
-    double mass[kLiq] = {0, 0};
-    const bool fastGas = m.stableGasPrune && prunable(m) && !c.adaptive;
-    if (frozen(c, mass, cand, fastGas ? 4 : 0)) gasStable = consider(c, cand, best, have) && cand.s.gasMass > 0;
-    else ++c.n.failures;
-    const bool prune = m.stableGasPrune && prunable(m) && gasStable && !c.adaptive;
-    double other = 0;
-    for (int k = 0; k < m.ns; ++k)
-        if (!isCondensable(m, k)) other += c.q[k];
-    if (other == 0 && m.nl) {
-        for (int i = 0; i < m.nl; ++i) mass[i] = c.q[m.condensable[i]];
-        if (frozen(c, mass, cand, 0)) consider(c, cand, best, have);
-        else ++c.n.failures;
-    }
-    for (int mask = 1; !prune && mask < (1 << m.nl); ++mask) {
-        int active[kLiq] = {0, 0}, n = 0;
-        bool possible = true;
-        for (int i = 0; i < m.nl; ++i)
-            if (mask & (1 << i)) {
-                if (c.q[m.condensable[i]] <= 0) possible = false;
-                else active[n++] = i;
-            }
-        if (!possible) continue;
-        for (int j = 0; j < 5; ++j) {
-            if (activeFlash(c, active, n, seeds[j], cand, -2, nullptr)) consider(c, cand, best, have);
-            else ++c.n.failures;
-        }
-        if (c.adaptive) {
-            if (activeFlash(c, active, n, -3, cand, -2, nullptr)) consider(c, cand, best, have);
-            else ++c.n.failures;
-        }
-        if (c.adaptive && n == 2)
-            for (int first = 1; first < 5; ++first)
-                for (int second = 1; second < 5; ++second) {
-                    if (first == second) continue;
-                    if (activeFlash(c, active, n, pairs[first - 1], cand, pairs[second - 1], nullptr))
-                        consider(c, cand, best, have);
-                    else ++c.n.failures;
-                }
-    }
-    // restart temperatures only when the search found no stable candidate
-    if (!have) have = temperatureSearch(c, best);
-    return have;
-}
+// A candidate of the search: its state, entropy density and status (kInvalid: the
+// cell's inputs are rejected; kNone: not converged).
+enum : int { kInvalid = -1, kNone = 0, kUnstable = 1, kStable = 2 };
+struct MixRecord {
+    ReactiveThermoState s;
+    double entropyD;
+    int status, pad;
+};
 
-// The recovery of one cell: the candidate search; with the boundary recovery (or
-// in a capillary batch, whose transported trace inventories can defeat the
-// reference seeds) a second search in log vapour fractions when the first found
-// nothing or left a condensable almost entirely liquid beside a gas phase, the
-// larger entropy (the first search on a tie) kept.
-__device__ bool recoverCell(MixCell& c, MixEval& result, bool capillaryBoundary) {
-    const ReactiveB200HemModel& m = c.m;
-    if (m.ns <= 0 || m.ns > kNs || m.nl < 0 || m.nl > kLiq || !fin(c.energy) || !(density(c) > 0)) return false;
-    for (int k = 0; k < m.ns; ++k)
-        if (!fin(c.q[k]) || c.q[k] < 0) return false;
-    MixEval reference;
-    const bool have = searchCandidates(c, reference);
-    if (!m.boundaryRecovery && !capillaryBoundary) {
-        if (have) result = reference;
-        return have;
-    }
-    if (have) {
-        bool boundary = false;
-        for (int i = 0; i < m.nl; ++i) {
-            const double q = c.q[m.condensable[i]];
-            if (q > 0 && reference.s.gasMass > 0) boundary |= reference.s.liquidMass[i] / q > 1 - 1e-4;
-        }
-        if (!boundary) { result = reference; return true; }
-    }
-    c.adaptive = true;
-    MixEval recovered;
-    const bool found = searchCandidates(c, recovered);
-    c.adaptive = false;
-    if (!found && !have) return false;
-    result = have && (!found || reference.entropyD >= recovered.entropyD) ? reference : recovered;
-    return true;
-}
+// Per-cell fixed-partition candidates, in the order they enter the selection: the
+// all-gas one, the all-liquid one (cells without non-condensable gas) and, for
+// models with stableGasPrune, the all-gas one without that policy's stall limit,
+// which the boundary recovery's second search takes.
+enum : int { kGasRecord = 0, kLiquidRecord = 1, kFullGasRecord = 2, kRecordKinds = 3 };
+
+// One batch's device arrays. `order` (optional) names the cells: item i works on
+// cell order[i], and every per-cell input is indexed by that cell; the records,
+// the work list and its counters belong to the handle and are indexed by item.
+struct MixBatch {
+    const ReactiveB200HemModel* model;
+    const double* q;
+    const double* energy;
+    size_t count;
+    const ReactiveThermoState* seed;
+    const ReactiveGpuHemCapillaryInputV2* capillary;
+    const uint32_t* order;
+    MixRecord* record[kRecordKinds];  // kFullGasRecord: null unless the model prunes
+    unsigned* list;                   // Newton items: item * kRecordKinds + kind
+    unsigned* counters;               // C_*
+    unsigned long long* totals;
+    ReactiveThermoState* out;
+    int* success;
+    ReactiveGpuHemOutputV1* outputs;
+};
+enum : int { C_LISTED, C_NEWTON, C_SEARCH, C_COUNT };
 
 enum : int { M_PHASES, M_RESIDUALS, M_CANDIDATES, M_STABLE, M_FD, M_SUCCEEDED, M_COUNT };
+
+__device__ __forceinline__ void flushTally(const Tally& n, unsigned long long* totals) {
+    const unsigned long long v[5] = {n.phases, n.residuals, n.candidates, n.stable, n.fd};
+    const int slot[5] = {M_PHASES, M_RESIDUALS, M_CANDIDATES, M_STABLE, M_FD};
+    for (int i = 0; i < 5; ++i) {
+        unsigned long long x = v[i];
+        for (int o = 16; o; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        if ((threadIdx.x & 31) == 0 && x) atomicAdd(totals + slot[i], x);
+    }
+}
 
 // A capillary cell input the reference's recoverCapillary accepts
 // (src/reactiveThermo/reactiveDeviceFlash.h:572-588): a color in [0, 1], a
@@ -759,55 +491,584 @@ __device__ __forceinline__ bool capillaryAccepted(const ReactiveB200HemModel& m,
     return fin(color) && color >= 0 && color <= 1 && fin(jump) && (jump == 0 || (m.nl == 1 && m.condensedKind[0] == 0));
 }
 
-// One thread per cell. `order` (optional) names the cells: thread item i works on
-// cell order[i], and every per-cell array is indexed by that cell. With
-// `capillary` each cell is the reference's capillary recovery: UV equilibrium
-// with the boundary search, or (equilibrium = 0) the frozen partition at the
-// seed's liquid masses. Results go to out/success, or to outputs[cell] for the
-// resident form; a failed cell gets its seed.
-__global__ void __launch_bounds__(kBlock) mixtureFlashKernel(const ReactiveB200HemModel* __restrict__ model,
-                                                            const double* __restrict__ q,
-                                                            const double* __restrict__ energy, size_t count,
-                                                            const ReactiveThermoState* __restrict__ seed,
-                                                            const ReactiveGpuHemCapillaryInputV2* capillary,
-                                                            const uint32_t* order, ReactiveThermoState* out,
-                                                            int* success, ReactiveGpuHemOutputV1* outputs,
-                                                            unsigned long long* totals) {
-    const ReactiveB200HemModel& m = *model;
+__device__ __forceinline__ void loadCell(const MixBatch& b, size_t item, MixCell& c) {
+    const size_t cell = b.order ? size_t(b.order[item]) : item;
+    for (int k = 0; k < kNs; ++k) c.q[k] = k < c.m.ns ? b.q[cell * size_t(c.m.ns) + k] : 0.0;
+    c.energy = b.energy[cell];
+    c.guess = b.seed[cell];
+    c.color = b.capillary ? b.capillary[cell].color : 0.0;
+    c.jump = b.capillary ? b.capillary[cell].pressureJump : 0.0;
+    c.adaptive = false;
+}
+// A capillary item with the partition frozen at the seed's liquid masses.
+__device__ __forceinline__ bool frozenItem(const MixBatch& b, size_t item) {
+    return b.capillary && !b.capillary[b.order ? size_t(b.order[item]) : item].equilibrium;
+}
+
+__device__ __forceinline__ void storeRecord(MixRecord& r, const MixEval& v, int status) {
+    r.s = v.s;
+    r.entropyD = v.entropyD;
+    r.status = status;
+}
+
+// The fixed-partition candidates' first part, one thread per item: the input
+// checks, the scalar all-gas solve with its stability test, and the list of the
+// partitions that need the (ln p, ln T) Newton.
+__global__ void __launch_bounds__(kBlock) mixtureScalar(MixBatch b) {
+    const ReactiveB200HemModel& m = *b.model;
+    Tally n;
+    for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < b.count; i += size_t(blockDim.x) * gridDim.x) {
+        MixCell c{m, {0, 0, 0, 0}, 0.0, ReactiveThermoState{}, false, n};
+        loadCell(b, i, c);
+        const bool frozen = frozenItem(b, i);
+        bool valid = !b.capillary || capillaryAccepted(m, c.color, c.jump);
+        if (valid && !frozen) {
+            valid = m.ns > 0 && m.ns <= kNs && m.nl >= 0 && m.nl <= kLiq && fin(c.energy) && density(c) > 0;
+            for (int k = 0; k < m.ns && valid; ++k) valid = fin(c.q[k]) && c.q[k] >= 0;
+        }
+        b.record[kLiquidRecord][i].status = kNone;
+        if (b.record[kFullGasRecord]) b.record[kFullGasRecord][i].status = kNone;
+        MixRecord& gas = b.record[kGasRecord][i];
+        gas.status = valid ? kNone : kInvalid;
+        if (!valid || !fin(c.energy)) continue;
+        const double mass0 = frozen ? c.guess.liquidMass[0] : 0.0, mass1 = frozen ? c.guess.liquidMass[1] : 0.0;
+        MixEval v;
+        if (m.scalarRecovery && mass0 == 0 && mass1 == 0 && scalarGas(c, v)) {
+            const int status = frozen || stableCandidate(c, v) ? kStable : kUnstable;
+            storeRecord(gas, v, status);
+            if (b.record[kFullGasRecord]) storeRecord(b.record[kFullGasRecord][i], v, status);
+        } else {
+            b.list[atomicAdd(b.counters + C_LISTED, 1u)] = unsigned(i) * kRecordKinds + kGasRecord;
+            if (!frozen && b.record[kFullGasRecord])
+                b.list[atomicAdd(b.counters + C_LISTED, 1u)] = unsigned(i) * kRecordKinds + kFullGasRecord;
+        }
+        if (!frozen && m.nl) {
+            double other = 0;
+            for (int k = 0; k < m.ns; ++k)
+                if (!isCondensable(m, k)) other += c.q[k];
+            if (other == 0) b.list[atomicAdd(b.counters + C_LISTED, 1u)] = unsigned(i) * kRecordKinds + kLiquidRecord;
+        }
+    }
+    __syncwarp();
+    flushTally(n, b.totals);
+}
+
+// The frozen partitions (fixed liquid masses) the scalar solve left: Newton in
+// (ln p, ln T) with the (0.7, 0.2) limiter and a halving line search; a stall limit
+// ends the solve as a failure after that many consecutive steps accepted below a
+// fraction of 1/32.
+//
+// Eight lanes per item: they evaluate eight consecutive fractions of a line search
+// at once and the first acceptable one is taken, the fraction a serial search
+// stops at. A partition that has no solution (a cold cell's all-gas one) halves
+// deep in most of its 70 steps; serially one such cell's chain of evaluations,
+// each of a few thousand dependent FP64 instructions, outlasted the batch.
+constexpr int kNewtonLanes = 8;
+constexpr int kSearchBlock = 128;
+constexpr int kTrials = 30;  // fractions 1 .. 2^-29
+
+__global__ void __launch_bounds__(kSearchBlock) mixtureNewton(MixBatch b) {
+    const ReactiveB200HemModel& m = *b.model;
+    const unsigned lane = threadIdx.x & 31u;
+    const int base = int(lane) / kNewtonLanes * kNewtonLanes, r = int(lane) - base;
+    const unsigned group = ((1u << kNewtonLanes) - 1u) << base;
+    const unsigned total = b.counters[C_LISTED];
+    Tally n;
+    MixCell c{m, {0, 0, 0, 0}, 0.0, ReactiveThermoState{}, false, n};
+    MixEval v;
+    MixRecord* record = nullptr;
+    double mass[kLiq] = {0, 0};
+    bool active = false, exhausted = false, first = false, frozen = false;
+    int stallLimit = 0, stalled = 0, it = 0, k = 0;
+    double p = 0, T = 0, s0 = 0, s1 = 0, previous = 0, scale = 0;
+    for (;;) {
+        if (!active && !exhausted) {
+            unsigned slot = 0;
+            if (r == 0) slot = atomicAdd(b.counters + C_NEWTON, 1u);
+            slot = __shfl_sync(group, slot, base);
+            if (slot < total) {
+                const unsigned entry = b.list[slot], item = entry / kRecordKinds;
+                const int kind = int(entry % kRecordKinds);
+                loadCell(b, item, c);
+                frozen = frozenItem(b, item);
+                record = b.record[kind] + item;
+                for (int i = 0; i < kLiq; ++i)
+                    mass[i] = frozen ? c.guess.liquidMass[i]
+                                     : (kind == kLiquidRecord && i < m.nl ? c.q[m.condensable[i]] : 0.0);
+                stallLimit = !frozen && kind == kGasRecord && m.stableGasPrune && prunable(m) ? 4 : 0;
+                p = clampd(c.guess.p, m.pmin, m.pmax);
+                T = clampd(c.guess.T, m.Tmin, m.Tmax);
+                active = first = true;
+                stalled = it = k = 0;
+            } else exhausted = true;
+        }
+        __syncwarp();
+        if (__all_sync(0xffffffffu, !active)) break;
+        // every lane's evaluation at one call site
+        double pe = p, te = T, fraction = 1;
+        bool point = active && (first ? r == 0 : k + r < kTrials);
+        if (active && !first) {
+            fraction = ldexp(1.0, -(k + r));
+            pe = p * exp(fraction * s0);
+            te = T * exp(fraction * s1);
+        }
+        bool ok = false;
+        if (point) ok = evaluate(c, mass, pe, te, v, false, nullptr);
+        __syncwarp();
+        if (!active) continue;
+        if (!first && ok) {
+            const double next = fmax(fabs(v.volume - 1), fabs(v.energy - c.energy) / scale);
+            ok = next < previous * (1 - 1e-4 * fraction) || next < fmin(m.vtol, m.etol);
+        }
+        const unsigned accepted = __ballot_sync(group, ok);
+        if (!accepted) {
+            k += kNewtonLanes;
+            if (first || k >= kTrials) active = false;  // the record stays kNone
+            continue;
+        }
+        const int owner = __ffs(accepted) - 1;
+        if (!first) {
+            p = __shfl_sync(group, pe, owner);
+            T = __shfl_sync(group, te, owner);
+            stalled = k + owner - base > 5 ? stalled + 1 : 0;
+            ++it;
+        }
+        // the owner of the accepted evaluation forms the next step
+        int code = 0;  // 1 converged, -1 failed
+        if (int(lane) == owner) {
+            scale = energyScale(v);
+            const double rv = v.volume - 1, re = (v.energy - c.energy) / scale;
+            const bool within = fabs(rv) <= m.vtol && fabs(re) <= m.etol;
+            if (stallLimit > 0 && stalled >= stallLimit
+                && !(fabs(rv) <= m.vtol && fabs(v.energy - c.energy) / scale <= m.etol))
+                code = -1;
+            else if (it >= 70) code = -1;
+            else if (within) {
+                v.s.volumeResidual = fabs(rv);
+                v.s.energyResidual = fabs(re);
+                v.s.iterations = it;
+                const int status = frozen || stableCandidate(c, v) ? kStable : kUnstable;
+                storeRecord(*record, v, status);
+                code = 1;
+            } else {
+                double jac[4][4] = {}, rhs[4] = {-rv, -re, 0, 0}, step[4] = {};
+                jac[0][0] = v.Vp * p; jac[0][1] = v.VT * T;
+                jac[1][0] = v.Ep * p / scale; jac[1][1] = v.ET * T / scale;
+                if (!solveDense(jac, rhs, 2, step)) code = -1;
+                const double limit = fmax(1., fmax(fabs(step[0]) / .7, fabs(step[1]) / .2));
+                s0 = step[0] / limit;
+                s1 = step[1] / limit;
+                previous = fmax(fabs(rv), fabs(re));
+            }
+        }
+        code = __shfl_sync(group, code, owner);
+        scale = __shfl_sync(group, scale, owner);
+        s0 = __shfl_sync(group, s0, owner);
+        s1 = __shfl_sync(group, s1, owner);
+        previous = __shfl_sync(group, previous, owner);
+        first = false;
+        k = 0;
+        if (code) active = false;
+    }
+    flushTally(n, b.totals);
+}
+
+// The Newton candidates of one search: the active set, the fraction seed (< 0: the
+// seed state's liquid fraction; -3 in the boundary recovery: a vapour fraction
+// from the non-condensable inventory), the second liquid's seed (-2: the first's)
+// and, in the restart search, the restart temperature (< 0: the seed state's).
+struct MixTask {
+    int active[kLiq], n;
+    double seed, second, restartT;
+};
+
+// Task `index` of the search's task list in its selection order, false past its end:
+// per active set (liquids present) the five seeds, in the boundary recovery the
+// sixth and, with two liquids, their twelve unequal pairs; in the restart search
+// the five seeds at each restart temperature of the set's legal interval.
+__device__ bool nthTask(const MixCell& c, bool restarts, int index, MixTask& t) {
+    const ReactiveB200HemModel& m = c.m;
+    constexpr double seeds[5] = {-1, .5, .95, .1, .9999};
+    constexpr double pairs[4] = {.1, .5, .95, .9999};
+    constexpr double fractions[4] = {.02, .25, .5, .75};
+    for (int mask = 1; mask < (1 << m.nl); ++mask) {
+        bool possible = true;
+        double lower = m.Tmin, upper = m.Tmax;
+        t.n = 0;
+        t.active[0] = t.active[1] = 0;
+        for (int i = 0; i < m.nl; ++i)
+            if (mask & (1 << i)) {
+                if (c.q[m.condensable[i]] <= 0) possible = false;
+                else {
+                    t.active[t.n++] = i;
+                    lower = fmax(lower, m.liquidTmin[i]);
+                    upper = fmin(upper, m.liquidTc[i] * (1 - 1e-10));
+                }
+            }
+        if (!possible || (restarts && !(upper > lower))) continue;
+        const int tasks = restarts ? 20 : 5 + (c.adaptive ? (t.n == 2 ? 13 : 1) : 0);
+        if (index >= tasks) {
+            index -= tasks;
+            continue;
+        }
+        t.second = -2;
+        t.restartT = restarts ? lower + (upper - lower) * fractions[index / 5] : -1.0;
+        if (restarts) t.seed = seeds[index % 5];
+        else if (index < 5) t.seed = seeds[index];
+        else if (index == 5) t.seed = -3;
+        else {
+            const int a = (index - 6) / 3, o = (index - 6) % 3;
+            t.seed = pairs[a];
+            t.second = pairs[o < a ? o : o + 1];
+        }
+        return true;
+    }
+    return false;
+}
+
+// The Newton start of a task, false when it has none.
+__device__ bool taskStart(const MixCell& c, const MixTask& t, double* x, double& scale) {
+    const ReactiveB200HemModel& m = c.m;
+    const double rho = density(c), gT = t.restartT >= 0 ? t.restartT : c.guess.T;
+    scale = fmax(1e5 * rho, fmax(fabs(c.energy), rho * 2000 * fmax(gT, m.Tmin)));
+    x[0] = log(clampd(c.guess.p, m.pmin, m.pmax));
+    x[1] = log(clampd(gT, m.Tmin, m.Tmax));
+    x[2] = x[3] = 0;
+    for (int j = 0; j < t.n; ++j) {
+        const int i = t.active[j];
+        const double selected = j == 1 && t.second != -2 ? t.second : t.seed;
+        const double previous = c.guess.liquidMass[i] / c.q[m.condensable[i]];
+        x[j + 2] = selected < 0 ? clampd(previous, 1e-8, 1 - 1e-8) : selected;
+        if (c.adaptive) {
+            double vapor = selected < 0 ? 1 - previous : 1 - selected;
+            if (selected == -3 || (selected < 0 && vapor < 1e-6)) {
+                double other = 0;
+                for (int k = 0; k < m.ns; ++k) {
+                    bool chosen = false;
+                    for (int a = 0; a < t.n; ++a) chosen |= k == m.condensable[t.active[a]];
+                    if (!chosen) other += c.q[k];
+                }
+                vapor = other > 0 ? fmin(1e-6, .01 * (other / c.q[m.condensable[i]])) : 1e-8;
+            }
+            if (!(vapor > 0 && fin(vapor))) return false;
+            x[j + 2] = log(fmin(1., vapor));
+        }
+    }
+    return true;
+}
+
+// The best stable candidate so far: the largest entropy density, the earliest in
+// selection order on a tie (the first maximum, whatever order candidates finish in).
+struct MixBest {
+    bool have;
+    double entropy;
+    int order;
+    __device__ bool takes(double e, int o) const { return !have || e > entropy || (e == entropy && o < order); }
+};
+
+// The tasks of one search over a warp. Groups of `width` lanes (two per Newton
+// unknown: five groups of six with one liquid, four of eight with two) each run
+// one task at a time and take the next when it ends; per round every lane makes
+// at most one evaluation, all at one call site: the start, the two sides of every
+// Jacobian column (bounded central differences: h = 2e-6 in ln p and ln T, 2e-5 in
+// the fractions, halved up to 12 times when neither side evaluates, one-sided when
+// only one does; the boundary recovery's coordinates step at least one ulp and
+// weight the two sides by their actual steps), or `width` consecutive fractions of
+// the line search, of which the first acceptable one is taken. The points, their
+// order and the accepted ones are those of a serial search, so the results are
+// its bits; a Newton step takes two rounds instead of seven or more evaluations
+// in a row. An accepted evaluation is the stability test's own point, so the test
+// reads its chemical potentials.
+__device__ __noinline__ void runTasks(MixCell& c, bool restarts, MixRecord* bestRecord, MixBest& best) {
+    const ReactiveB200HemModel& m = c.m;
+    const unsigned lane = threadIdx.x & 31u;
+    const int width = m.nl == 1 ? 6 : 8, groups = 32 / width;
+    const int g = int(lane) / width;
+    const bool inGroup = g < groups;
+    const int base = g * width, r = int(lane) - base;
+    const unsigned group = inGroup ? ((1u << width) - 1u) << base : 0u;
+    const double rho = density(c);
+    enum { IDLE, START, SIDES, TRIALS };
+    int st = IDLE, task = 0, it = 0, k = 0, owner = base, attempt = 0, nextTask = 0;
+    bool more = inGroup, converged = false, settled = false;
+    MixTask t{{0, 0}, 0, 0, 0, 0};
+    double x[4] = {}, f[4] = {}, step[4] = {}, column[4] = {}, scale = 1, previous = 0;
+    MixEval v, side;
+    for (;;) {
+        // idle groups take the next tasks in order
+        {
+            const unsigned idle = __ballot_sync(0xffffffffu, inGroup && r == 0 && st == IDLE && more);
+            if (inGroup && st == IDLE && more) {
+                task = nextTask + __popc(idle & ((1u << base) - 1u));
+                more = nthTask(c, restarts, task, t);
+                if (more) {
+                    if (r == 0) ++c.n.candidates;
+                    if (taskStart(c, t, x, scale)) st = START;
+                }
+            }
+            nextTask += __popc(idle);
+        }
+        if (__all_sync(0xffffffffu, st == IDLE)) {
+            if (!__any_sync(0xffffffffu, more)) break;
+            continue;
+        }
+        const int size = t.n + 2, j = r >> 1;
+        double xe[4] = {x[0], x[1], x[2], x[3]}, fe[4] = {}, fraction = 1, hp = 0, hm = 0;
+        bool point = false;
+        if (st == START) point = r == 0;
+        else if (st == SIDES) {
+            if (j < size && !settled) {
+                point = true;
+                const double h = ldexp(j < 2 ? 2e-6 : 2e-5, -attempt);
+                double xj = 0;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) xj = i == j ? x[i] : xj;
+                double xp = xj + h, xm = xj - h;
+                if (c.adaptive) {
+                    if (xp == xj) xp = nextafter(xj, HUGE_VAL);
+                    if (xm == xj) xm = nextafter(xj, -HUGE_VAL);
+                }
+                hp = xp - xj;
+                hm = xj - xm;
+                if (!c.adaptive) hp = hm = h;
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (i == j) xe[i] = (r & 1) ? xm : xp;
+            }
+        } else if (st == TRIALS && k + r < kTrials) {
+            point = true;
+            fraction = ldexp(1.0, -(k + r));
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (i < size) xe[i] = x[i] + fraction * step[i];
+            for (int i = 0; i < t.n; ++i) point = point && !rejectedCoordinate(c.adaptive, xe[i + 2]);
+        }
+        bool ok = false;
+        if (point) ok = activeResidual(c, t.active, t.n, xe, scale, fe, st == SIDES ? side : v);
+        __syncwarp();
+        bool finished = false, stable = false, evaluated = false;  // evaluated: (x, f) is a new iterate
+        if (st == SIDES) {
+            const bool other = __shfl_xor_sync(group, ok, 1);
+            double fo[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) fo[i] = __shfl_xor_sync(group, fe[i], 1);
+            bool exhausted = false;
+            if (j < size && !settled) {
+                const bool upper = !(r & 1), plus = upper ? ok : other, minus = upper ? other : ok;
+                if (plus || minus) {
+                    double maximum = 0;
+                    settled = true;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        if (i >= size) continue;
+                        const double fp = upper ? fe[i] : fo[i], fm = upper ? fo[i] : fe[i];
+                        double d;
+                        if (c.adaptive)
+                            d = plus && minus ? (hm / (hp + hm)) * ((fp - f[i]) / hp) + (hp / (hp + hm)) * ((f[i] - fm) / hm)
+                                              : plus ? (fp - f[i]) / hp : (f[i] - fm) / hm;
+                        else
+                            d = plus && minus ? (fp - fm) / (2 * hp) : plus ? (fp - f[i]) / hp : (f[i] - fm) / hp;
+                        column[i] = d;
+                        maximum = fmax(maximum, fabs(d));
+                        settled = settled && fin(d);
+                    }
+                    if (c.adaptive) settled = settled && maximum > 0;
+                }
+                if (!settled) exhausted = ++attempt >= 12;
+            }
+            const bool failed = __ballot_sync(group, exhausted) != 0;
+            const bool whole = __ballot_sync(group, j < size && !settled) == 0;
+            if (failed) finished = true;
+            else if (whole) {
+                double jac[4][4] = {}, rhs[4] = {}, answer[4] = {};
+#pragma unroll
+                for (int col = 0; col < 4; ++col)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const double d = __shfl_sync(group, column[i], base + (col < size ? 2 * col : 0));
+                        if (i < size && col < size) jac[i][col] = d;
+                    }
+                if (converged) {
+                    // the equilibrium sound speed of the converged point
+                    const double vp = __shfl_sync(group, v.s.p, owner), vs = __shfl_sync(group, v.s.soundFrozen, owner);
+                    rhs[0] = -1 / rho;
+                    rhs[1] = vp / (rho * scale);
+                    bool good = solveDense(jac, rhs, size, answer);
+                    const double squared = vp * answer[0], sound = good ? sqrt(squared) : 0.0;
+                    good = good && fin(squared) && squared > 0 && sound <= vs * (1 + 2e-3);
+                    finished = true;
+                    if (good && int(lane) == owner) {
+                        v.s.volumeResidual = fabs(f[0]);
+                        v.s.energyResidual = fabs(f[1]);
+                        v.s.chemicalResidual = maxAbs(f + 2, t.n);
+                        v.s.iterations = it;
+                        v.s.soundEquilibrium = sound;
+                        stable = true;
+                        for (int i = 0; i < m.nl; ++i) {
+                            if (c.q[m.condensable[i]] == 0) continue;
+                            const double affinity = v.muLiq[i] - v.muGas[i];
+                            stable = stable && (v.s.liquidMass[i] > 0 ? fin(affinity) && fabs(affinity) <= m.mutol * 2
+                                                                      : !(affinity < -m.mutol));
+                        }
+                    }
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) rhs[i] = i < size ? -f[i] : 0.0;
+                    if (!solveDense(jac, rhs, size, answer)) finished = true;
+                    else {
+                        double limiter = fmax(1., fmax(fabs(answer[0]) / .7, fabs(answer[1]) / .18));
+                        for (int i = 2; i < size; ++i) limiter = fmax(limiter, fabs(answer[i]) / (c.adaptive ? 2. : .3));
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) step[i] = i < size ? answer[i] / limiter : 0.0;
+                        previous = maxAbs(f, size);
+                        // the fractions a coordinate rejects form a prefix (each moves back
+                        // toward the valid x as the fraction halves): its end by bisection
+                        // on the trial's own expression, kTrials standing for none
+                        auto rejects = [&](int trial) {
+                            const double fm = ldexp(1.0, -trial);
+                            bool bad = false;
+                            for (int i = 0; i < t.n; ++i) bad |= rejectedCoordinate(c.adaptive, x[i + 2] + fm * step[i + 2]);
+                            return bad;
+                        };
+                        k = 0;
+                        if (rejects(0)) {
+                            int lower = 0, upper = kTrials;
+                            while (upper - lower > 1) {
+                                const int mid = (lower + upper) / 2;
+                                if (rejects(mid)) lower = mid; else upper = mid;
+                            }
+                            k = upper;
+                        }
+                        st = TRIALS;
+                        finished = k >= kTrials;
+                    }
+                }
+            }
+        } else if (st == START || st == TRIALS) {
+            if (st == TRIALS) ok = ok && maxAbs(fe, size) < previous * (1 - 1e-4 * fraction);
+            const unsigned accepted = __ballot_sync(group, ok);
+            if (accepted) {
+                owner = __ffs(accepted) - 1;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    x[i] = __shfl_sync(group, xe[i], owner);
+                    f[i] = __shfl_sync(group, fe[i], owner);
+                }
+                it = st == START ? 0 : it + 1;
+                evaluated = true;
+                finished = it >= 90;
+            } else {
+                k += width;
+                finished = st == START || k >= kTrials;
+            }
+        }
+        if (evaluated && !finished) {
+            converged = fabs(f[0]) <= m.vtol && fabs(f[1]) <= m.etol && maxAbs(f + 2, t.n) <= m.mutol;
+            st = SIDES;
+            settled = false;
+            attempt = 0;
+            if (r == 0) ++c.n.fd;
+        }
+        if (finished) st = IDLE;
+        // stable candidates enter the selection (a candidate's owner holds its state)
+        unsigned offers = __ballot_sync(0xffffffffu, stable);
+        if (stable) ++c.n.stable;
+        while (offers) {
+            const int from = __ffs(offers) - 1;
+            offers &= offers - 1;
+            const double e = __shfl_sync(0xffffffffu, v.entropyD, from);
+            const int o = __shfl_sync(0xffffffffu, task, from);
+            if (best.takes(e, o)) {
+                best = MixBest{true, e, o};
+                if (int(lane) == from) storeRecord(*bestRecord, v, kStable);
+            }
+            __syncwarp();
+        }
+    }
+}
+
+// One search (the candidate list, then the restart temperatures when it found no
+// stable candidate) into *bestRecord (shared by the warp): the fixed-partition
+// candidates' records, then the tasks.
+__device__ __noinline__ bool searchWarp(MixCell& c, const MixRecord& gas, const MixRecord& liquid,
+                                        MixRecord* bestRecord) {
+    const ReactiveB200HemModel& m = c.m;
+    const unsigned lane = threadIdx.x & 31u;
+    MixBest best{false, 0.0, 0};
+    auto offer = [&](const MixRecord& record, int order) {
+        if (record.status != kStable || !best.takes(record.entropyD, order)) return;
+        best = MixBest{true, record.entropyD, order};
+        if (lane == 0) *bestRecord = record;
+    };
+    offer(gas, -2);
+    offer(liquid, -1);
+    __syncwarp();
+    const bool prune = m.stableGasPrune && prunable(m) && gas.status == kStable && gas.s.gasMass > 0 && !c.adaptive;
+    if (!prune && m.nl) runTasks(c, false, bestRecord, best);
+    if (!best.have && m.nl) runTasks(c, true, bestRecord, best);
+    return best.have;
+}
+
+// The recovery of one item per warp, items from an on-device counter: the
+// candidate search; with the boundary recovery (or in a capillary batch, whose
+// transported trace inventories can defeat the reference seeds) a second search
+// in log vapour fractions when the first found nothing or left a condensable
+// almost entirely liquid beside a gas phase, the larger entropy (the first search
+// on a tie) kept. A frozen partition's result is its record. Results go to
+// out/success, or to outputs[cell] for the resident form; a failed cell gets its
+// seed.
+__global__ void __launch_bounds__(kSearchBlock) mixtureSearch(MixBatch b) {
+    const ReactiveB200HemModel& m = *b.model;
+    __shared__ MixRecord found[kSearchBlock / 32][2];
+    MixRecord* best = found[threadIdx.x >> 5];
+    const unsigned lane = threadIdx.x & 31u;
     Tally n;
     unsigned long long succeeded = 0;
-    for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < count; i += size_t(blockDim.x) * gridDim.x) {
-        const size_t cell = order ? size_t(order[i]) : i;
-        MixCell c{m, {0, 0, 0, 0}, energy[cell], seed[cell], false, n};
-        for (int k = 0; k < m.ns && k < kNs; ++k) c.q[k] = q[cell * size_t(m.ns) + k];
-        MixEval result;
-        bool ok;
-        if (capillary) {
-            const ReactiveGpuHemCapillaryInputV2 in = capillary[cell];
-            c.color = in.color;
-            c.jump = in.pressureJump;
-            if (!capillaryAccepted(m, c.color, c.jump)) ok = false;
-            else if (in.equilibrium) ok = recoverCell(c, result, true);
-            else {
-                const double mass[kLiq] = {c.guess.liquidMass[0], c.guess.liquidMass[1]};
-                ok = frozen(c, mass, result, 0);
+    MixCell c{m, {0, 0, 0, 0}, 0.0, ReactiveThermoState{}, false, n};
+    for (;;) {
+        unsigned i = 0;
+        if (lane == 0) i = atomicAdd(b.counters + C_SEARCH, 1u);
+        i = __shfl_sync(0xffffffffu, i, 0);
+        if (i >= b.count) break;
+        loadCell(b, i, c);
+        const MixRecord& gas = b.record[kGasRecord][i];
+        const ReactiveThermoState* result = nullptr;
+        if (gas.status == kInvalid) {
+        } else if (frozenItem(b, i)) {
+            if (gas.status == kStable) result = &gas.s;
+        } else {
+            const MixRecord& liquid = b.record[kLiquidRecord][i];
+            const bool have = searchWarp(c, gas, liquid, best);
+            if (have) result = &best[0].s;
+            if (m.boundaryRecovery || b.capillary) {
+                bool again = !have;
+                if (have)
+                    for (int l = 0; l < m.nl; ++l) {
+                        const double q = c.q[m.condensable[l]];
+                        if (q > 0 && best[0].s.gasMass > 0) again |= best[0].s.liquidMass[l] / q > 1 - 1e-4;
+                    }
+                if (again) {
+                    c.adaptive = true;
+                    const bool other = searchWarp(c, b.record[kFullGasRecord] ? b.record[kFullGasRecord][i] : gas,
+                                                  liquid, best + 1);
+                    if (other && !(have && best[0].entropyD >= best[1].entropyD)) result = &best[1].s;
+                }
             }
-        } else ok = recoverCell(c, result, false);
-        const ReactiveThermoState& st = ok ? result.s : c.guess;
-        if (out) out[cell] = st;
-        if (success) success[cell] = ok ? 1 : 0;
-        if (outputs) {
-            outputs[cell].state = st;
-            outputs[cell].success = ok ? 1 : 0;
         }
-        succeeded += ok ? 1 : 0;
+        const size_t cell = b.order ? size_t(b.order[i]) : size_t(i);
+        const double* from = reinterpret_cast<const double*>(result ? result : b.seed + cell);
+        double* to = reinterpret_cast<double*>(b.outputs ? &b.outputs[cell].state : b.out + cell);
+        constexpr unsigned words = sizeof(ReactiveThermoState) / sizeof(double);
+        if (lane < words) to[lane] = from[lane];
+        if (lane == 0) {
+            if (b.success) b.success[cell] = result ? 1 : 0;
+            if (b.outputs) b.outputs[cell].success = result ? 1 : 0;
+            succeeded += result ? 1 : 0;
+        }
+        __syncwarp();  // the shared records are rewritten by the next item
     }
-    atomicAdd(totals + M_PHASES, n.phases);
-    atomicAdd(totals + M_RESIDUALS, n.residuals);
-    atomicAdd(totals + M_CANDIDATES, n.candidates);
-    atomicAdd(totals + M_STABLE, n.stable);
-    atomicAdd(totals + M_FD, n.fd);
-    atomicAdd(totals + M_SUCCEEDED, succeeded);
+    flushTally(n, b.totals);
+    if (lane == 0 && succeeded) atomicAdd(b.totals + M_SUCCEEDED, succeeded);
 }
 
 // The capillary primitive initialisation (initializeCapillaryTP,
@@ -909,6 +1170,10 @@ struct MixtureFlash {
     int* success = nullptr;
     ReactiveGpuHemCapillaryInputV2* capillary = nullptr;  // allocated by the first capillary batch
     unsigned long long* totals = nullptr;
+    MixRecord* record[kRecordKinds] = {};
+    unsigned* list = nullptr;
+    unsigned* counters = nullptr;
+    unsigned newtonBlocks = 1, searchBlocks = 1;  // whole waves of resident blocks
     template <class T> T* alloc(size_t n) {
         void* p = nullptr;
         check(cudaMalloc(&p, n * sizeof(T)), "cudaMalloc");
@@ -938,6 +1203,17 @@ MixtureFlash* mixtureCreate(const ReactiveB200HemModel& m, size_t capacity, int 
     f->out = f->alloc<ReactiveThermoState>(capacity);
     f->success = f->alloc<int>(capacity);
     f->totals = f->alloc<unsigned long long>(M_COUNT);
+    f->record[kGasRecord] = f->alloc<MixRecord>(capacity);
+    f->record[kLiquidRecord] = f->alloc<MixRecord>(capacity);
+    if (m.stableGasPrune) f->record[kFullGasRecord] = f->alloc<MixRecord>(capacity);
+    f->list = f->alloc<unsigned>(capacity * kRecordKinds);
+    f->counters = f->alloc<unsigned>(C_COUNT);
+    int sms = 0, perSm = 0;
+    check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "attribute");
+    check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, mixtureNewton, kSearchBlock, 0), "occupancy");
+    f->newtonBlocks = unsigned(std::max(1, perSm) * std::max(1, sms));
+    check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, mixtureSearch, kSearchBlock, 0), "occupancy");
+    f->searchBlocks = unsigned(std::max(1, perSm) * std::max(1, sms));
     check(cudaMemcpyAsync(f->model, &m, sizeof(m), cudaMemcpyHostToDevice, f->stream), "H2D model");
     check(cudaStreamSynchronize(f->stream), "sync");
     return f.release();
@@ -945,6 +1221,27 @@ MixtureFlash* mixtureCreate(const ReactiveB200HemModel& m, size_t capacity, int 
 
 void mixtureDestroy(MixtureFlash* f) { delete f; }
 size_t mixtureDeviceBytes(const MixtureFlash* f) { return f ? f->bytes : 0; }
+
+// The batch's launches on the handle's stream: the scalar all-gas solves, the
+// fixed-partition Newtons they leave, then the searches. The handle's entry lock
+// keeps batches (which share the records) one after another.
+static void launchRecovery(MixtureFlash* f, MixBatch b) {
+    for (int i = 0; i < kRecordKinds; ++i) b.record[i] = f->record[i];
+    b.model = f->model;
+    b.list = f->list;
+    b.counters = f->counters;
+    b.totals = f->totals;
+    check(cudaMemsetAsync(f->counters, 0, C_COUNT * sizeof(unsigned), f->stream), "memset");
+    mixtureScalar<<<gridFor(b.count, kBlock), kBlock, 0, f->stream>>>(b);
+    check(cudaGetLastError(), "mixture scalar solves");
+    const size_t newtonGroups = kSearchBlock / kNewtonLanes, searchWarps = kSearchBlock / 32;
+    const size_t newtonNeed = (kRecordKinds * b.count + newtonGroups - 1) / newtonGroups;
+    const size_t searchNeed = (b.count + searchWarps - 1) / searchWarps;
+    mixtureNewton<<<unsigned(std::min<size_t>(f->newtonBlocks, newtonNeed)), kSearchBlock, 0, f->stream>>>(b);
+    check(cudaGetLastError(), "mixture Newton");
+    mixtureSearch<<<unsigned(std::min<size_t>(f->searchBlocks, searchNeed)), kSearchBlock, 0, f->stream>>>(b);
+    check(cudaGetLastError(), "mixture search");
+}
 
 void mixtureRun(MixtureFlash* f, const double* q, const double* energy, size_t count,
                 const ReactiveGpuHemCapillaryInputV2* capillary, ReactiveThermoState* states, int* success,
@@ -966,10 +1263,15 @@ void mixtureRun(MixtureFlash* f, const double* q, const double* energy, size_t c
               "H2D capillary");
     check(cudaMemsetAsync(f->totals, 0, M_COUNT * sizeof(unsigned long long), s), "memset");
     check(cudaEventRecord(a, s), "event");
-    mixtureFlashKernel<<<gridFor(count, kBlock), kBlock, 0, s>>>(f->model, f->q, f->energy, count, f->seed,
-                                                                  capillary ? f->capillary : nullptr, nullptr, f->out,
-                                                                  f->success, nullptr, f->totals);
-    check(cudaGetLastError(), "mixture flash");
+    MixBatch batch{};
+    batch.q = f->q;
+    batch.energy = f->energy;
+    batch.count = count;
+    batch.seed = f->seed;
+    batch.capillary = capillary ? f->capillary : nullptr;
+    batch.out = f->out;
+    batch.success = f->success;
+    launchRecovery(f, batch);
     check(cudaEventRecord(b, s), "event");
     check(cudaMemcpyAsync(states, f->out, count * sizeof(ReactiveThermoState), cudaMemcpyDeviceToHost, s), "D2H");
     check(cudaMemcpyAsync(success, f->success, count * sizeof(int), cudaMemcpyDeviceToHost, s), "D2H success");
@@ -1056,9 +1358,15 @@ void mixtureRunResident(MixtureFlash* f, const double* q, const double* energy, 
     check(cudaEventCreate(&b), "event");
     check(cudaMemsetAsync(f->totals, 0, M_COUNT * sizeof(unsigned long long), s), "memset");
     check(cudaEventRecord(a, s), "event");
-    mixtureFlashKernel<<<gridFor(count, kBlock), kBlock, 0, s>>>(f->model, q, energy, count, seed, capillary, order,
-                                                                  nullptr, nullptr, output, f->totals);
-    check(cudaGetLastError(), "mixture flash");
+    MixBatch batch{};
+    batch.q = q;
+    batch.energy = energy;
+    batch.count = count;
+    batch.seed = seed;
+    batch.capillary = capillary;
+    batch.order = order;
+    batch.outputs = output;
+    launchRecovery(f, batch);
     check(cudaEventRecord(b, s), "event");
     unsigned long long t[M_COUNT] = {};
     check(cudaMemcpyAsync(t, f->totals, sizeof(t), cudaMemcpyDeviceToHost, s), "D2H totals");
