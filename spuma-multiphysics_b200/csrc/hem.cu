@@ -2,7 +2,9 @@
 //
 // Launch sequence per batch (all on one stream, no host synchronisation, no
 // allocation; capturable in a CUDA graph):
-//   1 inputs     per cell: (rho, e, seed p/T/liquid mass)
+//   1 inputs     per cell: (rho, e, seed p/T/liquid mass); with the two-phase bound
+//                passGas also decides the cells that are plainly gas, and
+//                passSinglePhase the others outside the bound
 //   2 queue      persistent lane-level work queue over (candidate, cell) items:
 //                all seven candidates of every cell; with the model's
 //                stableGasPrune option, the all-gas/all-liquid items first, then
@@ -331,13 +333,7 @@ __device__ __forceinline__ bool gasDecides(const HemConst& C, const CandRecord& 
     return C.stableGasPrune && gas.status == 2 && gas.st.gasMass > 0;
 }
 
-// Cells whose two-phase seeds provably fail (the two-phase bound) have only
-// their all-gas and all-liquid candidates: one thread per cell solves them
-// through the same out-of-line solvers the work queue's state machines restate
-// (bit for bit the queue's candidates), selects as selectCandidates does (the
-// stable candidate of larger entropy, the all-gas one on a tie) and writes the
-// outputs; a cell with neither goes to the restart list. The other cells are
-// listed for the work queue.
+// Warp-aggregated append of `value` to a device list.
 __device__ __forceinline__ void appendTo(unsigned* list, unsigned* counter, bool take, unsigned value) {
     const unsigned mask = __ballot_sync(0xffffffffu, take);
     unsigned slot = 0;
@@ -346,70 +342,252 @@ __device__ __forceinline__ void appendTo(unsigned* list, unsigned* counter, bool
     if (take) list[slot + __popc(mask & ((1u << (threadIdx.x & 31)) - 1))] = value;
 }
 
+// What passGas reads of the model, passed by value: the species' constants are
+// then operands from the constant bank instead of loads.
+struct GasPass {
+    PureSpecies gas;
+    double Tmin, Tmax, pmin, pmax, vtol, etol, gasTmin, gasTmax, liquidFloor;
+    int enforceBounds, scalarRecovery;
+};
+
+// The all-gas candidate of one cell where its whole solve and its stability test
+// take the short way: scalarGas' iterates (the same routines on the same
+// temperatures, so its bits), decided without a root solve. False hands the cell
+// to the general pass.
 //
-// FROM_CONSERVED: the pass forms each cell's inputs itself from the SoA conserved
-// rows and the seeds (as inputsFromConserved does) and stores them in `in` only
-// for the cells it hands to the work queue or the restart search, the two later
-// readers of `in`; the cells it decides never write their inputs. `seed` may be
-// `state` (an in-place recovery): a thread reads its own cell's seed before it
-// writes that cell's state and touches no other cell's.
+// The bracket probe of a solve that moves (scalarGas widens the seed by `radius`
+// toward the residual's zero before its first Newton step) is checked for
+// acceptance only, by its mechanical half: its energy residual's sign is known,
+// since cv > 0 makes the residual rise with T, once the solution lies at least
+// half a radius inside the bracket (cv times half a radius is orders of magnitude
+// above the tolerance). Every other course (a step out of the bracket or past half
+// a radius, a rejected probe) goes to the general pass.
+__device__ __forceinline__ bool gasCell(const GasPass& G, const HemConst& C, double q, double e, double gT,
+                                        unsigned& phases, double* row) {
+    const PureSpecies& sp = G.gas;
+    DensityTerms d;
+    if (!isfinite(e) || !densityTerms(sp, q, d)) return false;
+    GasProbe g;
+    bool clear;
+    auto mechanics = [&](double T, GasProbe& at, bool& apart) {
+        return probeMechanics(sp, d, T, at) && at.p >= G.pmin && at.p <= G.pmax && T >= G.Tmin && T <= G.Tmax
+               && !(G.enforceBounds && (T < G.gasTmin || T > G.gasTmax)) && gasRootIsV0(sp, d, at, apart) == 1;
+    };
+    const double T0 = clampd(gT, G.Tmin, G.Tmax);
+    ++phases;
+    if (!(T0 > 0) || !mechanics(T0, g, clear) || !probeEnergy(sp, d, g)) return false;
+    double T = T0, F = fma(d.iV, g.eM, -e), cv = __dmul_rn(d.iV, g.cvM);
+    const double cp0 = __dmul_rn(probeCp(g, 1.0 / g.dpdV), sp.invW);
+    const double tolerance = G.etol * fmax(1e5 * q, q * cp0 * T);
+    if (!isfinite(F) || !isfinite(cv) || !(cv > 0)) return false;
+    int it = 0;
+    if (fabs(F) > tolerance) {
+        const double radius = fmax(1., .01 * T0);
+        double lower = T0, upper = T0;
+        if (F > 0) lower = fmax(G.Tmin, __dsub_rn(T0, radius)); else upper = fmin(G.Tmax, __dadd_rn(T0, radius));
+        if (!(upper - lower > .75 * radius)) return false;
+        {
+            GasProbe edge;
+            bool unused;
+            if (!mechanics(F > 0 ? lower : upper, edge, unused)) return false;
+        }
+        while (fabs(F) > tolerance) {
+            if (F > 0) upper = T; else lower = T;
+            const double next = T - F / cv;
+            if (!(next > lower && next < upper) || !(fabs(next - T0) <= .5 * radius) || ++it > 8) return false;
+            T = next;
+            ++phases;
+            if (!mechanics(T, g, clear) || !probeEnergy(sp, d, g)) return false;
+            F = fma(d.iV, g.eM, -e);
+            cv = __dmul_rn(d.iV, g.cvM);
+            if (!isfinite(F) || !isfinite(cv) || !(cv > 0)) return false;
+        }
+    }
+    if (!clear || !belowSaturation(C, g.p, T)) return false;
+    PhaseProps ph;
+    ChemTerms chem;
+    double sR;
+    gasProperties(sp, d, g, ph, chem, sR);
+    Eval v;
+    if (!gasOnly(ph, q, g.p, T, v)) return false;
+    const double eres = fabs(__dsub_rn(v.energy, e)) / energyScale(v, q);
+    if (!(eres <= G.etol)) return false;
+    // the state record (stateFromEval of the all-gas partition)
+    row[0] = g.p;
+    row[1] = T;
+    row[2] = q;
+    row[3] = v.energy / q;
+    row[4] = v.entropyD / q;
+    row[5] = row[6] = v.soundFrozen;
+    row[7] = 0;
+    row[8] = eres;
+    row[9] = 0;
+    row[10] = 1;
+    row[11] = row[12] = 0;
+    row[13] = q;
+    row[14] = row[15] = row[16] = row[17] = 0;
+    row[18] = q;
+    row[19] = v.cpD / q;
+    row[20] = v.cv;
+    row[21] = __hiloint2double(it, 0);  // iterations, activeLiquids
+    return true;
+}
+
+// First pass of a search with the two-phase bound: one thread per cell. A cell
+// outside the bound whose density also excludes the all-liquid partition has only
+// its all-gas candidate; where gasCell decides it, its outputs are written here.
+// Cells inside the bound are listed for the work queue, the others for the general
+// single-phase pass, with their inputs stored.
+//
+// Bound by FP64 latency and issue: the solve runs in registers (no stack: the
+// routines it shares with the general solvers are inlined, the species' constants
+// come from the constant bank), and the 176-byte records leave through a
+// per-warp shared-memory stage as full lines (a thread's own 22 stores would
+// touch 22 x 32 sectors a warp). The outputs are not read again by the flash:
+// streaming stores.
+//
+// FROM_CONSERVED: the inputs come from the SoA conserved rows and the seeds (as
+// inputsFromConserved forms them), else from `in`. `seed` may be `state` (an
+// in-place recovery): a warp reads its own cells' seeds before it writes their
+// states and touches no other cell's.
+constexpr int kGasThreads = 128, kStageRow = 23;  // 22 words a record and one of padding against bank conflicts
+#ifndef RB200_GAS_MINBLOCKS
+#define RB200_GAS_MINBLOCKS 5
+#endif
 template <bool FROM_CONSERVED>
+__global__ void __launch_bounds__(kGasThreads, RB200_GAS_MINBLOCKS) passGas(
+    const __grid_constant__ GasPass G, const HemConst* __restrict__ Cp, CellInput* __restrict__ in,
+    const double* __restrict__ cons, size_t stride, const ReactiveThermoState* seed, size_t count,
+    ReactiveThermoState* state, ReactiveTransportState* transport, int* success, unsigned* list, unsigned* general,
+    unsigned* counters, unsigned long long* totals) {
+    __shared__ double stage[kGasThreads / 32][32 * kStageRow];
+    const HemConst& C = *Cp;
+    double* rows = stage[threadIdx.x >> 5];
+    const unsigned lane = threadIdx.x & 31u;
+    const size_t first = blockIdx.x * size_t(blockDim.x) + (threadIdx.x & ~31u), c = first + lane;
+    Counts n;
+    bool queue = false, other = false, gas = false;
+    if (c < count) {
+        CellInput x;
+        if (FROM_CONSERVED) {
+            const double rho = __ldcs(cons + c), mx = __ldcs(cons + stride + c), my = __ldcs(cons + 2 * stride + c),
+                         mz = __ldcs(cons + 3 * stride + c), E = __ldcs(cons + 4 * stride + c);
+            x.q = rho;
+            x.e = E - .5 * (mx * mx + my * my + mz * mz) / rho;
+            x.gT = __ldcs(&seed[c].T);
+            x.noTwoPhase = twoPhaseImpossible(C, x.q, x.e);
+        } else {
+            x.q = in[c].q;
+            x.e = in[c].e;
+            x.gT = in[c].gT;
+            x.noTwoPhase = in[c].noTwoPhase;
+        }
+        if (!x.noTwoPhase) queue = true;
+        else {
+            gas = G.scalarRecovery && x.q * (1 + 1e-12) < G.liquidFloor
+                  && gasCell(G, C, x.q, x.e, x.gT, n.phases, rows + lane * kStageRow);
+            if (gas) {
+                ++n.stable;
+                n.candidates += 5;  // the two-phase seeds, failed without their solves
+                n.failures += 6;    // those and the all-liquid partition below its density floor
+            } else {
+                other = true;
+                n.phases = 0;  // the general pass counts its own
+            }
+        }
+        if (FROM_CONSERVED && (queue || other)) {
+            x.gp = __ldcs(&seed[c].p);
+            x.gml = __ldcs(&seed[c].liquidMass[0]);
+            in[c] = x;
+        }
+    }
+    appendTo(list, counters + LIST, queue, unsigned(c));
+    appendTo(general, counters + GENERAL, other, unsigned(c));
+    const unsigned decided = __ballot_sync(0xffffffffu, gas);
+    __syncwarp();
+    if (decided) {
+        constexpr int words = int(sizeof(ReactiveThermoState) / sizeof(double));
+        if (state) {
+            double* out = reinterpret_cast<double*>(state + first);
+#pragma unroll 2
+            for (int i = int(lane); i < 32 * words; i += 32) {
+                const int r = i / words;
+                if ((decided >> r) & 1u) __stcs(out + i, rows[r * kStageRow + i - r * words]);
+            }
+        }
+        if (transport) {
+            // p, T, rho, cv, frozen sound, gas mass, dilatation 0
+            double* out = reinterpret_cast<double*>(transport + first);
+            for (int i = int(lane); i < 32 * 7; i += 32) {
+                const int r = i / 7, f = i - 7 * r;
+                const int from = f < 3 ? f : (f == 3 ? 20 : (f == 4 ? 5 : 18));
+                if ((decided >> r) & 1u) __stcs(out + i, f == 6 ? 0.0 : rows[r * kStageRow + from]);
+            }
+        }
+        if (success && gas) __stcs(success + c, 1);
+    }
+    flushCounts(n, totals);
+}
+
+// Cells whose two-phase seeds provably fail (the two-phase bound) and that passGas
+// left: they have only their all-gas and all-liquid candidates, and one thread per
+// cell solves them through the same out-of-line solvers the work queue's state
+// machines restate (bit for bit the queue's candidates), selects as
+// selectCandidates does (the stable candidate of larger entropy, the all-gas one
+// on a tie) and writes the outputs; a cell with neither goes to the restart list.
 __global__ void __launch_bounds__(kPassThreads, RB200_PASS_MINBLOCKS) passSinglePhase(const HemConst* __restrict__ Cp,
-                                                                CellInput* __restrict__ in,
-                                                                const double* __restrict__ cons, size_t stride,
-                                                                const ReactiveThermoState* seed,
-                                                                size_t count, ReactiveThermoState* state,
+                                                                const CellInput* __restrict__ in,
+                                                                const unsigned* __restrict__ general,
+                                                                ReactiveThermoState* state,
                                                                 ReactiveTransportState* transport, int* success,
-                                                                unsigned* list, unsigned* fallback, unsigned* counters,
+                                                                unsigned* fallback, unsigned* counters,
                                                                 unsigned long long* totals) {
     const HemConst& C = *Cp;
     Counts n;
-    for (size_t base = blockIdx.x * size_t(blockDim.x); base < count; base += size_t(blockDim.x) * gridDim.x) {
-        const size_t c = base + threadIdx.x;
-        bool queue = false, restart = false;
-        if (c < count) {
-            const CellInput x = FROM_CONSERVED ? conservedInput(C, cons, stride, c, 1, seed) : in[c];
-            if (!x.noTwoPhase) queue = true;
-            else {
-                double bestEntropy = 0;
-                bool have = false;
-                for (int kind = 0; kind < 2; ++kind) {
-                    const double mass = kind ? x.q : 0.0;
-                    Eval v;
-                    CandidateOut o{};
-                    GasPoint g;
-                    bool known = false;
-                    const bool floor = kind == 1 && x.q * (1 + 1e-12) < C.liquidFloor;
-                    if (floor || !frozenSolve(C, x, mass, 0, v, o, n, g, known)) {
-                        ++n.failures;
-                        continue;
-                    }
-                    const bool stable = stableAt(C, x.q, v.liqMass, v.p, v.T, n, known ? &g : nullptr);
-                    if (!stable) {
-                        ++n.failures;
-                        continue;
-                    }
-                    ++n.stable;
-                    if (!have || v.entropyD > bestEntropy) {
-                        // the best so far goes straight to the outputs (a later, better
-                        // candidate overwrites it); a cell with none keeps its state
-                        have = true;
-                        bestEntropy = v.entropyD;
-                        ReactiveThermoState st;
-                        stateFromEval(v, x.q, o, st);
-                        writeOutputs(st, c, state, transport);
-                    }
+    const unsigned items = counters[GENERAL];
+    for (size_t base = blockIdx.x * size_t(blockDim.x); base < items; base += size_t(blockDim.x) * gridDim.x) {
+        const size_t item = base + threadIdx.x;
+        bool restart = false;
+        unsigned c = 0;
+        if (item < items) {
+            c = general[item];
+            const CellInput x = in[c];
+            double bestEntropy = 0;
+            bool have = false;
+            for (int kind = 0; kind < 2; ++kind) {
+                const double mass = kind ? x.q : 0.0;
+                Eval v;
+                CandidateOut o{};
+                GasPoint g;
+                bool known = false;
+                const bool floor = kind == 1 && x.q * (1 + 1e-12) < C.liquidFloor;
+                if (floor || !frozenSolve(C, x, mass, 0, v, o, n, g, known)) {
+                    ++n.failures;
+                    continue;
                 }
-                n.candidates += 5;  // the two-phase seeds, failed without their solves
-                n.failures += 5;
-                if (have) {
-                    if (success) __stcs(success + c, 1);
-                } else restart = true;
+                const bool stable = stableAt(C, x.q, v.liqMass, v.p, v.T, n, known ? &g : nullptr);
+                if (!stable) {
+                    ++n.failures;
+                    continue;
+                }
+                ++n.stable;
+                if (!have || v.entropyD > bestEntropy) {
+                    // the best so far goes straight to the outputs (a later, better
+                    // candidate overwrites it); a cell with none keeps its state
+                    have = true;
+                    bestEntropy = v.entropyD;
+                    ReactiveThermoState st;
+                    stateFromEval(v, x.q, o, st);
+                    writeOutputs(st, c, state, transport);
+                }
             }
-            if (FROM_CONSERVED && (queue || restart)) in[c] = x;
+            n.candidates += 5;  // the two-phase seeds, failed without their solves
+            n.failures += 5;
+            if (have) {
+                if (success) __stcs(success + c, 1);
+            } else restart = true;
         }
-        appendTo(list, counters + LIST, queue, unsigned(c));
-        appendTo(fallback, counters + FALLBACK, restart, unsigned(c));
+        appendTo(fallback, counters + FALLBACK, restart, c);
     }
     flushCounts(n, totals);
 }
@@ -779,9 +957,11 @@ struct HemDevice {
     CandRecord* rec = nullptr;  // 7 x capacity
     CandRecord* fb = nullptr;   // 4 x capacity
     unsigned* list = nullptr;
+    unsigned* general = nullptr;
     unsigned* fallback = nullptr;
     unsigned* counters = nullptr;
     unsigned long long* totals = nullptr;
+    GasPass gasPass{};
     // host-path staging
     double* dq = nullptr;
     double* de = nullptr;
@@ -845,9 +1025,8 @@ struct HemDevice {
         launchPlainFlash(cst, in, count, seed, state, transport, success, counters, totals, s);
     }
     // Launches steps 2-7 for `count` prepared inputs, or, given the SoA conserved
-    // rows of a pure fluid (cons, stride), forms the inputs first: inside the
-    // single-phase pass when the two-phase bound is on, else with
-    // inputsFromConserved.
+    // rows of a pure fluid (cons, stride), forms the inputs first: inside passGas
+    // when the two-phase bound is on, else with inputsFromConserved.
     void launchSearch(size_t count, const ReactiveThermoState* seed, ReactiveThermoState* state,
                       ReactiveTransportState* transport, int* success, cudaStream_t s,
                       const double* cons = nullptr, size_t stride = 0) {
@@ -869,14 +1048,16 @@ struct HemDevice {
         } else if (hostConst.domeN) {
             // single-phase cells one thread each (selected and written there), the
             // rest through the work queue and the selection below
+            const unsigned blocks = unsigned((count + kGasThreads - 1) / kGasThreads);
             if (fused)
-                passSinglePhase<true><<<passBlocks, kPassThreads, 0, s>>>(cst, in, cons, stride, seed, count, state,
-                                                                          transport, success, list, fallback,
-                                                                          counters, totals);
+                passGas<true><<<blocks, kGasThreads, 0, s>>>(gasPass, cst, in, cons, stride, seed, count, state, transport,
+                                                             success, list, general, counters, totals);
             else
-                passSinglePhase<false><<<passBlocks, kPassThreads, 0, s>>>(cst, in, nullptr, 0, nullptr, count, state,
-                                                                           transport, success, list, fallback,
-                                                                           counters, totals);
+                passGas<false><<<blocks, kGasThreads, 0, s>>>(gasPass, cst, in, nullptr, 0, nullptr, count, state,
+                                                              transport, success, list, general, counters, totals);
+            check(cudaGetLastError(), "passGas");
+            passSinglePhase<<<passBlocks, kPassThreads, 0, s>>>(cst, in, general, state, transport, success, fallback,
+                                                                counters, totals);
             check(cudaGetLastError(), "passSinglePhase");
             passQueue<<<passBlocks, kPassThreads, 0, s>>>(cst, in, count, list, 0, 7, rec, counters, Q_A, totals);
             check(cudaGetLastError(), "passQueue");
@@ -1032,6 +1213,7 @@ void* create(const void* raw, size_t bytes, size_t capacity, bool hostPath, char
         d->rec = d->alloc<CandRecord>(7 * capacity);
         d->fb = d->alloc<CandRecord>(4 * capacity);
         d->list = d->alloc<unsigned>(capacity);
+        d->general = d->alloc<unsigned>(capacity);
         d->fallback = d->alloc<unsigned>(capacity);
         d->counters = d->alloc<unsigned>(NCOUNTERS);
         d->totals = d->alloc<unsigned long long>(NTOTALS);
@@ -1041,6 +1223,9 @@ void* create(const void* raw, size_t bytes, size_t capacity, bool hostPath, char
         check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, passQueue, kPassThreads, 0), "occupancy");
         check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d->device), "attribute");
         d->passBlocks = std::max(1, perSm) * std::max(1, sms);
+        const HemConst& h = d->hostConst;
+        d->gasPass = GasPass{h.gas, h.Tmin, h.Tmax, h.pmin, h.pmax, h.vtol, h.etol, h.gasTmin, h.gasTmax,
+                             h.liquidFloor, h.enforceBounds, h.scalarRecovery};
         if (hostPath) d->ensureHostPath();
         buildDome(*d);
         check(cudaStreamSynchronize(d->stream), "sync");
@@ -1086,8 +1271,20 @@ std::string species(const ReactiveB200Table& t, PureSpecies& sp) {
         sp.polynomial[r] = g.polynomial;
         sp.regionMin[r] = g.minimumTemperature;
         for (int j = 0; j < 9; ++j) sp.coeff[r][j] = g.coefficient[j];
+        const double* a = g.coefficient;
+        const bool nine = g.polynomial == 9;
+        const double* c = a + (nine ? 2 : 0);
+        sp.powers[r] = NasaPowers{nine ? a[0] : 0.0, nine ? a[1] : 0.0, c[0], c[1], c[2], c[3], c[4],
+                                  c[1] / 2, c[2] / 3, c[3] / 4, c[4] / 5, nine ? a[7] : a[5],
+                                  c[2] / 2, c[3] / 3, c[4] / 4, nine ? a[8] : a[6]};
     }
     sp.regionMaxLast = s.regions[s.regionCount - 1].maximumTemperature;
+    sp.twoB = 2 * sp.b;
+    sp.bb = sp.b * sp.b;
+    sp.covolumeHi = (1.0 + kSqrt2) * sp.b;
+    sp.covolumeLo = (1.0 - kSqrt2) * sp.b;
+    sp.twoA = 2 * sp.a;
+    sp.kappaPlus1 = 1.0 + sp.kappa;
     return "";
 }
 
@@ -1189,6 +1386,7 @@ std::string phaseLine(PureSpecies& sp) {
     sp.rhoC = rc;
     sp.dRho = rc - .5 * (rl + rg);
     sp.dT = tc - tmid;
+    sp.lineSlope = sp.dRho / sp.dT;
     return std::isfinite(sp.dRho) && sp.dT > 0 ? "" : "HEM reported-phase construction failed";
 }
 

@@ -154,21 +154,66 @@ __device__ __forceinline__ int liquidFromShared(const HemConst& C, int shared, c
 }
 
 // What an accepted gas probe at (p, T) hands to the evaluations that follow at
-// the same point: the gas table's T-terms, the gas phase's properties (without
-// the chemical potential) at the probe's density, which is the gas root of the
-// cubic at (p, T), with their chemical-potential intermediates, and the cubic's
-// roots when the probe solved it (`roots`; otherwise an evaluation that needs
-// them solves the cubic itself, through the same routine). `clear` (meaningful
-// without roots): the cubic has no liquid root, or one above the covolume and at
-// least 1e-6 of its volume below the middle root, both by margins far above
-// rounding.
+// the same point: the density's and the probe's terms, and, once completeGas has
+// formed them, the gas table's T-terms and the gas phase's properties (without the
+// chemical potential) at the probe's density, which is the gas root of the cubic
+// at (p, T), with their chemical-potential intermediates; and the cubic's roots
+// when the probe solved it (`roots`; otherwise an evaluation that needs them solves
+// the cubic itself, through the same routine). `clear` (meaningful without roots):
+// the cubic has no liquid root, or one above the covolume and at least 1e-6 of its
+// volume below the middle root, both by margins far above rounding.
 struct GasPoint {
+    DensityTerms d;
+    GasProbe probe;
     TTerms t;
     Roots r;
     PhaseProps gas;
     ChemTerms chem;
     bool roots, clear;
 };
+
+// The accepted point's T-terms and properties from its probe.
+__device__ __forceinline__ void gasProperties(const PureSpecies& sp, const DensityTerms& d, const GasProbe& g,
+                                              PhaseProps& s, ChemTerms& chem, double& sR) {
+    const double idp = 1.0 / g.dpdV, cpM = probeCp(g, idp);
+    sR = probeEntropy(sp, g);
+    chem = ChemTerms{d.iv, d.id, log(__dmul_rn(__dmul_rn(g.RT, d.iv), sp.invRefP)), d.logRatio};
+    s.p = g.p;
+    s.rho = d.q;
+    s.V = d.V;
+    s.e = __dmul_rn(g.eM, sp.invW);
+    s.h = __dmul_rn(fma(g.p, d.V, g.eM), sp.invW);
+    s.s = __dmul_rn(fma(kGas, __dsub_rn(sR, chem.lg), __dmul_rn(d.L, g.da)), sp.invW);
+    s.cp = __dmul_rn(cpM, sp.invW);
+    s.cv = __dmul_rn(g.cvM, sp.invW);
+    s.alpha = __dmul_rn(-__dmul_rn(g.dpdT, idp), d.iV);
+    s.kappaT = __dmul_rn(-idp, d.iV);
+}
+__device__ RB200_FLASH_FN void completeGas(const HemConst& C, GasPoint& g) {
+    double sR;
+    gasProperties(C.gas, g.d, g.probe, g.gas, g.chem, sR);
+    g.t = TTerms{g.probe.T, g.probe.aa, g.probe.da, g.probe.d2a, g.probe.alphaRoot, g.probe.cpR, g.probe.hRT, sR};
+}
+
+// The phase sums of the all-gas partition at an accepted gas point (the whole
+// density q is gas at its own volume).
+__device__ __forceinline__ bool gasOnly(const PhaseProps& ph, double q, double p, double T, Eval& v) {
+    v.p = p;
+    v.T = T;
+    v.gasMass = q;
+    v.volume = 1.0;
+    v.energy = __dmul_rn(q, ph.e);
+    v.entropyD = __dmul_rn(q, ph.s);
+    v.cpD = __dmul_rn(q, ph.cp);
+    v.gRho = q;
+    v.cv = ph.cv;
+    // -(1/q)^2 / (-kappaT/q + T (alpha/q)^2 / cp)
+    const double specific = 1.0 / q, vt = __dmul_rn(ph.alpha, specific);
+    const double adiabatic = fma(__dmul_rn(T, vt), vt / ph.cp, -__dmul_rn(ph.kappaT, specific));
+    if (!fin(v.cv) || v.cv <= 0 || !(adiabatic < 0)) return false;
+    v.soundFrozen = sqrt(__dmul_rn(-specific, specific) / adiabatic);
+    return fin(v.soundFrozen) && v.soundFrozen > 0 && fin(v.energy) && fin(v.entropyD) && fin(v.cpD);
+}
 
 // Phase sums at (p, T) for liquid mass `mass` out of total density q. With
 // `virt` the liquid is also evaluated when absent and both chemical potentials
@@ -195,6 +240,7 @@ __device__ RB200_FLASH_FN bool evaluate(const HemConst& C, double q, double mass
     const double gas = q - mass;
     if (!fin(gas) || gas < 0 || gas > q) return false;
     v.gasMass = gas;
+    if (known && mass == 0 && !virt) return gasOnly(known->gas, q, p, T, v);
     const bool needLiquid = mass > 0 || (virt && q > 0);
     const bool shared = C.samePure && gas > 0 && needLiquid;
     TTerms t;
@@ -336,69 +382,75 @@ __device__ RB200_FLASH_FN bool gasRootAt(const HemConst& C, double q, double p, 
 // against 1e-14, ||h| - |q|| >= 1e-8 against 1e-10), the other roots at least
 // 1e-6 of V0 away from V0 (so V0 is no near-double root and dp/dV stays off
 // zero there), and 1e-9 of V0 (or of the line's density) from the covolume,
-// the classification centre and the reported-phase line. `phase` is the
-// reported phase of the (T, q) evaluation; `clear` as GasPoint::clear.
-__device__ __forceinline__ int gasRootIsV0(const PureSpecies& sp, const TTerms& t, double p, double q, int phase,
-                                           bool& clear) {
-    const double T = t.T, V0 = sp.W / q, ip = 1.0 / p;
-    const double b = sp.b, b2 = b * b, RTp = kGas * T * ip, aap = t.aa * ip, bn = b - RTp;
-    const double cn = -(2.0 * RTp * b - aap + 3.0 * b2), dn = b2 * RTp + b2 * b - aap * b;
-    const double center = -bn * kThird, delta2 = (bn * bn - 3.0 * cn) * (1.0 / 9.0);
-    const double qc = 2.0 * bn * bn * bn * (1.0 / 27.0) - bn * cn * kThird + dn;
-    const double delta = delta2 > 0 ? sqrt(delta2) : 0.0, h = 2.0 * delta * delta2;
-    const double disc = qc * qc - h * h, margin = 1e-9 * V0;
+// the classification centre and the reported-phase line. `clear` as GasPoint::clear.
+__device__ __forceinline__ int gasRootIsV0(const PureSpecies& sp, const DensityTerms& d, const GasProbe& g, bool& clear) {
+    const double T = g.T, V0 = d.V, q = d.q, ip = 1.0 / g.p;
+    const double b = sp.b, b2 = sp.bb, RTp = __dmul_rn(g.RT, ip), bn = __dsub_rn(b, RTp);
+    const double cn = fma(g.aa, ip, -fma(__dmul_rn(2.0, RTp), b, __dmul_rn(3.0, b2)));
+    const double dn = fma(b2, RTp, fma(b2, b, -__dmul_rn(__dmul_rn(g.aa, ip), b)));
+    const double center = __dmul_rn(-bn, kThird), delta2 = __dmul_rn(fma(bn, bn, -__dmul_rn(3.0, cn)), 1.0 / 9.0);
+    const double qc = fma(__dmul_rn(__dmul_rn(2.0 / 27.0, bn), bn), bn, fma(__dmul_rn(-kThird, bn), cn, dn));
+    const double delta = delta2 > 0 ? sqrt(delta2) : 0.0, h = __dmul_rn(__dmul_rn(2.0, delta), delta2);
+    const double disc = fma(qc, qc, -__dmul_rn(h, h)), margin = __dmul_rn(1e-9, V0);
     clear = false;
-    if (!(fabs(fabs(h) - fabs(qc)) >= 1e-8) || !(fabs(disc) >= 1e-10) || !(V0 - b > margin)) return -1;
+    if (!(fabs(__dsub_rn(fabs(h), fabs(qc))) >= 1e-8) || !(fabs(disc) >= 1e-10) || !(__dsub_rn(V0, b) > margin)) return -1;
     bool single = disc > 0;  // one real root: V0
     clear = single;
     if (!single) {
-        const double s = bn + V0, tq = cn + V0 * s, d2 = s * s - 4.0 * tq;
+        const double s = __dadd_rn(bn, V0), tq = fma(V0, s, cn), d2 = fma(s, s, -__dmul_rn(4.0, tq));
         if (!(d2 > 0)) return -1;
-        const double r = sqrt(d2), v1 = .5 * (-s + r), v2 = .5 * (-s - r);
-        if (v1 > V0 + 1e-6 * V0) return 0;  // the largest root, the gas root if any, is not V0
-        if (!(v1 < V0 - 1e-6 * V0) || !(fabs(v1 - b) > margin) || !(fabs(v2 - b) > margin)) return -1;
+        const double r = sqrt(d2), v1 = __dmul_rn(.5, __dsub_rn(r, s)), v2 = __dmul_rn(-.5, __dadd_rn(s, r));
+        if (v1 > __dmul_rn(1 + 1e-6, V0)) return 0;  // the largest root, the gas root if any, is not V0
+        if (!(v1 < __dmul_rn(1 - 1e-6, V0)) || !(fabs(__dsub_rn(v1, b)) > margin) || !(fabs(__dsub_rn(v2, b)) > margin))
+            return -1;
         single = !(v1 > b);  // V0 the only root above the covolume
         // three physical roots with the liquid one off the spinodal, or V0 alone
-        clear = single || (v2 > b && v1 - v2 > 1e-6 * v1);
+        clear = single || (v2 > b && __dsub_rn(v1, v2) > __dmul_rn(1e-6, v1));
     }
     if (single && !(T > sp.Tc)) {
         // a lone root is the gas root when it is not below the centre
-        if (!(fabs(V0 - center) > margin)) return -1;
+        if (!(fabs(__dsub_rn(V0, center)) > margin)) return -1;
         if (V0 < center) return 0;
     }
-    if (phase == -2) return 1;  // above the reported-phase line's temperature: no density test
-    const double rhoMid = sp.rhoC + (T - sp.tcLine) * sp.dRho / sp.dT;
-    if (q < rhoMid * (1 - 1e-9)) return phase == -1 ? 1 : -1;
-    if (q > rhoMid * (1 + 1e-9)) return phase == 0 ? 0 : -1;
+    if (T >= sp.tcLine) return 1;  // above the reported-phase line's temperature: no density test
+    const double rhoMid = fma(__dsub_rn(T, sp.tcLine), sp.lineSlope, sp.rhoC);
+    if (q < __dmul_rn(rhoMid, 1 - 1e-9)) return 1;
+    if (q > __dmul_rn(rhoMid, 1 + 1e-9)) return 0;
     return -1;
 }
 
 // Energy residual of the all-gas state at (T, rho) and the gas-root check: the
-// properties at (T, rho), then the gas root of the cubic at the resulting
-// pressure must be that density: decided by gasRootIsV0 where its margins
-// allow, else by the root solve. `g` receives the point: the T-terms, the
-// properties at rho with their chemical-potential intermediates, and the roots
-// when they were solved.
+// probe at (T, rho), then the gas root of the cubic at the resulting pressure must
+// be that density: decided by gasRootIsV0 where its margins allow, else by the
+// root solve. `g` receives the point: the density's and the probe's terms, and the
+// roots when they were solved.
 __device__ RB200_FLASH_FN bool gasProbe(const HemConst& C, double q, double eIn, double T, double& F, double& cv, double& p,
                                 double& cp, GasPoint& g, Counts& n) {
-    int phase;
     ++n.phases;
-    if (!fin(T) || !fin(q) || T <= 0 || q <= 0) return false;
-    if (tTermsBody(C.gas, T, g.t) != EOS_OK || prTrhoTBody(C.gas, g.t, q, false, g.gas, phase, &g.chem) != EOS_OK)
+    if (!fin(T) || T <= 0) return false;
+    if (!densityTerms(C.gas, q, g.d) || !probeMechanics(C.gas, g.d, T, g.probe) || !probeEnergy(C.gas, g.d, g.probe))
         return false;
-    p = g.gas.p;  // finite and positive
+    p = g.probe.p;  // finite and positive
     if (!inBounds(C, p, T)) return false;
     if (C.enforceBounds && (T < C.gasTmin || T > C.gasTmax)) return false;
-    const int decided = gasRootIsV0(C.gas, g.t, p, q, phase, g.clear);
+    const int decided = gasRootIsV0(C.gas, g.d, g.probe, g.clear);
     if (decided == 0) return false;
     g.roots = decided < 0;
     if (g.roots) {
         ++n.phases;
+        g.t.T = T;  // the root check's T-terms (it forms no chemical potential and reads no entropy)
+        g.t.aa = g.probe.aa;
+        g.t.da = g.probe.da;
+        g.t.d2a = g.probe.d2a;
+        g.t.q = g.probe.alphaRoot;
+        g.t.cpR = g.probe.cpR;
+        g.t.hRT = g.probe.hRT;
+        g.t.sR = 0;
         if (!gasRootAt(C, q, p, g)) return false;
     }
-    F = q * g.gas.e - eIn;
-    cv = q * g.gas.cv;
-    cp = g.gas.cp;
+    F = fma(g.d.iV, g.probe.eM, -eIn);
+    cv = __dmul_rn(g.d.iV, g.probe.cvM);
+    cp = __dmul_rn(probeCp(g.probe, 1.0 / g.probe.dpdV), C.gas.invW);
     return fin(F) && fin(cv) && cv > 0;
 }
 
@@ -457,6 +509,7 @@ __device__ RB200_FLASH_FN bool scalarGas(const HemConst& C, const CellInput& in,
         if (!gasProbe(C, q, in.e, T, F, cv, p, d3, g, n)) return false;
     }
     if (fabs(F) > C.etol * scale) return false;
+    completeGas(C, g);
     if (!evaluate(C, q, 0.0, p, T, false, v, n, &g)) return false;
     o.vres = fabs(v.volume - 1);
     o.eres = fabs(v.energy - in.e) / energyScale(v, q);
@@ -634,12 +687,15 @@ __device__ RB200_FLASH_FN bool twoPhaseSolve(const HemConst& C, const CellInput&
 // attraction term) or the root is not a liquid by the reported-phase line
 // (unavailable, also stable). T at or above the table's start is at or above
 // the liquid range's lower end, where the full test would fail the candidate.
-__device__ __forceinline__ bool gasStableBelowSaturation(const HemConst& C, double p, double T, const GasPoint& g) {
+__device__ __forceinline__ bool belowSaturation(const HemConst& C, double p, double T) {
     if (!C.domeN || C.satN < 2 || !(T >= C.satT0)) return false;
     const double cell = floor((T - C.satT0) * C.satInvStep) - 1;
     if (!(cell >= 0) || !(cell < C.satN)) return false;
     const double ps = C.satP[int(cell)];
-    if (!(p < ps * (1 - 1e-6))) return false;
+    return p < ps * (1 - 1e-6);
+}
+__device__ __forceinline__ bool gasStableBelowSaturation(const HemConst& C, double p, double T, const GasPoint& g) {
+    if (!belowSaturation(C, p, T)) return false;
     if (!g.roots) return g.clear;
     if (!g.r.liquid) return true;  // no liquid root: unavailable, stable
     if (g.r.count != 3) return false;

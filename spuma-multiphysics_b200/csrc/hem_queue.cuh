@@ -227,6 +227,7 @@ __device__ inline bool plan(const HemConst& C, QueueLane& L, Eval& v, Record rec
             if (!(L.it < 70 && fabs(L.F) > C.etol * L.scale)) {
                 if (fabs(L.F) > C.etol * L.scale) { L.st = Q_FZ_NEWTON_INIT; continue; }
                 // (P, T0) are the last probe's point: its terms serve the final evaluation
+                completeGas(C, L.g);
                 L.req = REQ_POINT; L.rm = 0; L.rp = L.P; L.rT = L.T0; L.rv = false; L.known = true;
                 L.st = Q_SG_FINAL;
                 return true;

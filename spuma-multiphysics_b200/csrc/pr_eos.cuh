@@ -40,6 +40,14 @@ enum RootChoice : int { ROOT_AUTO = 0, ROOT_GAS = 1, ROOT_LIQUID = 2 };
 
 constexpr int kMaxRegions = 8;
 
+// One NASA region as powers of T, both polynomial kinds in one form:
+//   cp/R = (m2/T + m1)/T + c0 + T(c1 + T(c2 + T(c3 + T c4)))
+//   h/RT = (hc + m1 ln T - m2/T)/T + c0 + T(h1 + T(h2 + T(h3 + T h4)))
+//   s/R  = -(m2/(2T) + m1)/T + c0 ln T + sc + T(c1 + T(s2 + T(s3 + T s4)))
+struct NasaPowers {
+    double m2, m1, c0, c1, c2, c3, c4, h1, h2, h3, h4, hc, s2, s3, s4, sc;
+};
+
 // Immutable per-species constants, derived on the host from the model image.
 struct PureSpecies {
     double a, b, kappa, W, Tc, refP;
@@ -52,6 +60,10 @@ struct PureSpecies {
     double regionMin[kMaxRegions];
     double regionMaxLast;
     double coeff[kMaxRegions][9];
+    NasaPowers powers[kMaxRegions];
+    double twoB, bb, covolumeHi, covolumeLo;  // 2b, b^2, (1 + sqrt2) b, (1 - sqrt2) b
+    double twoA, kappaPlus1;                  // 2a, 1 + kappa
+    double lineSlope;                         // dRho/dT of the reported-phase line
 };
 
 struct PhaseProps {
@@ -111,6 +123,87 @@ __device__ __forceinline__ void nasaEval(const PureSpecies& sp, double T, double
 
 __device__ __forceinline__ double cubicAt(double V, double bn, double cn, double dn) {
     return ((V + bn) * V + cn) * V + dn;
+}
+
+// ---------------------------------------------------------------------------
+// The all-gas partition at a fixed density: its properties need no root of the
+// cubic, the density's own terms are formed once per cell, and a temperature probe
+// forms only what its residual and its checks read. Every sum is written as
+// explicit fused or rounded operations, so each place these routines are inlined
+// (the single-phase pass, the work queue, the plain form) gives the same bits.
+
+// Terms of the density q: V = W/q, 1/(V - b), 1/(V^2 + 2bV - b^2), the factors of
+// dp/dV, the attraction logarithm (and over 2 sqrt2 b), 1/V.
+struct DensityTerms {
+    double q, V, iv, id, iv2, g2, logRatio, L, iV;
+};
+__device__ __forceinline__ bool densityTerms(const PureSpecies& sp, double q, DensityTerms& d) {
+    if (!fin(q) || q <= 0) return false;
+    const double V = sp.W / q;
+    const double den = fma(V, __dadd_rn(V, sp.twoB), -sp.bb), vmb = __dsub_rn(V, sp.b);
+    if (!(V > sp.b) || !(den > 0) || !(vmb > 0)) return false;
+    d.q = q;
+    d.V = V;
+    d.iv = 1.0 / vmb;
+    d.id = 1.0 / den;
+    d.iv2 = __dmul_rn(d.iv, d.iv);
+    d.g2 = __dmul_rn(__dmul_rn(2.0, __dadd_rn(V, sp.b)), __dmul_rn(d.id, d.id));
+    d.logRatio = log(__dadd_rn(V, sp.covolumeHi) / __dadd_rn(V, sp.covolumeLo));
+    d.L = __dmul_rn(d.logRatio, sp.invL);
+    d.iV = __dmul_rn(q, sp.invW);
+    return true;
+}
+
+// A probe at (T, d): a*alpha and its T-derivatives, p and its derivatives, and
+// (probeEnergy) cp/R and h/RT of the ideal gas, the molar energy and cv.
+struct GasProbe {
+    double T, iT, RT, alphaRoot, aa, da, d2a, p, dpdV, dpdT, cpR, hRT, eM, cvM;
+};
+// p(T, V) with 0 < p and dp/dV < 0, both finite: the mechanical half of a probe.
+__device__ __forceinline__ bool probeMechanics(const PureSpecies& sp, const DensityTerms& d, double T, GasProbe& g) {
+    g.T = T;
+    g.iT = 1.0 / T;
+    const double root = sqrt(__dmul_rn(T, sp.invTc)), f = fma(-sp.kappa, root, sp.kappaPlus1);
+    if (fabs(f) <= 1e-14) return false;
+    // sqrt(T/Tc)/T = 1/(Tc sqrt(T/Tc)): d|f|/dT = -+ kappa/(2 Tc sqrt(T/Tc)), and its own
+    // derivative is -1/(2T) times it
+    const double a = fabs(f), half = __dmul_rn(__dmul_rn(.5, sp.kappa), __dmul_rn(root, g.iT));
+    const double df = f > 0 ? -half : half, d2f = __dmul_rn(__dmul_rn(-.5, df), g.iT);
+    g.alphaRoot = a;
+    g.aa = __dmul_rn(sp.a, __dmul_rn(a, a));
+    g.da = __dmul_rn(sp.twoA, __dmul_rn(a, df));
+    g.d2a = __dmul_rn(sp.twoA, fma(df, df, __dmul_rn(a, d2f)));
+    g.RT = __dmul_rn(kGas, T);
+    g.p = fma(g.RT, d.iv, -__dmul_rn(g.aa, d.id));
+    g.dpdV = fma(g.aa, d.g2, -__dmul_rn(g.RT, d.iv2));
+    g.dpdT = fma(kGas, d.iv, -__dmul_rn(g.da, d.id));
+    return fin(g.p) && g.p > 0 && g.dpdV < 0 && fin(g.dpdV) && fin(g.dpdT) && g.aa > 0 && fin(g.d2a);
+}
+// e = RT (h/RT - 1) + L (T da - aa) and cv = R (cp/R - 1) + L T d2a per kmol; cv > 0.
+__device__ __forceinline__ bool probeEnergy(const PureSpecies& sp, const DensityTerms& d, GasProbe& g) {
+    const NasaPowers& n = sp.powers[nasaRegion(sp, g.T)];
+    const double T = g.T, iT = g.iT;
+    g.cpR = fma(T, fma(T, fma(T, fma(T, n.c4, n.c3), n.c2), n.c1), n.c0);
+    g.hRT = fma(T, fma(T, fma(T, fma(T, n.h4, n.h3), n.h2), n.h1), fma(n.hc, iT, n.c0));
+    if (n.m1 != 0 || n.m2 != 0) {
+        g.cpR = fma(fma(n.m2, iT, n.m1), iT, g.cpR);
+        g.hRT = fma(fma(n.m1, log(T), -__dmul_rn(n.m2, iT)), iT, g.hRT);
+    }
+    g.eM = fma(g.RT, __dsub_rn(g.hRT, 1.0), __dmul_rn(d.L, fma(T, g.da, -g.aa)));
+    g.cvM = fma(kGas, __dsub_rn(g.cpR, 1.0), __dmul_rn(__dmul_rn(d.L, T), g.d2a));
+    return fin(g.eM) && fin(g.cvM) && g.cvM > 0;
+}
+// cp per kmol: cv - T (dp/dT)^2 / (dp/dV).
+__device__ __forceinline__ double probeCp(const GasProbe& g, double idp) {
+    return fma(-__dmul_rn(g.T, g.dpdT), __dmul_rn(g.dpdT, idp), g.cvM);
+}
+// The probe's s/R of the ideal gas (its logarithm only the accepted point needs).
+__device__ __forceinline__ double probeEntropy(const PureSpecies& sp, const GasProbe& g) {
+    const NasaPowers& n = sp.powers[nasaRegion(sp, g.T)];
+    const double T = g.T;
+    double s = fma(T, fma(T, fma(T, fma(T, n.s4, n.s3), n.s2), n.c1), fma(n.c0, log(T), n.sc));
+    if (n.m1 != 0 || n.m2 != 0) s = fma(-fma(__dmul_rn(.5, n.m2), g.iT, n.m1), g.iT, s);
+    return s;
 }
 
 // Physical roots (finite, above the covolume), smallest and largest.
