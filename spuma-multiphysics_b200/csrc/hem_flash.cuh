@@ -63,8 +63,10 @@ struct HemConst {
 
 struct CellInput {
     double q, e, gp, gT, gml;  // mass density, internal energy density, seed p, T, liquid mass
-    int noTwoPhase;            // no two-phase candidate can converge (the dome bound)
+    int skip;                  // SKIP_*: candidates that provably cannot converge
 };
+// No two-phase candidate (the dome bound); no all-gas, no all-liquid partition (singlePhaseImpossible).
+enum : int { SKIP_TWO_PHASE = 1, SKIP_GAS = 2, SKIP_LIQUID = 4 };
 
 // True when the cell's (1/q, e/q) lies provably outside every saturation tie
 // line widened by the margins: the two-phase seeds would all fail.

@@ -159,8 +159,8 @@ __device__ __forceinline__ bool densityTerms(const PureSpecies& sp, double q, De
 struct GasProbe {
     double T, iT, RT, alphaRoot, aa, da, d2a, p, dpdV, dpdT, cpR, hRT, eM, cvM;
 };
-// p(T, V) with 0 < p and dp/dV < 0, both finite: the mechanical half of a probe.
-__device__ __forceinline__ bool probeMechanics(const PureSpecies& sp, const DensityTerms& d, double T, GasProbe& g) {
+// The mechanical half of a probe, false at the cusp of |1 + kappa (1 - sqrt(T/Tc))|.
+__device__ __forceinline__ bool probeTerms(const PureSpecies& sp, const DensityTerms& d, double T, GasProbe& g) {
     g.T = T;
     g.iT = 1.0 / T;
     const double root = sqrt(__dmul_rn(T, sp.invTc)), f = fma(-sp.kappa, root, sp.kappaPlus1);
@@ -177,7 +177,11 @@ __device__ __forceinline__ bool probeMechanics(const PureSpecies& sp, const Dens
     g.p = fma(g.RT, d.iv, -__dmul_rn(g.aa, d.id));
     g.dpdV = fma(g.aa, d.g2, -__dmul_rn(g.RT, d.iv2));
     g.dpdT = fma(kGas, d.iv, -__dmul_rn(g.da, d.id));
-    return fin(g.p) && g.p > 0 && g.dpdV < 0 && fin(g.dpdV) && fin(g.dpdT) && g.aa > 0 && fin(g.d2a);
+    return g.aa > 0 && fin(g.d2a);
+}
+// The same with 0 < p and dp/dV < 0, both finite.
+__device__ __forceinline__ bool probeMechanics(const PureSpecies& sp, const DensityTerms& d, double T, GasProbe& g) {
+    return probeTerms(sp, d, T, g) && fin(g.p) && g.p > 0 && g.dpdV < 0 && fin(g.dpdV) && fin(g.dpdT);
 }
 // e = RT (h/RT - 1) + L (T da - aa) and cv = R (cp/R - 1) + L T d2a per kmol; cv > 0.
 __device__ __forceinline__ bool probeEnergy(const PureSpecies& sp, const DensityTerms& d, GasProbe& g) {
