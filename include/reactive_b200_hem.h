@@ -125,7 +125,7 @@ int reactive_gpu_hem_vjp_device_v3(void* hem, const double* conserved, size_t st
  * whose own memory pool owns the whole device and forbids other allocations. It
  * takes the model image and DEVICE
  * arrays like reactive_gpu_hem_run_device_v3 but needs no handle: its scratch is
- * one file-scope device array (about 9 MB, held by every GPU that loads this
+ * one file-scope device array (about 6 MB, held by every GPU that loads this
  * library until the process exits) for at most 4,096 cells per call; larger
  * batches are rejected with an error. Every call looks up the array's address on
  * the current device; the first call on each device also loads this library's

@@ -12,9 +12,8 @@
 //   4 queue      their five two-phase seeds
 //   5 select     first maximum entropy among stable candidates, in reference
 //                order; cells without one are queued for the restart search
-//   6 pass C     persistent queue over (queued cell, 4 restart temperatures),
-//                each running the 5 seeds and keeping its first best
-//   7 select     over the 4 restarts; cells still without a candidate fail
+//   6 pass C     a warp per queued cell: 4 restart temperatures x 5 seeds on its
+//                lanes, the first best written; cells still without one fail
 // Candidate records live in HBM (192 B each); every loop in the solvers is
 // bounded and no thread waits on another, so every launch terminates.
 #include "hem_flash.cuh"
@@ -47,13 +46,6 @@ struct CandRecord {
     int pad;
 };
 static_assert(sizeof(CandRecord) == 192, "candidate record layout");
-
-// Warp-wide dynamic fetch of 32 consecutive items from a device counter.
-__device__ __forceinline__ unsigned fetchItems(unsigned* counter) {
-    unsigned base = 0;
-    if ((threadIdx.x & 31) == 0) base = atomicAdd(counter, 32u);
-    return __shfl_sync(0xffffffffu, base, 0);
-}
 
 __global__ void inputsFromHost(const HemConst* __restrict__ Cp, const double* q, const double* energy,
                                const ReactiveThermoState* guess, size_t count, int ns, CellInput* in) {
@@ -703,50 +695,60 @@ __global__ void selectCandidates(const HemConst* __restrict__ Cp, const CandReco
     }
 }
 
-// Pass C: restart temperatures x queued cells; each item runs the five seeds.
+// Pass C: the restart search of the cells without a candidate, one warp per cell:
+// twenty lanes run the twenty two-phase solves (four restart temperatures x five
+// seeds) side by side, and the first maximum of the entropy density in the serial
+// order (temperatures, then seeds: the lane order) is written; a cell without one
+// keeps its seed and fails. The solves of one cell are long serial Newton chains;
+// one thread running a temperature's five in turn had them five times as long.
 __global__ void __launch_bounds__(kPassThreads, RB200_PASS_MINBLOCKS) passRestarts(const HemConst* __restrict__ Cp,
                                                              const CellInput* __restrict__ in,
-                                                             const unsigned* __restrict__ fallback, CandRecord* fb,
-                                                             size_t capacity, unsigned* counters,
-                                                             unsigned long long* totals) {
+                                                             const unsigned* __restrict__ fallback,
+                                                             const ReactiveThermoState* seed,
+                                                             ReactiveThermoState* state,
+                                                             ReactiveTransportState* transport, int* success,
+                                                             unsigned* counters, unsigned long long* totals) {
     const HemConst& C = *Cp;
     Counts n;
-    const unsigned queued = counters[FALLBACK];
-    const unsigned total = 4u * queued;
+    const unsigned queued = counters[FALLBACK], lane = threadIdx.x & 31u;
     const double lower = fmax(C.Tmin, C.liquidTmin), upper = fmin(C.Tmax, C.liquidTc * (1 - 1e-10));
+    constexpr unsigned solves = 20;
     for (;;) {
-        const unsigned base = fetchItems(counters + Q_C);
-        if (base >= total) break;
-        const unsigned item = base + (threadIdx.x & 31);
-        if (item < total) {
-            const unsigned t = item / queued, slot = item % queued;
-            const CellInput x = in[fallback[slot]];
-            CandRecord* out = fb + size_t(t) * capacity + slot;
-            out->status = 0;
+        unsigned slot = 0;
+        if (lane == 0) slot = atomicAdd(counters + Q_C, 1u);
+        slot = __shfl_sync(0xffffffffu, slot, 0);
+        if (slot >= queued) break;
+        const size_t c = fallback[slot];
+        const CellInput x = in[c];
+        Eval v;
+        CandidateOut o{};
+        bool have = false;
+        if (lane < solves) {
             if (x.skip & SKIP_TWO_PHASE) {  // no restart seed can converge either
-                n.candidates += 5;
-                n.failures += 5;
+                ++n.candidates;
+                ++n.failures;
             } else if (upper > lower) {
-                const double restartT = lower + (upper - lower) * kRestart[t];
-                bool have = false;
-                double bestEntropy = 0;
-                for (int s = 0; s < 5; ++s) {
-                    Eval v;
-                    CandidateOut o{};
-                    const bool ok = twoPhaseSolve(C, x, kSeeds[s], restartT, v, o, n);
-                    if (!ok) { ++n.failures; continue; }
-                    const bool stable = stableAt(C, x.q, v.liqMass, v.p, v.T, n);
-                    if (!stable) { ++n.failures; continue; }
-                    ++n.stable;
-                    if (!have || v.entropyD > bestEntropy) {
-                        have = true;
-                        bestEntropy = v.entropyD;
-                        stateFromEval(v, x.q, o, out->st);
-                        out->entropyD = v.entropyD;
-                        out->status = 2;
-                    }
-                }
+                have = twoPhaseSolve(C, x, kSeeds[lane % 5], lower + (upper - lower) * kRestart[lane / 5], v, o, n)
+                       && stableAt(C, x.q, v.liqMass, v.p, v.T, n);
+                if (have) ++n.stable; else ++n.failures;
             }
+        }
+        __syncwarp();
+        double best = have ? v.entropyD : -HUGE_VAL;
+        for (int s = 16; s; s >>= 1) best = fmax(best, __shfl_xor_sync(0xffffffffu, best, s));
+        const unsigned winners = __ballot_sync(0xffffffffu, have && v.entropyD == best);
+        const unsigned writer = winners ? unsigned(__ffs(winners) - 1) : 0u;
+        if (lane == writer) {
+            if (winners) {
+                ReactiveThermoState st;
+                stateFromEval(v, x.q, o, st);
+                writeOutputs(st, c, state, transport);
+            } else {
+                if (seed && state) writeOutputs(seed[c], c, state, nullptr);
+                if (transport && seed) writeOutputs(seed[c], c, nullptr, transport);
+                atomicAdd(counters + FAILED, 1u);
+            }
+            if (success) success[c] = winners ? 1 : 0;
         }
     }
     flushCounts(n, totals);
@@ -930,30 +932,6 @@ __global__ void keepFailed(const ReactiveThermoState* __restrict__ seed, const i
     }
 }
 
-__global__ void selectRestarts(const CandRecord* fb, size_t capacity, const unsigned* fallback,
-                               const ReactiveThermoState* seed, ReactiveThermoState* state,
-                               ReactiveTransportState* transport, int* success, unsigned* counters) {
-    const unsigned queued = counters[FALLBACK];
-    for (unsigned slot = blockIdx.x * blockDim.x + threadIdx.x; slot < queued; slot += blockDim.x * gridDim.x) {
-        const size_t c = fallback[slot];
-        int best = -1;
-        double bestEntropy = 0;
-        for (int t = 0; t < 4; ++t) {
-            const CandRecord& r = fb[size_t(t) * capacity + slot];
-            if (r.status == 2 && (best < 0 || r.entropyD > bestEntropy)) { best = t; bestEntropy = r.entropyD; }
-        }
-        if (best >= 0) {
-            writeOutputs(fb[size_t(best) * capacity + slot].st, c, state, transport);
-            if (success) success[c] = 1;
-        } else {
-            if (seed && state) writeOutputs(seed[c], c, state, nullptr);
-            if (transport && seed) writeOutputs(seed[c], c, nullptr, transport);
-            if (success) success[c] = 0;
-            atomicAdd(counters + FAILED, 1u);
-        }
-    }
-}
-
 // One thread per cell running the whole search in order (the layout of the
 // reference's hemKernel, src/reactiveTransport/reactiveGpuHem.cuh:64-80): the
 // plain form the candidate-parallel passes are measured against. No pruning.
@@ -1021,7 +999,6 @@ struct HemDevice {
     HemConst* cst = nullptr;
     CellInput* in = nullptr;
     CandRecord* rec = nullptr;  // 7 x capacity
-    CandRecord* fb = nullptr;   // 4 x capacity
     unsigned* list = nullptr;
     unsigned* general = nullptr;
     unsigned* fallback = nullptr;
@@ -1090,7 +1067,7 @@ struct HemDevice {
         check(cudaMemsetAsync(counters, 0, NCOUNTERS * sizeof(unsigned), s), "memset counters");
         launchPlainFlash(cst, in, count, seed, state, transport, success, counters, totals, s);
     }
-    // Launches steps 2-7 for `count` prepared inputs, or, given the SoA conserved
+    // Launches steps 2-6 for `count` prepared inputs, or, given the SoA conserved
     // rows of a pure fluid (cons, stride), forms the inputs first: inside passGas
     // when the two-phase bound is on, else with inputsFromConserved.
     void launchSearch(size_t count, const ReactiveThermoState* seed, ReactiveThermoState* state,
@@ -1134,11 +1111,9 @@ struct HemDevice {
         selectCandidates<<<gridFor(count, 256), 256, 0, s>>>(cst, rec, count, selectList, state, transport, success,
                                                              fallback, counters);
         check(cudaGetLastError(), "selectCandidates");
-        passRestarts<<<passBlocks, kPassThreads, 0, s>>>(cst, in, fallback, fb, capacity, counters, totals);
+        passRestarts<<<passBlocks, kPassThreads, 0, s>>>(cst, in, fallback, seed, state, transport, success, counters,
+                                                         totals);
         check(cudaGetLastError(), "passRestarts");
-        selectRestarts<<<gridFor(count, 256), 256, 0, s>>>(fb, capacity, fallback, seed, state, transport, success,
-                                                           counters);
-        check(cudaGetLastError(), "selectRestarts");
     }
 };
 
@@ -1277,7 +1252,6 @@ void* create(const void* raw, size_t bytes, size_t capacity, bool hostPath, char
         d->cst = d->alloc<HemConst>(1);
         d->in = d->alloc<CellInput>(capacity);
         d->rec = d->alloc<CandRecord>(7 * capacity);
-        d->fb = d->alloc<CandRecord>(4 * capacity);
         d->list = d->alloc<unsigned>(capacity);
         d->general = d->alloc<unsigned>(capacity);
         d->fallback = d->alloc<unsigned>(capacity);
@@ -1935,7 +1909,7 @@ int reactive_gpu_hem_run_counters_v3(void* raw, ReactiveGpuHemProfileV1* profile
 // same work-queue flash as reactive_gpu_hem_run_device_v3 with no handle: its
 // scratch (the derived model constants, per-cell inputs, candidate records,
 // lists and queue counters) lives in one file-scope __device__ array sized for
-// at most kStaticHemCells cells (about 9 MB). Every GPU that loads this library
+// at most kStaticHemCells cells (about 6 MB). Every GPU that loads this library
 // holds that array until the process exits.
 //
 // Every call looks up the array's device address with cudaGetSymbolAddress for
@@ -1955,8 +1929,7 @@ constexpr size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 constexpr size_t kStaticConst = 0;
 constexpr size_t kStaticIn = align256(kStaticConst + sizeof(HemConst));
 constexpr size_t kStaticRec = align256(kStaticIn + kStaticHemCells * sizeof(CellInput));
-constexpr size_t kStaticFb = align256(kStaticRec + 7 * kStaticHemCells * sizeof(CandRecord));
-constexpr size_t kStaticList = align256(kStaticFb + 4 * kStaticHemCells * sizeof(CandRecord));
+constexpr size_t kStaticList = align256(kStaticRec + 7 * kStaticHemCells * sizeof(CandRecord));
 constexpr size_t kStaticFallback = align256(kStaticList + kStaticHemCells * sizeof(unsigned));
 constexpr size_t kStaticCounters = align256(kStaticFallback + kStaticHemCells * sizeof(unsigned));
 constexpr size_t kStaticTotals = align256(kStaticCounters + NCOUNTERS * sizeof(unsigned));
@@ -2018,7 +1991,6 @@ extern "C" int reactive_gpu_hem_run_static_v3(const void* model, size_t modelByt
         auto* cst = reinterpret_cast<HemConst*>(base + kStaticConst);
         auto* in = reinterpret_cast<CellInput*>(base + kStaticIn);
         auto* rec = reinterpret_cast<CandRecord*>(base + kStaticRec);
-        auto* fb = reinterpret_cast<CandRecord*>(base + kStaticFb);
         auto* list = reinterpret_cast<unsigned*>(base + kStaticList);
         auto* fallback = reinterpret_cast<unsigned*>(base + kStaticFallback);
         auto* counters = reinterpret_cast<unsigned*>(base + kStaticCounters);
@@ -2041,9 +2013,8 @@ extern "C" int reactive_gpu_hem_run_static_v3(const void* model, size_t modelByt
         check(cudaGetLastError(), "passQueue");
         selectCandidates<<<gridFor(count, 256), 256, 0, s>>>(cst, rec, count, nullptr, state, transport, success,
                                                              fallback, counters);
-        passRestarts<<<blocks, kPassThreads, 0, s>>>(cst, in, fallback, fb, kStaticHemCells, counters, totals);
-        selectRestarts<<<gridFor(count, 256), 256, 0, s>>>(fb, kStaticHemCells, fallback, seed, state, transport,
-                                                           success, counters);
+        passRestarts<<<blocks, kPassThreads, 0, s>>>(cst, in, fallback, seed, state, transport, success, counters,
+                                                     totals);
         check(cudaGetLastError(), "select");
         return 0;
     } catch (const std::exception& e) {
