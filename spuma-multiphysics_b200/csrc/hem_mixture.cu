@@ -77,6 +77,10 @@ struct MixCell {
     bool adaptive;
     Tally& n;
     double color = 0, jump = 0;
+    // the reported-phase lines of the last gas composition and of the pure liquids:
+    // forming one takes a mixing and a cubic solve at least, as much as the
+    // evaluation it labels
+    mix::PhaseLine gasLine{}, liquidLine[kLiq]{};
 };
 
 __device__ __forceinline__ bool fin(double x) { return x == x && fabs(x) <= 1.79769313486231570815e308; }
@@ -117,7 +121,7 @@ __device__ __noinline__ int gasPhase(MixCell& c, double p, double T, const doubl
                 if (T < sp.regions[0].minimumTemperature || T > sp.regions[sp.regionCount - 1].maximumTemperature)
                     return mix::BAD_INPUT;
             }
-    return mix::tp(c.m.phase[0], T, p, Y, mix::GAS, chem, out);
+    return mix::tp(c.m.phase[0], T, p, Y, mix::GAS, chem, out, &c.gasLine);
 }
 
 // The pure liquid of condensed phase i at (p, T) on its liquid root.
@@ -127,7 +131,7 @@ __device__ __noinline__ int liquidPhase(MixCell& c, int i, double p, double T, b
     if (T < c.m.liquidTmin[i]) return mix::BAD_INPUT;
     if (T >= c.m.liquidTc[i] * (1 - 1e-10)) return mix::UNAVAILABLE;
     const double pure[kNs] = {1, 0, 0, 0};
-    return mix::tp(c.m.phase[i + 1], T, p, pure, mix::LIQUID, chem, out);
+    return mix::tp(c.m.phase[i + 1], T, p, pure, mix::LIQUID, chem, out, &c.liquidLine[i]);
 }
 
 __device__ __forceinline__ void addPhase(MixEval& v, double mass, const mix::Props& p, double pressure) {
@@ -269,7 +273,7 @@ __device__ __noinline__ bool gasProbe(MixCell& c, double T, double& F, double& c
     for (int k = 0; k < c.m.ns; ++k) Y[k] = c.q[k] / rho;
     ++c.n.phases;
     mix::Props prop;
-    if (mix::trho(c.m.phase[0], T, rho, Y, false, prop) != mix::OK) return false;
+    if (mix::trho(c.m.phase[0], T, rho, Y, false, prop, &c.gasLine) != mix::OK) return false;
     const double gasP = prop.p;
     p = gasP + c.color * c.jump;
     if (!inBounds(c.m, p, T)) return false;
@@ -517,8 +521,8 @@ __device__ __forceinline__ void storeRecord(MixRecord& r, const MixEval& v, int 
 __global__ void __launch_bounds__(kBlock) mixtureScalar(MixBatch b) {
     const ReactiveB200HemModel& m = *b.model;
     Tally n;
+    MixCell c{m, {0, 0, 0, 0}, 0.0, ReactiveThermoState{}, false, n};
     for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < b.count; i += size_t(blockDim.x) * gridDim.x) {
-        MixCell c{m, {0, 0, 0, 0}, 0.0, ReactiveThermoState{}, false, n};
         loadCell(b, i, c);
         const bool frozen = frozenItem(b, i);
         bool valid = !b.capillary || capillaryAccepted(m, c.color, c.jump);
@@ -535,6 +539,7 @@ __global__ void __launch_bounds__(kBlock) mixtureScalar(MixBatch b) {
         MixEval v;
         if (m.scalarRecovery && mass0 == 0 && mass1 == 0 && scalarGas(c, v)) {
             const int status = frozen || stableCandidate(c, v) ? kStable : kUnstable;
+            n.stable += !frozen && status == kStable;
             storeRecord(gas, v, status);
             if (b.record[kFullGasRecord]) storeRecord(b.record[kFullGasRecord][i], v, status);
         } else {
@@ -648,6 +653,7 @@ __global__ void __launch_bounds__(kSearchBlock) mixtureNewton(MixBatch b) {
                 v.s.energyResidual = fabs(re);
                 v.s.iterations = it;
                 const int status = frozen || stableCandidate(c, v) ? kStable : kUnstable;
+                n.stable += !frozen && status == kStable;
                 storeRecord(*record, v, status);
                 code = 1;
             } else {
@@ -1017,7 +1023,7 @@ __device__ __noinline__ bool searchWarp(MixCell& c, const MixRecord& gas, const 
 // on a tie) kept. A frozen partition's result is its record. Results go to
 // out/success, or to outputs[cell] for the resident form; a failed cell gets its
 // seed.
-__global__ void __launch_bounds__(kSearchBlock) mixtureSearch(MixBatch b) {
+__global__ void __launch_bounds__(kSearchBlock, 3) mixtureSearch(MixBatch b) {
     const ReactiveB200HemModel& m = *b.model;
     __shared__ MixRecord found[kSearchBlock / 32][2];
     MixRecord* best = found[threadIdx.x >> 5];

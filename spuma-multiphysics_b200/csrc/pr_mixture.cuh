@@ -59,8 +59,10 @@ RB200_HD inline int moles(const ReactiveB200Table& t, const double* Y, double* x
     return OK;
 }
 
-// NASA7/9 cp/R, h/RT, s/R of species k at T.
-RB200_HD inline void nasa(const ReactiveB200Species& sp, double T, double& cpR, double& hRT, double& sR) {
+// NASA7/9 cp/R, h/RT, s/R of species k at T (iT = 1/T, lT = ln T, shared by the
+// species of one evaluation).
+RB200_HD inline void nasa(const ReactiveB200Species& sp, double T, double iT, double lT, double& cpR, double& hRT,
+                          double& sR) {
     int r = 0;
     for (int j = 1; j < sp.regionCount; ++j) {
         const double edge = sp.regions[j].minimumTemperature;
@@ -68,7 +70,7 @@ RB200_HD inline void nasa(const ReactiveB200Species& sp, double T, double& cpR, 
         r = j;
     }
     const double* a = sp.regions[r].coefficient;
-    const double T2 = T * T, T3 = T2 * T, T4 = T3 * T, iT = 1.0 / T, lT = log(T);
+    const double T2 = T * T, T3 = T2 * T, T4 = T3 * T;
     if (sp.regions[r].polynomial == 7) {
         cpR = a[0] + a[1] * T + a[2] * T2 + a[3] * T3 + a[4] * T4;
         hRT = a[0] + .5 * a[1] * T + a[2] * T2 / 3.0 + .25 * a[3] * T3 + .2 * a[4] * T4 + a[5] * iT;
@@ -116,6 +118,21 @@ RB200_HD inline int mixing(const ReactiveB200Table& t, double T, const double* x
     const bool good = finiteD(m.a) && finiteD(m.b) && finiteD(m.aa) && finiteD(m.da) && finiteD(m.d2a);
     return good && m.a > 0 && m.b > 0 && m.aa > 0 ? OK : NONFINITE;
 }
+
+// The reported-phase line of one composition (reportedPhase): its end points do not
+// depend on the state, so a caller that evaluates one composition at many states
+// keeps the line between them. status is what forming the line returned.
+struct PhaseLine {
+    double x[kMaxNs];
+    double tmid, midT;
+    int status;
+    bool ready;
+    RB200_HD bool holds(const ReactiveB200Table& t, const double* y) const {
+        bool same = ready;
+        for (int k = 0; k < t.ns; ++k) same = same && x[k] == y[k];
+        return same;
+    }
+};
 
 struct Roots {
     double V[3];  // ascending physical molar volumes (> b)
@@ -212,19 +229,13 @@ RB200_HD inline int roots(const Mixing& m, double T, double p, Roots& r) {
     return OK;
 }
 
-// The reported phase of a mixture state (Cantera's density heuristic): above the
-// mixture's pseudo-critical T supercritical; below it, gas-like when rho is under
-// the line from the critical density to the mid density of the two roots at
-// T_mid = Tc - 100 K (or Tc / 2), the pressure there raised by 4% until the cubic
-// has both roots above pc or three roots (at most 100 cubic solves).
-RB200_HD inline int reportedPhase(const ReactiveB200Table& t, double T, const double* x, double W, double rho,
-                                  const Mixing& atT, int& phase) {
-    const double tc = atT.a * kOmB / (atT.b * kOmA * kR), pc = kOmB * kR * tc / atT.b, vc = kOmVc * kR * tc / pc;
-    if (T >= tc) {
-        phase = SUPERCRITICAL;
-        return OK;
-    }
-    const double tmid = tc - 100.0 < 0 ? .5 * tc : tc - 100.0, ratio = tc / tmid;
+// The line's end at T_mid = Tc - 100 K (or Tc / 2): the mid density of the two
+// roots there, the pressure raised by 4% until the cubic has both roots above pc or
+// three roots (at most 100 cubic solves).
+RB200_HD inline int phaseLine(const ReactiveB200Table& t, const double* x, double W, double tc, double pc,
+                              PhaseLine& line) {
+    line.tmid = tc - 100.0 < 0 ? .5 * tc : tc - 100.0;
+    const double tmid = line.tmid, ratio = tc / tmid;
     double pp = pc * exp(-.8734 * ratio * ratio - 3.4522 * ratio + 4.2918), liquidV = -1;
     bool found = false;
     Mixing m;
@@ -239,19 +250,41 @@ RB200_HD inline int reportedPhase(const ReactiveB200Table& t, double T, const do
         } else found = true;
     }
     if (!found || !(liquidV > 0) || !finiteD(liquidV)) return NONFINITE;
-    const double rhoC = W / vc, midT = .5 * (W / liquidV + W / (kR * tmid / pp));
-    const double rhoMid = rhoC + (T - tc) * (rhoC - midT) / (tc - tmid);
+    line.midT = .5 * (W / liquidV + W / (kR * tmid / pp));
+    return OK;
+}
+
+// The reported phase of a mixture state (Cantera's density heuristic): above the
+// mixture's pseudo-critical T supercritical; below it, gas-like when rho is under
+// the line from the critical density to phaseLine's mid density. kept (optional):
+// the line of the last composition.
+RB200_HD inline int reportedPhase(const ReactiveB200Table& t, double T, const double* x, double W, double rho,
+                                  const Mixing& atT, int& phase, PhaseLine* kept) {
+    const double tc = atT.a * kOmB / (atT.b * kOmA * kR), pc = kOmB * kR * tc / atT.b, vc = kOmVc * kR * tc / pc;
+    if (T >= tc) {
+        phase = SUPERCRITICAL;
+        return OK;
+    }
+    PhaseLine line;
+    if (kept && kept->holds(t, x)) line = *kept;
+    else {
+        line.ready = true;
+        for (int k = 0; k < kMaxNs; ++k) line.x[k] = x[k];
+        line.status = phaseLine(t, x, W, tc, pc, line);
+        if (kept) *kept = line;
+    }
+    if (line.status) return line.status;
+    const double rhoC = W / vc, rhoMid = rhoC + (T - tc) * (rhoC - line.midT) / (tc - line.tmid);
     phase = rho < rhoMid ? GASLIKE : LIQUIDLIKE;
     return finiteD(rhoMid) ? OK : NONFINITE;
 }
 
-// Properties at (T, rho) and mass fractions Y; chem: the species chemical potentials.
-RB200_HD inline int trho(const ReactiveB200Table& t, double T, double rho, const double* Y, bool chem, Props& s) {
-    if (!finiteD(T) || !finiteD(rho) || T <= 0 || rho <= 0) return BAD_INPUT;
-    double x[kMaxNs] = {}, W = 0;
-    if (const int st = moles(t, Y, x, W)) return st;
-    Mixing m;
-    if (const int st = mixing(t, T, x, m)) return st;
+// Properties at (T, rho); chem: the species chemical potentials. The composition
+// comes as its mole fractions x, molar mass W and mixing terms m at T; kept as in
+// reportedPhase. (See trho for mass fractions.)
+RB200_HD inline int trhoMixed(const ReactiveB200Table& t, double T, double rho, const double* x, double W,
+                              const Mixing& m, bool chem, Props& s, PhaseLine* kept) {
+    if (!finiteD(rho) || rho <= 0) return BAD_INPUT;
     const double b = m.b, V = W / rho;
     if (!(V > b)) return NO_ROOT;
     const double den = V * V + 2.0 * V * b - b * b, vmb = V - b;
@@ -264,10 +297,11 @@ RB200_HD inline int trho(const ReactiveB200Table& t, double T, double rho, const
     if (!finiteD(dpdV) || !finiteD(dpdT) || dpdV >= 0) return UNSTABLE;
     const double logRatio = log((V + (1.0 + kRt2) * b) / (V + (1.0 - kRt2) * b));
     const double L = logRatio / (2.0 * kRt2 * b);
+    const double iT = 1.0 / T, lT = log(T);
     double h0 = 0, s0 = 0, cp0 = 0, xlx = 0, hk[kMaxNs], sk[kMaxNs];
     for (int k = 0; k < t.ns; ++k) {
         double cpR, hRT, sR;
-        nasa(t.species[k], T, cpR, hRT, sR);
+        nasa(t.species[k], T, iT, lT, cpR, hRT, sR);
         hk[k] = hRT;
         sk[k] = sR;
         cp0 += x[k] * kR * cpR;
@@ -277,7 +311,8 @@ RB200_HD inline int trho(const ReactiveB200Table& t, double T, double rho, const
     }
     const double z = p * V / RT;
     const double hM = h0 + (RT * (z - 1.0) + L * (T * m.da - m.aa));
-    const double sM = s0 - kR * xlx - kR * log(p / t.refPressure) + (kR * log(z * (1.0 - b / V)) + L * m.da);
+    const double lnP = log(p / t.refPressure);
+    const double sM = s0 - kR * xlx - kR * lnP + (kR * log(z * (1.0 - b / V)) + L * m.da);
     const double cvV = cp0 + V * dpdT - kR + L * T * m.d2a;  // dH/dT at constant V
     const double cpM = cvV - (V + T * dpdT / dpdV) * dpdT;
     const double cvM = cpM + T * dpdT * dpdT / dpdV;
@@ -291,21 +326,32 @@ RB200_HD inline int trho(const ReactiveB200Table& t, double T, double rho, const
     if (!(s.cp > 0) || !(s.cv > 0) || !(s.kappaT > 0) || !(sound2 > 0)) return UNSTABLE;
     s.sound = sqrt(sound2);
     if (chem) {
+        const double lnZ = log(z), lnV = log(V / vmb);
         for (int k = 0; k < t.ns; ++k) {
             double pp = 0;
             for (int i = 0; i < t.ns; ++i) pp += x[i] * t.aBinary[k][i] * (m.q[i] * m.q[k]);
             const double bk = t.species[k].b, num = 2.0 * b * pp - m.aa * bk;
-            s.mu[k] = RT * (hk[k] - sk[k]) + RT * log(fmax(1e-300, x[k])) + RT * log(p / t.refPressure)
-                    - RT * log(z) + RT * log(V / vmb) + RT * bk / vmb - num / (2.0 * kRt2 * b * b) * logRatio
+            s.mu[k] = RT * (hk[k] - sk[k]) + RT * log(fmax(1e-300, x[k])) + RT * lnP
+                    - RT * lnZ + RT * lnV + RT * bk / vmb - num / (2.0 * kRt2 * b * b) * logRatio
                     - m.aa * bk * V / (b * den);
             if (!finiteD(s.mu[k])) return NONFINITE;
         }
     }
-    if (const int st = reportedPhase(t, T, x, W, rho, m, s.phase)) return st;
+    if (const int st = reportedPhase(t, T, x, W, rho, m, s.phase, kept)) return st;
     const double check[] = {s.e, s.h, s.s, s.cp, s.cv, s.alpha, s.kappaT, s.sound};
     for (double c : check)
         if (!finiteD(c)) return NONFINITE;
     return OK;
+}
+
+RB200_HD inline int trho(const ReactiveB200Table& t, double T, double rho, const double* Y, bool chem, Props& s,
+                         PhaseLine* kept = nullptr) {
+    if (!finiteD(T) || !finiteD(rho) || T <= 0 || rho <= 0) return BAD_INPUT;
+    double x[kMaxNs] = {}, W = 0;
+    if (const int st = moles(t, Y, x, W)) return st;
+    Mixing m;
+    if (const int st = mixing(t, T, x, m)) return st;
+    return trhoMixed(t, T, rho, x, W, m, chem, s, kept);
 }
 
 // Partial molar enthalpies [J/kmol] of the mixture of mass fractions Y at the
@@ -343,7 +389,7 @@ RB200_HD inline int partialEnthalpies(const ReactiveB200Table& t, double T, cons
             dpp += x[i] * pair * (2.0 * dq[i] / m.q[i] + 2.0 * dq[k] / m.q[k]);
         }
         double cpR, hRT, sR;
-        nasa(t.species[k], T, cpR, hRT, sR);
+        nasa(t.species[k], T, 1.0 / T, log(T), cpR, hRT, sR);
         const double bk = t.species[k].b;
         const double dpdn = RT / vmb + RT * bk / (vmb * vmb) - 2.0 * pp / den + 2.0 * vmb * m.aa * bk / (den * den);
         const double departure = V * dpdn - RT - bk / (2.0 * kRt2 * b * b) * logRatio * fac
@@ -358,7 +404,7 @@ RB200_HD inline int partialEnthalpies(const ReactiveB200Table& t, double T, cons
 // gas-side), with the pressure postcondition |p(T, rho) - p| <= 1e-7 max(1, p)
 // and the reported phase consistent with a GAS / LIQUID choice.
 RB200_HD inline int tp(const ReactiveB200Table& t, double T, double p, const double* Y, int choice, bool chem,
-                       Props& s) {
+                       Props& s, PhaseLine* kept = nullptr) {
     if (!finiteD(T) || !finiteD(p) || T <= 0 || p <= 0) return BAD_INPUT;
     double x[kMaxNs] = {}, W = 0;
     if (const int st = moles(t, Y, x, W)) return st;
@@ -371,7 +417,7 @@ RB200_HD inline int tp(const ReactiveB200Table& t, double T, double p, const dou
         if (!r.liquid) return UNAVAILABLE;
         sel = 0;
     } else if (choice == GAS && !r.gas) return UNAVAILABLE;
-    if (const int st = trho(t, T, W / r.V[sel], Y, chem, s)) return st;
+    if (const int st = trhoMixed(t, T, W / r.V[sel], x, W, m, chem, s, kept)) return st;
     if (fabs(s.p - p) > 1e-7 * fmax(1.0, p)) return NONFINITE;
     s.p = p;
     if (choice == GAS && s.phase >= 0) return UNAVAILABLE;
