@@ -343,32 +343,44 @@ struct GasPass {
 };
 
 // SKIP_GAS and SKIP_LIQUID for a cell whose all-gas or all-liquid partition
-// provably cannot converge, so that its long hopeless solve is not run (most of a
-// saturated cell's evaluations: its density has no single-phase state, and the
-// (ln p, ln T) Newton halves its way through 70 steps before it gives up; on
-// 1,000,000 cells, 60% saturated, 133 of 155 phase evaluations a cell).
+// provably cannot become a stable candidate, so that its solve, often a long
+// hopeless one, is not run (most of a saturated cell's evaluations: its density
+// has no single-phase state, and the (ln p, ln T) Newton halves its way through 70
+// steps before it gives up; on 1,000,000 cells, 60% saturated, 133 of 155 phase
+// evaluations a cell).
 //
 // A converged partition has the cell's volume (to vtol) and energy (to etol of
 // max(1e5 q, q cp T)) on one root of the cubic, so it lies on the isochore V0 = W/q
-// at the temperature where u(T, V0) = e/q. That temperature is unique (cv =
-// R (cp/R - 1) + L T d2a > 0) and is found here by Newton, with no root in the way.
-// With x = dp/dV over R T/(V - b)^2 there:
-//   x > 0.1   the isochore is unstable there. A root needs x <= 0, a temperature
-//             10% off, where only an energy scale blown up by cp could accept it:
-//             etol cp T / cv >= 0.1 T asks for |x| of 1e-8 and below, and the
-//             pair of roots around such a point is 1e-8 of V apart, inside the cubic's
-//             near-repeated band (|disc| < 1e-14, |h| - |q| < 1e-10), which has
-//             no pair.
-//   x < -0.1  cp/cv is bounded, so the partition's temperature is this one to
-//             1e-6. It then fails where its pressure is out of range, where V0 is on
-//             the other side of the cubic's centre (below it, V0 is not the largest
-//             root, or the lone root's side is the liquid's; above it the
-//             reverse; both below the critical temperature), where the reported
-//             phase is the other one, or where the species' or the liquid's
-//             range excludes the temperature; each by a margin of 1e-3 or more
-//             (1e-6 for the temperature ranges).
-// In between, and where the Newton does not settle, nothing is skipped.
-__device__ __forceinline__ int singlePhaseImpossible(const GasPass& G, double q, double e, double gT) {
+// at a temperature T' with cv |T' - T| <= etol max(1e5, cp T'), T the isochore's own
+// temperature of the cell's energy: unique (cv = R (cp/R - 1) + L T d2a > 0) and
+// found here by Newton, with no root in the way. With x = dp/dV over R T/(V - b)^2,
+// cp/cv <= 1 + 10/|x|: either T' is T to 1e-5, or |x(T')| < 1e-3 and the root lies
+// on the edge of the spinodal, where cp lets the energy off.
+//
+// Below .985 of the critical temperature a root that close to the spinodal is no
+// stable candidate: the pressure there is off the saturation pressure by 0.5% at
+// least, and the affinity by thousands of mutol. (Nearer the critical point than
+// that, T' - T > .005 T takes |x(T')| < 1e-6, whose pair of roots lies inside the
+// cubic's near-repeated band, |disc| < 1e-14, which has no pair.) So with
+//   x > -1e-3    neither partition can be stable;
+//   otherwise    the partition's temperature is T to 1e-5, and
+//                p > psat    the gas is supersaturated, p < psat the liquid
+//                            superheated: the stability test's affinity and tangent
+//                            plane reject them (a pressure 1e-3 off is 5e-5 of RT or more
+//                            where the table holds, Z_g - Z_l >= .05),
+//                V0 < center V0 is not the largest root, or the lone root's side
+//                            is the liquid's; above it the reverse,
+//                rho, T      the reported phase is the other one, or the species'
+//                            or the liquid's range excludes the temperature,
+//                each by a margin of 1e-3 or more (1e-5 for the temperature ranges).
+// Nearer the critical temperature the spinodal's edge is left out by a wide margin
+// instead (|x| > .1: a T' on it would be 7% off, which takes cp/cv > 1e7 and a pair
+// of roots inside the near-repeated band), and saturation is not used. An isochore
+// whose temperature lies below Tmin by more than 1e-3 has no T' but on the
+// spinodal's edge either (T' >= Tmin takes cp/cv > 1e6): neither partition; that is
+// the colder half of the saturated cells. Where the Newton does not settle otherwise,
+// nothing is skipped.
+__device__ __forceinline__ int singlePhaseImpossible(const GasPass& G, const HemConst& C, double q, double e, double gT) {
     const PureSpecies& sp = G.gas;
     DensityTerms d;
     if (!isfinite(e) || !densityTerms(sp, q, d)) return 0;
@@ -379,12 +391,14 @@ __device__ __forceinline__ int singlePhaseImpossible(const GasPass& G, double q,
         if (!(T > 0) || !probeTerms(sp, d, T, g) || !probeEnergy(sp, d, g)) return 0;
         const double step = fma(d.iV, g.eM, -e) / __dmul_rn(d.iV, g.cvM);
         settled = fabs(step) <= 1e-8 * T;
+        if (T == G.Tmin && step > 1e-3 * T) return SKIP_GAS | SKIP_LIQUID;
         if (!settled) T = clampd(T - step, G.Tmin, G.Tmax);
     }
     if (!settled || !isfinite(g.p) || !isfinite(g.dpdV)) return 0;
     const double scale = g.RT * d.iv2, thermal = g.RT * d.iv;
-    if (g.dpdV > .1 * scale) return SKIP_GAS | SKIP_LIQUID;
-    if (!(g.dpdV < -.1 * scale)) return 0;
+    const bool cold = T < .985 * sp.Tc;
+    if (g.dpdV > (cold ? -1e-3 : .1) * scale) return SKIP_GAS | SKIP_LIQUID;
+    if (!cold && !(g.dpdV < -.1 * scale)) return 0;
     if (g.p < G.pmin - 1e-3 * thermal || g.p > G.pmax + 1e-3 * thermal) return SKIP_GAS | SKIP_LIQUID;
     if (!(g.p > 0)) return 0;
     int skip = 0;
@@ -398,11 +412,21 @@ __device__ __forceinline__ int singlePhaseImpossible(const GasPass& G, double q,
         if (q > 1.001 * rhoMid) skip |= SKIP_GAS;
         if (q < .999 * rhoMid) skip |= SKIP_LIQUID;
     }
-    if (G.enforceBounds && (T < G.gasTmin * (1 - 1e-6) || T > G.gasTmax * (1 + 1e-6))) skip |= SKIP_GAS;
-    if (T < G.liquidTmin * (1 - 1e-6) || T > G.liquidTc * (1 + 1e-6)) skip |= SKIP_LIQUID;
+    if (cold && C.satN > 4 && T >= C.satT0) {
+        // the table's pressures around T, one more cell out than its own
+        const int cell = int((T - C.satT0) * C.satInvStep);
+        if (cell >= 1 && cell + 2 < C.satN) {
+            const double below = C.satP[cell - 1], above = C.satP[cell + 2];
+            if (below > 0 && above > 0) {
+                if (g.p > above * (1 + 1e-3)) skip |= SKIP_GAS;
+                if (g.p < below * (1 - 1e-3)) skip |= SKIP_LIQUID;
+            }
+        }
+    }
+    if (G.enforceBounds && (T < G.gasTmin * (1 - 1e-5) || T > G.gasTmax * (1 + 1e-5))) skip |= SKIP_GAS;
+    if (T < G.liquidTmin * (1 - 1e-5) || T > G.liquidTc * (1 + 1e-5)) skip |= SKIP_LIQUID;
     return skip;
 }
-
 
 // The all-gas candidate of one cell where its whole solve and its stability test
 // take the short way: scalarGas' iterates (the same routines on the same
@@ -550,7 +574,7 @@ __global__ void __launch_bounds__(kGasThreads, RB200_GAS_MINBLOCKS) passGas(
             }
         }
         if (queue || other) {
-            x.skip |= singlePhaseImpossible(G, x.q, x.e, x.gT);
+            x.skip |= singlePhaseImpossible(G, C, x.q, x.e, x.gT);
             if (FROM_CONSERVED) {
                 x.gp = __ldcs(&seed[c].p);
                 x.gml = __ldcs(&seed[c].liquidMass[0]);
