@@ -1335,12 +1335,7 @@ std::string species(const ReactiveB200Table& t, PureSpecies& sp) {
         sp.polynomial[r] = g.polynomial;
         sp.regionMin[r] = g.minimumTemperature;
         for (int j = 0; j < 9; ++j) sp.coeff[r][j] = g.coefficient[j];
-        const double* a = g.coefficient;
-        const bool nine = g.polynomial == 9;
-        const double* c = a + (nine ? 2 : 0);
-        sp.powers[r] = NasaPowers{nine ? a[0] : 0.0, nine ? a[1] : 0.0, c[0], c[1], c[2], c[3], c[4],
-                                  c[1] / 2, c[2] / 3, c[3] / 4, c[4] / 5, nine ? a[7] : a[5],
-                                  c[2] / 2, c[3] / 3, c[4] / 4, nine ? a[8] : a[6]};
+        sp.powers[r] = nasaPowers(g.polynomial, g.coefficient);
     }
     sp.regionMaxLast = s.regions[s.regionCount - 1].maximumTemperature;
     sp.twoB = 2 * sp.b;

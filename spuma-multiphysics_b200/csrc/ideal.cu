@@ -25,79 +25,134 @@ namespace {
 constexpr int kIdealMaxSpecies = 4;
 
 struct IdealConst {
-    int ns;
+    int ns, logs;  // logs: some species' polynomials have the 1/T terms, which read ln T
     double r[kIdealMaxSpecies];  // R / W_k, J/(kg K)
     PureSpecies sp[kIdealMaxSpecies];
     double Tmin, Tmax, tol;
 };
 
-// Mixture e(T), cv(T), r and d cv / dT at mass fractions Y.
-__device__ inline void mixture(const IdealConst& G, const double* Y, double T, double& e, double& cv, double& r,
-                               double* cvSlope) {
-    e = cv = r = 0;
-    double slope = 0;
-    for (int k = 0; k < G.ns; ++k) {
-        double cpR, hRT, sR;
-        nasaEval(G.sp[k], T, cpR, hRT, sR);
-        e += Y[k] * G.r[k] * T * (hRT - 1);
-        cv += Y[k] * G.r[k] * (cpR - 1);
-        r += Y[k] * G.r[k];
-        if (cvSlope) {
-            // d cp/R / dT of the region's polynomial
-            const PureSpecies& s = G.sp[k];
-            const double* a = s.coeff[nasaRegion(s, T)];
-            const double iT = 1 / T;
-            const double d = s.polynomial[nasaRegion(s, T)] == 7
-                ? a[1] + 2 * a[2] * T + 3 * a[3] * T * T + 4 * a[4] * T * T * T
-                : -2 * a[0] * iT * iT * iT - a[1] * iT * iT + a[3] + 2 * a[4] * T + 3 * a[5] * T * T
-                      + 4 * a[6] * T * T * T;
-            slope += Y[k] * G.r[k] * d;
-        }
+// cp/R and h/RT of species k at T (iT = 1/T).
+__device__ __forceinline__ void speciesTerms(const PureSpecies& sp, double T, double iT, double& cpR, double& hRT) {
+    const NasaPowers& n = sp.powers[nasaRegion(sp, T)];
+    cpR = n.c0 + T * (n.c1 + T * (n.c2 + T * (n.c3 + T * n.c4)));
+    hRT = n.c0 + n.hc * iT + T * (n.h1 + T * (n.h2 + T * (n.h3 + T * n.h4)));
+    if (n.m1 != 0 || n.m2 != 0) {  // only these terms read ln T
+        cpR += (n.m2 * iT + n.m1) * iT;
+        hRT += (n.m1 * log(T) - n.m2 * iT) * iT;
     }
-    if (cvSlope) *cvSlope = slope;
+}
+
+// Energy residual F = rho e(T) - energy and rho cv(T) of the partial densities q
+// (qr: each times its gas constant), per volume. The formation energies are as large as
+// a hundred times rho cv dT of interest, so they meet the energy they cancel against
+// first, in fused multiply-adds of the unrounded partial densities.
+template <int NS>
+__device__ __forceinline__ void mixture(const IdealConst& G, const double* q, const double* qr, double energy, double T,
+                                        double& F, double& cv) {
+    double thermal = 0, iT = 0, lT = 0;
+    if (G.logs) {
+        iT = 1 / T;
+        lT = log(T);
+    }
+    F = -energy;
+    cv = 0;
+#pragma unroll
+    for (int k = 0; k < NS; ++k) {
+        const NasaPowers& n = G.sp[k].powers[nasaRegion(G.sp[k], T)];
+        F = fma(q[k], G.r[k] * n.hc, F);
+        thermal += qr[k] * (T * (n.c0 - 1 + T * (n.h1 + T * (n.h2 + T * (n.h3 + T * n.h4)))) + (n.m1 * lT - n.m2 * iT));
+        cv += qr[k] * (n.c0 - 1 + T * (n.c1 + T * (n.c2 + T * (n.c3 + T * n.c4))) + (n.m2 * iT + n.m1) * iT);
+    }
+    F += thermal;
 }
 
 __device__ inline bool inRange(const IdealConst& G, double T) { return T >= G.Tmin && T <= G.Tmax && T > 0; }
 
-__global__ void idealClosure(const IdealConst* __restrict__ Gp, const double* __restrict__ q, size_t stride,
-                             size_t count, const double* Tseed, double* Tout, ReactiveTransportState* transport,
-                             int* success) {
+// The reference's recovery of T from e(T) = e: bracket, then safeguarded Newton.
+template <int NS>
+__device__ bool bracketedT(const IdealConst& G, const double* q, const double* qr, double energy, double T0, double F0,
+                           double tolerance, double& T, double& cv, double& F) {
+    T = T0;
+    F = F0;
+    double lo = T, hi = T, fl = F0, fh = F0, radius = fmax(1., .01 * T);
+    for (int j = 0; j < 24 && fabs(F) > tolerance && (fl > 0 || fh < 0); ++j, radius *= 2) {
+        double slope;
+        if (fl > 0) { lo = fmax(G.Tmin, T0 - radius); mixture<NS>(G, q, qr, energy, lo, fl, slope); }
+        if (fh < 0) { hi = fmin(G.Tmax, T0 + radius); mixture<NS>(G, q, qr, energy, hi, fh, slope); }
+    }
+    bool ok = fabs(F) <= tolerance || (fl <= 0 && fh >= 0 && hi > lo);
+    for (int it = 0; ok && it < 70 && fabs(F) > tolerance; ++it) {
+        if (F > 0) hi = T; else lo = T;
+        const double next = T - F / cv;
+        T = isfinite(next) && next > lo && next < hi ? next : .5 * (lo + hi);
+        mixture<NS>(G, q, qr, energy, T, F, cv);
+    }
+    return ok && fabs(F) <= tolerance;
+}
+
+// Bound by the latency of the Newton's dependent FP64 chain (each e(T) needs the one
+// before it) and by issue. The bracket's probes only confine the Newton steps: e
+// rises with T (cv > 0), so the bracket that ends at the first widened radius past
+// the solution is known once the solution is, and steps that stayed inside it
+// are the steps the bracketed Newton takes. So the Newton runs first, and only a
+// step that left that bracket (or [Tmin, Tmax], or an iterate with cv <= 0)
+// goes back to the bracketed form. At the usual few per cent off the seed that
+// leaves four evaluations of seven to ten. The accepted iterate takes the Newton
+// step of the residual it was accepted with (within the tolerance, 4e-14 of T, no
+// further evaluation), so T is the solution to round-off and a smooth function of q.
+template <int NS>
+__global__ void __launch_bounds__(128) idealClosure(const IdealConst* __restrict__ Gp, const double* __restrict__ q,
+                                                    size_t stride, size_t count, const double* Tseed, double* Tout,
+                                                    ReactiveTransportState* transport, int* success) {
     const IdealConst& G = *Gp;
     for (size_t c = blockIdx.x * size_t(blockDim.x) + threadIdx.x; c < count; c += size_t(blockDim.x) * gridDim.x) {
-        double rho = 0, Y[kIdealMaxSpecies];
-        for (int k = 0; k < G.ns; ++k) rho += q[size_t(k) * stride + c];
-        for (int k = 0; k < G.ns; ++k) Y[k] = q[size_t(k) * stride + c] / rho;
-        const double mx = q[size_t(G.ns) * stride + c], my = q[size_t(G.ns + 1) * stride + c],
-                     mz = q[size_t(G.ns + 2) * stride + c], E = q[size_t(G.ns + 3) * stride + c];
-        const double eIn = (E - .5 * (mx * mx + my * my + mz * mz) / rho) / rho;
+        double rho = 0, y[NS], yr[NS], gas = 0;  // partial densities, times the gas constants, their sum
+#pragma unroll
+        for (int k = 0; k < NS; ++k) {
+            rho += y[k] = q[size_t(k) * stride + c];
+            gas += yr[k] = y[k] * G.r[k];
+        }
+        const double mx = q[size_t(NS) * stride + c], my = q[size_t(NS + 1) * stride + c],
+                     mz = q[size_t(NS + 2) * stride + c], E = q[size_t(NS + 3) * stride + c];
+        const double energy = E - .5 * (mx * mx + my * my + mz * mz) / rho;
         const double T0 = Tseed[c];
-        bool ok = isfinite(rho) && rho > 0 && isfinite(eIn) && inRange(G, T0);
-        double T = T0, e = 0, cv = 0, r = 0;
+        bool ok = isfinite(rho) && rho > 0 && isfinite(energy) && inRange(G, T0);
+        double T = T0, cv = 0;
         if (ok) {
-            mixture(G, Y, T, e, cv, r, nullptr);
-            const double tolerance = .25 * G.tol * fmax(1e5, (cv + r) * T);
-            double lo = T, hi = T, fl = e - eIn, fh = fl, F = fl, radius = fmax(1., .01 * T);
-            for (int j = 0; j < 24 && fabs(F) > tolerance && (fl > 0 || fh < 0); ++j, radius *= 2) {
-                double ee, cc, rr;
-                if (fl > 0) { lo = fmax(G.Tmin, T0 - radius); mixture(G, Y, lo, ee, cc, rr, nullptr); fl = ee - eIn; }
-                if (fh < 0) { hi = fmin(G.Tmax, T0 + radius); mixture(G, Y, hi, ee, cc, rr, nullptr); fh = ee - eIn; }
-            }
-            ok = fabs(F) <= tolerance || (fl <= 0 && fh >= 0 && hi > lo);
-            for (int it = 0; ok && it < 70 && fabs(F) > tolerance; ++it) {
+            double F;
+            mixture<NS>(G, y, yr, energy, T, F, cv);
+            const double tolerance = .25 * G.tol * fmax(1e5 * rho, (cv + gas) * T), F0 = F, cv0 = cv;
+            double lo = F0 > 0 ? G.Tmin : T0, hi = F0 > 0 ? T0 : G.Tmax, far = 0;
+            bool direct = cv > 0;
+            for (int it = 0; direct && it < 70 && fabs(F) > tolerance; ++it) {
                 if (F > 0) hi = T; else lo = T;
                 const double next = T - F / cv;
-                T = isfinite(next) && next > lo && next < hi ? next : .5 * (lo + hi);
-                mixture(G, Y, T, e, cv, r, nullptr);
-                F = e - eIn;
+                direct = next > lo && next < hi;
+                if (!direct) break;
+                T = next;
+                far = fmax(far, fabs(T - T0));
+                mixture<NS>(G, y, yr, energy, T, F, cv);
+                direct = cv > 0;
             }
-            ok = ok && fabs(F) <= tolerance && cv > 0;
+            if (direct) {
+                double radius = fmax(1., .01 * T0);
+                while (radius < fabs(T - T0)) radius *= 2;
+                direct = far < radius;
+                ok = fabs(F) <= tolerance;
+            }
+            if (!direct) {
+                cv = cv0;
+                ok = bracketedT<NS>(G, y, yr, energy, T0, F0, tolerance, T, cv, F);
+            }
+            ok = ok && cv > 0;
+            if (ok) T = fmin(fmax(T - F / cv, G.Tmin), G.Tmax);
         }
         if (success) success[c] = ok ? 1 : 0;
         if (!ok) continue;
-        const double p = rho * r * T;
-        const double sound = sqrt((cv + r) / cv * r * T);
+        const double p = gas * T, iRho = 1 / rho;
+        const double sound = sqrt((cv + gas) / cv * (p * iRho));
         Tout[c] = T;
-        transport[c] = ReactiveTransportState{p, T, rho, cv, sound, rho, 0.0};
+        transport[c] = ReactiveTransportState{p, T, rho, cv * iRho, sound, rho, 0.0};
     }
 }
 
@@ -126,15 +181,16 @@ __global__ void idealClosureVjp(const IdealConst* __restrict__ Gp, const double*
         const double T = Tconv[c];
         // species terms at the converged T (constants), mixed with dual Y
         D e(0.0), cv(0.0), r(0.0);
-        double cvSlope = 0, Yv[NS];
-#pragma unroll
-        for (int k = 0; k < NS; ++k) Yv[k] = Y[k].v;
-        double ev, cvv, rv;
-        mixture(G, Yv, T, ev, cvv, rv, &cvSlope);
+        double cvSlope = 0, cvv = 0;
+        const double iT = 1 / T;
 #pragma unroll
         for (int k = 0; k < NS; ++k) {
-            double cpR, hRT, sR;
-            nasaEval(G.sp[k], T, cpR, hRT, sR);
+            double cpR, hRT;
+            speciesTerms(G.sp[k], T, iT, cpR, hRT);
+            const NasaPowers& n = G.sp[k].powers[nasaRegion(G.sp[k], T)];
+            cvv += Y[k].v * G.r[k] * (cpR - 1);
+            cvSlope += Y[k].v * G.r[k] * (n.c1 + T * (2 * n.c2 + T * (3 * n.c3 + T * 4 * n.c4))
+                                          - (2 * n.m2 * iT + n.m1) * iT * iT);
             e += Y[k] * D(G.r[k] * T * (hRT - 1));
             cv += Y[k] * D(G.r[k] * (cpR - 1));
             r += Y[k] * D(G.r[k]);
@@ -183,7 +239,7 @@ std::string speciesFromTable(const ReactiveB200Species& s, PureSpecies& sp) {
             if (!std::isfinite(g.coefficient[j])) return "Invalid ideal-gas NASA coefficient";
         sp.polynomial[r] = g.polynomial;
         sp.regionMin[r] = g.minimumTemperature;
-        for (int j = 0; j < 9; ++j) sp.coeff[r][j] = g.coefficient[j];
+        sp.powers[r] = nasaPowers(g.polynomial, g.coefficient);
     }
     sp.regionMaxLast = s.regions[s.regionCount - 1].maximumTemperature;
     return "";
@@ -210,6 +266,7 @@ void* reactive_ideal_gas_create_v3(const void* table, size_t bytes, double Tmin,
         require(std::isfinite(tolerance) && tolerance > 0 && tolerance < 1, "Invalid closure tolerance");
         std::unique_ptr<IdealDevice> d(new IdealDevice);
         d->host.ns = t.ns;
+        d->host.logs = 0;
         d->host.Tmin = Tmin;
         d->host.Tmax = Tmax;
         d->host.tol = tolerance;
@@ -220,6 +277,8 @@ void* reactive_ideal_gas_create_v3(const void* table, size_t bytes, double Tmin,
                         && Tmax <= d->host.sp[k].regionMaxLast,
                     "Temperature range outside a species' NASA regions");
             d->host.r[k] = kGas / t.species[k].molecularWeight;
+            for (int r = 0; r < t.species[k].regionCount; ++r)
+                d->host.logs |= d->host.sp[k].powers[r].m1 != 0 || d->host.sp[k].powers[r].m2 != 0;
         }
         check(cudaGetDevice(&d->device), "cudaGetDevice");
         check(cudaMalloc(&d->dev, sizeof(IdealConst)), "cudaMalloc");
@@ -241,8 +300,14 @@ int reactive_ideal_gas_run_device_v3(void* gas, const double* q, size_t stride, 
         require(gas && q && Tseed && T && transport && count && stride >= count, "Invalid ideal-gas arguments");
         auto& d = *static_cast<IdealDevice*>(gas);
         require(variables == size_t(d.host.ns) + 4, "Ideal-gas closure needs variables = species + 4");
-        idealClosure<<<gridFor(count, 128), 128, 0, static_cast<cudaStream_t>(stream)>>>(d.dev, q, stride, count,
-                                                                                        Tseed, T, transport, success);
+        auto s = static_cast<cudaStream_t>(stream);
+        const unsigned grid = gridFor(count, 128);
+        switch (d.host.ns) {
+        case 1: idealClosure<1><<<grid, 128, 0, s>>>(d.dev, q, stride, count, Tseed, T, transport, success); break;
+        case 2: idealClosure<2><<<grid, 128, 0, s>>>(d.dev, q, stride, count, Tseed, T, transport, success); break;
+        case 3: idealClosure<3><<<grid, 128, 0, s>>>(d.dev, q, stride, count, Tseed, T, transport, success); break;
+        default: idealClosure<4><<<grid, 128, 0, s>>>(d.dev, q, stride, count, Tseed, T, transport, success); break;
+        }
         check(cudaGetLastError(), "idealClosure");
         return 0;
     } catch (const std::exception& e) {

@@ -48,6 +48,13 @@ struct NasaPowers {
     double m2, m1, c0, c1, c2, c3, c4, h1, h2, h3, h4, hc, s2, s3, s4, sc;
 };
 
+inline NasaPowers nasaPowers(int polynomial, const double* a) {
+    const bool nine = polynomial == 9;
+    const double* c = a + (nine ? 2 : 0);
+    return NasaPowers{nine ? a[0] : 0.0, nine ? a[1] : 0.0, c[0], c[1], c[2], c[3], c[4], c[1] / 2, c[2] / 3,
+                      c[3] / 4, c[4] / 5, nine ? a[7] : a[5], c[2] / 2, c[3] / 3, c[4] / 4, nine ? a[8] : a[6]};
+}
+
 // Immutable per-species constants, derived on the host from the model image.
 struct PureSpecies {
     double a, b, kappa, W, Tc, refP;
@@ -103,24 +110,6 @@ __device__ __forceinline__ void nasaEvalT(const PureSpecies& sp, double T, doubl
         sR = -.5 * c0 - c1 + lT * c2 + c3 + .5 * c4 + c5 * kThird + .25 * c6 + a[8];
     }
 }
-// NASA7/9 cp/R, h/RT, s/R at T (the ideal-gas closure's form).
-__device__ __forceinline__ void nasaEval(const PureSpecies& sp, double T, double& cpR, double& hRT, double& sR) {
-    const int r = nasaRegion(sp, T);
-    const double* a = sp.coeff[r];
-    const double T2 = T * T, T3 = T2 * T, T4 = T3 * T, iT = 1.0 / T, lT = log(T);
-    if (sp.polynomial[r] == 7) {
-        cpR = a[0] + a[1] * T + a[2] * T2 + a[3] * T3 + a[4] * T4;
-        hRT = a[0] + .5 * a[1] * T + a[2] * T2 / 3.0 + .25 * a[3] * T3 + .2 * a[4] * T4 + a[5] * iT;
-        sR = a[0] * lT + a[1] * T + .5 * a[2] * T2 + a[3] * T3 / 3.0 + .25 * a[4] * T4 + a[6];
-    } else {
-        const double c0 = a[0] * iT * iT, c1 = a[1] * iT, c2 = a[2], c3 = a[3] * T, c4 = a[4] * T2,
-                     c5 = a[5] * T3, c6 = a[6] * T4;
-        cpR = c0 + c1 + c2 + c3 + c4 + c5 + c6;
-        hRT = -c0 + lT * c1 + c2 + .5 * c3 + c4 / 3.0 + .25 * c5 + .2 * c6 + a[7] * iT;
-        sR = -.5 * c0 - c1 + lT * c2 + c3 + .5 * c4 + c5 / 3.0 + .25 * c6 + a[8];
-    }
-}
-
 __device__ __forceinline__ double cubicAt(double V, double bn, double cn, double dn) {
     return ((V + bn) * V + cn) * V + dn;
 }
