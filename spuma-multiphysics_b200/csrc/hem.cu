@@ -19,6 +19,7 @@
 #include "hem_flash.cuh"
 #include "hem_common.cuh"
 #include "hem_queue.cuh"
+#include "hem_two_phase.cuh"
 #include "hem_mixture.h"
 #include "common.cuh"
 #include "../../include/reactive_b200_hem.h"
@@ -319,6 +320,90 @@ __global__ void __launch_bounds__(kPassThreads, RB200_PASS_MINBLOCKS) passQueue(
         __syncwarp();
     }
     flushCounts(n, totals);
+}
+
+// The five two-phase candidates of every cell, or of list[0..counters[LIST]), of a
+// pure fluid: a persistent queue of (seed, cell) items, seed-major, whose lanes run
+// one solve each in registers and take the next item when it ends, so that all
+// lanes of a warp evaluate together whatever their solves' lengths. Bound by the
+// latency of the evaluations' FP64 chains.
+#ifndef RB200_TP_MINBLOCKS
+#define RB200_TP_MINBLOCKS 3
+#endif
+__global__ void __launch_bounds__(kPassThreads, RB200_TP_MINBLOCKS) passTwoPhase(const HemConst* __restrict__ Cp,
+                                                                                const __grid_constant__ PureSpecies sp,
+                                                                                const CellInput* __restrict__ in,
+                                                                                size_t count,
+                                                                                const unsigned* __restrict__ list,
+                                                                                CandRecord* rec, unsigned* counters,
+                                                                                unsigned long long* totals) {
+    const HemConst& C = *Cp;
+    Counts n;
+    const unsigned cells = list ? counters[LIST] : unsigned(count), total = 5u * cells, lane = threadIdx.x & 31u;
+    TwoPhaseSolve s;
+    TwoPhasePoint o;
+    CandRecord* record = nullptr;
+    bool active = false, exhausted = cells == 0;
+    for (;;) {
+        const unsigned need = __ballot_sync(0xffffffffu, !active && !exhausted);
+        if (need) {
+            unsigned base = 0;
+            if (lane == unsigned(__ffs(need) - 1)) base = atomicAdd(counters + Q_B, unsigned(__popc(need)));
+            base = __shfl_sync(0xffffffffu, base, __ffs(need) - 1);
+            if (!active && !exhausted) {
+                const unsigned item = base + __popc(need & ((1u << lane) - 1));
+                if (item < total) {
+                    const unsigned seed = item / cells, slot = item - seed * cells;
+                    const size_t c = list ? list[slot] : slot;
+                    record = rec + size_t(2 + seed) * count + c;
+                    record->status = 0;
+                    ++n.candidates;
+                    const CellInput x = in[c];
+                    if (x.skip & SKIP_TWO_PHASE) ++n.failures;  // outside every saturation tie line
+                    else {
+                        twoPhaseStart(C, x, kSeeds[seed], -1.0, s);
+                        active = true;
+                    }
+                } else exhausted = true;
+            }
+        }
+        if (!__any_sync(0xffffffffu, active)) {
+            if (__all_sync(0xffffffffu, exhausted)) break;
+            continue;
+        }
+        bool ok = false;
+        if (active) {
+            ++n.residuals;
+            n.phases += 2;
+            ok = twoPhasePoint(C, sp, s.q, s.e, s.scale, s.x0 + s.fraction * s.s0, s.x1 + s.fraction * s.s1,
+                               s.x2 + s.fraction * s.s2, o);
+        }
+        __syncwarp();
+        if (active) {
+            const int code = twoPhaseAdvance(C, sp, s, ok, o, n);
+            if (code != TP_RUNNING) {
+                active = false;
+                bool stable = false;
+                if (code == TP_CONVERGED && twoPhaseState(C, sp, s, o, record->st, record->entropyD, stable, n))
+                    record->status = stable ? 2 : 1;
+                if (stable) ++n.stable; else ++n.failures;
+            }
+        }
+        __syncwarp();
+    }
+    flushCounts(n, totals);
+}
+
+// The five two-phase candidates of the listed (or all) cells: in registers where one
+// species' tables serve both phases and the Jacobian is analytic, else through the
+// work queue.
+void launchSeeds(const HemConst& hostConst, const HemConst* cst, const CellInput* in, size_t count,
+                 const unsigned* cells, CandRecord* rec, unsigned* counters, unsigned long long* totals, int blocks,
+                 cudaStream_t s) {
+    if (hostConst.samePure && hostConst.analyticJacobian)
+        passTwoPhase<<<blocks, kPassThreads, 0, s>>>(cst, hostConst.gas, in, count, cells, rec, counters, totals);
+    else passQueue<<<blocks, kPassThreads, 0, s>>>(cst, in, count, cells, 2, 5, rec, counters, Q_B, totals);
+    check(cudaGetLastError(), "two-phase seeds");
 }
 
 __device__ __forceinline__ bool gasDecides(const HemConst& C, const CandRecord& gas) {
@@ -1110,8 +1195,7 @@ struct HemDevice {
             check(cudaGetLastError(), "passQueue");
             compactSeedCells<<<gridFor(count, 256), 256, 0, s>>>(cst, rec, count, list, counters);
             check(cudaGetLastError(), "compactSeedCells");
-            passQueue<<<passBlocks, kPassThreads, 0, s>>>(cst, in, count, list, 2, 5, rec, counters, Q_B, totals);
-            check(cudaGetLastError(), "passQueue");
+            launchSeeds(hostConst, cst, in, count, list, rec, counters, totals, passBlocks, s);
         } else if (hostConst.domeN) {
             // single-phase cells one thread each (selected and written there), the
             // rest through the work queue and the selection below
@@ -1126,11 +1210,13 @@ struct HemDevice {
             passSinglePhase<<<passBlocks, kPassThreads, 0, s>>>(cst, in, general, state, transport, success, fallback,
                                                                 counters, totals);
             check(cudaGetLastError(), "passSinglePhase");
-            passQueue<<<passBlocks, kPassThreads, 0, s>>>(cst, in, count, list, 0, 7, rec, counters, Q_A, totals);
+            passQueue<<<passBlocks, kPassThreads, 0, s>>>(cst, in, count, list, 0, 2, rec, counters, Q_A, totals);
             check(cudaGetLastError(), "passQueue");
+            launchSeeds(hostConst, cst, in, count, list, rec, counters, totals, passBlocks, s);
         } else {
-            passQueue<<<passBlocks, kPassThreads, 0, s>>>(cst, in, count, nullptr, 0, 7, rec, counters, Q_A, totals);
+            passQueue<<<passBlocks, kPassThreads, 0, s>>>(cst, in, count, nullptr, 0, 2, rec, counters, Q_A, totals);
             check(cudaGetLastError(), "passQueue");
+            launchSeeds(hostConst, cst, in, count, nullptr, rec, counters, totals, passBlocks, s);
         }
         selectCandidates<<<gridFor(count, 256), 256, 0, s>>>(cst, rec, count, selectList, state, transport, success,
                                                              fallback, counters);
@@ -2025,9 +2111,10 @@ extern "C" int reactive_gpu_hem_run_static_v3(const void* model, size_t modelByt
         if (hostConst.stableGasPrune) {
             passQueue<<<blocks, kPassThreads, 0, s>>>(cst, in, count, nullptr, 0, 2, rec, counters, Q_A, totals);
             compactSeedCells<<<gridFor(count, 256), 256, 0, s>>>(cst, rec, count, list, counters);
-            passQueue<<<blocks, kPassThreads, 0, s>>>(cst, in, count, list, 2, 5, rec, counters, Q_B, totals);
+            launchSeeds(hostConst, cst, in, count, list, rec, counters, totals, blocks, s);
         } else {
-            passQueue<<<blocks, kPassThreads, 0, s>>>(cst, in, count, nullptr, 0, 7, rec, counters, Q_A, totals);
+            passQueue<<<blocks, kPassThreads, 0, s>>>(cst, in, count, nullptr, 0, 2, rec, counters, Q_A, totals);
+            launchSeeds(hostConst, cst, in, count, nullptr, rec, counters, totals, blocks, s);
         }
         check(cudaGetLastError(), "passQueue");
         selectCandidates<<<gridFor(count, 256), 256, 0, s>>>(cst, rec, count, nullptr, state, transport, success,

@@ -1,12 +1,21 @@
-"""GPU: partitions that provably cannot become a stable candidate (an all-gas or
-all-liquid state of a cell inside the dome) are not solved: every bit of states and
-flags equals the exhaustive search's."""
+"""GPU: the pure-fluid search's passes that leave work out or rewrite it.
+
+* Partitions that provably cannot converge (an all-gas or all-liquid state of a
+  cell inside the dome) are not solved: every bit of states and flags equals the
+  exhaustive search's.
+* The two-phase candidates in registers (analytic Jacobian) against the general
+  evaluation of the one-thread-per-cell form and against the oracle flash.
+"""
 import numpy as np
 import pytest
+import torch
 
-from spuma_multiphysics_b200 import _abi as A, cases
+from oracle import oracle
+from spuma_multiphysics_b200 import _abi as A, cases, thermo_data as td
 from spuma_multiphysics_b200.eos import PureFluid
+from spuma_multiphysics_b200.hem import GpuHem
 from spuma_multiphysics_b200.thermo_data import N2O
+import flash_cases as F
 from test_two_phase_bound_gpu import assert_same, both
 
 pytestmark = pytest.mark.gpu
@@ -53,3 +62,35 @@ def test_skipped_partitions_change_no_bit(part):
     rho, e = np.ascontiguousarray(rho), np.ascontiguousarray(e)
     on, off = both(rho, e, guess)
     assert_same(on, off)
+
+
+# one cell, a warp's and a block's edges; liquid fractions from both ends of the tie line
+@pytest.mark.parametrize("n", [1, 31, 33, 129, 3000])
+@pytest.mark.parametrize("beta", [(0.0, 1.0), (1e-7, 1e-4), (1 - 1e-4, 1 - 1e-7)])
+def test_two_phase_candidates_equal_the_general_evaluation(n, beta):
+    rng = np.random.default_rng(7 * n + 1)
+    rho, e, guess = tie_line_states(rng.uniform(185.0, 306.0, n), rng.uniform(*beta, n))
+    guess["T"] += rng.uniform(-3.0, 3.0, n)
+    guess["p"] *= rng.uniform(.9, 1.1, n)
+    hem = GpuHem(capacity=n)
+    try:
+        cons = torch.zeros((5, n), dtype=torch.float64, device="cuda")
+        cons[0], cons[4] = torch.from_numpy(rho).cuda(), torch.from_numpy(e).cuda()
+        seed = torch.from_numpy(guess.view(np.uint8).copy()).cuda()
+        out = []
+        for per_cell in (False, True):
+            state, ok = torch.zeros_like(seed), torch.zeros(n, dtype=torch.int32, device="cuda")
+            hem.run_device(cons, n, n, 5, seed, state, None, ok, torch.cuda.current_stream().cuda_stream, per_cell)
+            torch.cuda.synchronize()
+            out.append((state.cpu().numpy().view(A.THERMO_DTYPE), ok.cpu().numpy()))
+    finally:
+        hem.close()
+    (got, ok), (general, general_ok) = out
+    ref, ref_ok, _ = F.oracle_flash(oracle, td.model_bytes(td.pure_model()), rho, e, guess)
+    for other, other_ok in ((general, general_ok), (ref, ref_ok)):
+        s = F.compare(got, ok, other, other_ok)
+        assert s["success_equal"] and s["label_mismatch"] == 0, s
+        # both stop at residuals below 1e-9: in the energy, of at most 2000 T per mass, which
+        # over cv > 1500 is 1.4e-9 of T each, and by Clausius-Clapeyron (h_fg W / RT < 13 from
+        # 185 K) 13 times that of p
+        assert s["p_rel"] <= 4e-8 and s["T_rel"] <= 3e-9 and s["ml_rel"] <= F.STATE_TOL, s
