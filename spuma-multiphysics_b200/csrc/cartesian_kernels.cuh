@@ -1823,14 +1823,4 @@ __global__ void cartGradientVjp(CartView v, const double* __restrict__ q, const 
     }
 }
 
-// out[k] = sum over blocks of partial[b*nv + k], one warp per variable, fixed order.
-__global__ void foldPartials(const double* __restrict__ partial, int blocks, int nv, double* out) {
-    const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (k >= nv) return;
-    double s = 0;
-    for (int b = lane; b < blocks; b += 32) s += partial[size_t(b) * nv + k];
-    s = warpSum(s);
-    if (lane == 0) out[k] = s;
-}
-
 }  // namespace rb200

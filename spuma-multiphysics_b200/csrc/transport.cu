@@ -286,6 +286,7 @@ struct Transport {
         v.faces = cfg.faces; v.nBoundary = boundary.size(); v.mechanical = cfg.mechanical;
         v.viscosity = cfg.viscosity; v.conductivity = cfg.conductivity; v.diffusivity = cfg.diffusivity;
         v.waveFactor = cfg.waveFactor;
+        v.fluxes = !cfg.mechanical && cfg.variables <= FW_FIELDS;
         v.face = faceDevice; v.row = rowDevice; v.incidence = incidenceDevice; v.boundary = boundaryDevice;
         v.invV = invDevice; v.state = stateDevice; v.q = q; v.primitive = primitive; v.grad = grad;
         v.gasY = gasY; v.gasH = gasH; v.work = work; v.carrier = carrier; v.faceSpeed = faceSpeed; v.step = step;
@@ -420,8 +421,9 @@ struct Transport {
         finish();
         require(!status, "Invalid WALE gradient/filter width/eddy viscosity");
     }
-    // Face work (+ gradients) for one flux evaluation on device data.
-    void launchFaces(const double* qSoA, const ReactiveTransportState* state, cudaStream_t s) {
+    // Face work (+ gradients) for one flux evaluation on device data; speeds: also
+    // the face speeds of the CFL query on the same state.
+    void launchFaces(const double* qSoA, const ReactiveTransportState* state, cudaStream_t s, bool speeds = false) {
         GraphView g = v;
         g.q = qSoA;
         g.state = state;
@@ -430,22 +432,44 @@ struct Transport {
             cellGradients<<<gridFor(v.cells, 256), 256, 0, s>>>(g);
             launched();
         }
-        faceWork<<<gridFor(v.faces, 128), 128, 0, s>>>(g);
+        faceWork<<<gridFor(v.faces, 128), 128, 0, s>>>(g, speeds);
         launched();
         ++deviceProfile.transportFaceLaunches;
     }
+    // result (finished fluxes only): also the CFL step of the face speeds.
     void launchRates(const double* qSoA, const ReactiveTransportState* state, double* out, size_t stride,
-                     int mode, double dt, cudaStream_t s) {
+                     int mode, double dt, cudaStream_t s, double cfl = 0, double maximumStep = 0,
+                     double* result = nullptr) {
         GraphView g = v;
         g.q = qSoA;
         g.state = state;
-        cellRates<8><<<gridFor(v.cells, 128), 128, 0, s>>>(g, out, stride, mode, dt);
+        if (!v.fluxes) {
+            cellRates<8><<<gridFor(v.cells, 128), 128, 0, s>>>(g, out, stride, mode, dt);
+            launched();
+            return;
+        }
+        const unsigned blocks = result ? unsigned(reduceBlocks) : gridFor(v.cells, 256);
+        cellRatesFromFluxes<8><<<blocks, 256, 0, s>>>(g, out, stride, mode, dt, result ? cfl : 0.0, maximumStep,
+                                                      reduceScratch);
         launched();
+        if (result) {
+            minimumReduce<<<1, 1024, 0, s>>>(reduceScratch, blocks, result);
+            launched();
+        }
     }
     void launchLedger(const double* qSoA, const ReactiveTransportState* state, double* rate, cudaStream_t s) {
         GraphView g = v;
         g.q = qSoA;
         g.state = state;
+        // partials of the finished fluxes in the CFL reduction's scratch
+        const size_t blocks = std::min<size_t>((v.nBoundary + 255) / 256, reduceBlocks / cfg.variables);
+        if (v.fluxes && blocks > 1) {
+            boundaryLedgerPartials<<<unsigned(blocks), 256, 0, s>>>(g, reduceScratch);
+            launched();
+            foldPartials<<<1, 32 * unsigned(cfg.variables), 0, s>>>(reduceScratch, int(blocks), int(cfg.variables), rate);
+            launched();
+            return;
+        }
         boundaryLedger<<<unsigned(cfg.variables), 256, 0, s>>>(g, rate);
         launched();
     }
@@ -895,7 +919,7 @@ struct Transport {
                 launched();
             }
             if (v.capillary) check(cudaMemsetAsync(flags, 0, sizeof(unsigned), stream), "memset");
-            faceWork<<<gridFor(v.faces, 128), 128, 0, stream>>>(g);
+            faceWork<<<gridFor(v.faces, 128), 128, 0, stream>>>(g, false);
             launched();
             ++deviceProfile.transportFaceLaunches;
             if (v.wale || v.capillary) {
