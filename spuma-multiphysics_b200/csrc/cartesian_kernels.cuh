@@ -30,12 +30,18 @@ constexpr int kCartMaxNs = 4;
 struct CartView {
     int nx, ny, nz;
     size_t cells, fixed, all;
-    double area[3], dist[3];      // internal faces per axis (ownerWeight 0.5)
+    double area[3], dist[3], invDist[3];  // internal faces per axis (ownerWeight 0.5)
     const double* invV;
     const ReactiveTransportFace* face;
     size_t sideBase[6];           // -x,+x,-y,+y,-z,+z: first face of the side block
     size_t boundaryBase, nBoundary;
-    const ReactiveTransportPrimitive* primitive;  // cells + fixed (velocities, as the face-graph kernels use)
+    // a cell's flux inputs, SoA, written by cartInputs before any other kernel of an
+    // entry: velocity, p, T, rho, frozen sound, 1/rho and 1/(rho cv); the fixed
+    // states' come from the arrays they are given in
+    struct Inputs {
+        double *u[3], *p, *T, *rho, *c, *irho, *ircv;
+    } in;
+    ReactiveTransportPrimitive* primitive;  // cells + fixed
     double viscosity, conductivity, waveFactor;
     bool wale;
     double cw;
@@ -43,7 +49,7 @@ struct CartView {
     // WALE scalar closure: turbulent Prandtl / Schmidt numbers (0 disables a
     // term), mixture cp (all) and effective species enthalpies (SoA ns x all)
     bool sgs;
-    double pr, sc;
+    double pr, sc, invPr, invSc;
     const double* mixCp;
     const double* spH;
     // cells [ownBegin, ownEnd) are this handle's own: the stage update, the CFL
@@ -60,7 +66,8 @@ struct CartView {
 struct CellData {
     double q[kCartMaxNs + 4];
     double u[3];
-    double p, T, rho, cv, c;
+    double p, T, rho, c;
+    double irho, ircv;         // 1/rho and 1/(rho cv): the CFL speeds' diffusivities
     double cp, h[kCartMaxNs];  // WALE scalar closure only
 };
 
@@ -69,7 +76,7 @@ struct CellData {
 template <class R> struct CellT {
     R q[kCartMaxNs + 4];
     R u[3];
-    R p, T, rho, cv, c;
+    R p, T, rho, c;
     R cp, h[kCartMaxNs];  // WALE scalar closure only
 };
 template <int NS, class R, bool SGS = false> __device__ __forceinline__ CellT<R> asCell(const CellData& d) {
@@ -78,7 +85,7 @@ template <int NS, class R, bool SGS = false> __device__ __forceinline__ CellT<R>
     for (int k = 0; k < NS + 4; ++k) r.q[k] = R(d.q[k]);
 #pragma unroll
     for (int a = 0; a < 3; ++a) r.u[a] = R(d.u[a]);
-    r.p = R(d.p); r.T = R(d.T); r.rho = R(d.rho); r.cv = R(d.cv); r.c = R(d.c);
+    r.p = R(d.p); r.T = R(d.T); r.rho = R(d.rho); r.c = R(d.c);
     if constexpr (SGS) {
         r.cp = R(d.cp);
 #pragma unroll
@@ -87,26 +94,74 @@ template <int NS, class R, bool SGS = false> __device__ __forceinline__ CellT<R>
     return r;
 }
 
-// SGS: also the cell's mixture cp (when Pr_t > 0) and, with its conserved
-// variables, its species enthalpies (when Sc_t > 0).
+// The cells' flux inputs (CartView::Inputs) from the conserved rows and the
+// states, with fromPrimitive the velocities from the caller's primitives instead.
+// The stage kernels read a cell's inputs up to seven times: as SoA their loads
+// coalesce (the 56-byte states and 32-byte primitives cost a warp 70 and 16
+// wavefronts a cell where these cost two a field), and the two reciprocals
+// replace five divisions a face of the CFL speed.
+__global__ void __launch_bounds__(256) cartInputs(CartView v, const double* __restrict__ q,
+                                                  const ReactiveTransportState* __restrict__ st, int ns,
+                                                  bool fromPrimitive) {
+    for (size_t c = blockIdx.x * size_t(blockDim.x) + threadIdx.x; c < v.all; c += size_t(blockDim.x) * gridDim.x) {
+        ReactiveTransportPrimitive p{};
+        if (fromPrimitive) p = v.primitive[c];
+        else {
+            for (int k = 0; k < ns; ++k) p.rho += q[size_t(k) * v.all + c];
+            for (int d = 0; d < 3; ++d) p.u[d] = q[size_t(ns + d) * v.all + c] / p.rho;
+        }
+        if (c >= v.cells) {
+            v.primitive[c] = p;
+            continue;
+        }
+        const ReactiveTransportState s = st[c];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) v.in.u[d][c] = p.u[d];
+        v.in.p[c] = s.p;
+        v.in.T[c] = s.T;
+        v.in.rho[c] = s.rho;
+        v.in.c[c] = s.sound;
+        v.in.irho[c] = 1 / s.rho;
+        v.in.ircv[c] = 1 / (s.rho * s.cv);
+    }
+}
+
+// Entry e (a cell, or cells + a fixed state). SGS: also its mixture cp (when
+// Pr_t > 0) and, with its conserved variables, its species enthalpies (when Sc_t > 0).
 template <int NS, bool SGS = false>
-__device__ __forceinline__ void loadCell(const CartView& v, const double* __restrict__ q,
-                                         const ReactiveTransportState* __restrict__ st, size_t c, CellData& d,
-                                         bool needQ) {
+__device__ __forceinline__ void loadShared(const CartView& v, const double* __restrict__ q, size_t e, CellData& d,
+                                           bool needQ) {
     if (needQ) {
 #pragma unroll
-        for (int k = 0; k < NS + 4; ++k) d.q[k] = q[size_t(k) * v.all + c];
+        for (int k = 0; k < NS + 4; ++k) d.q[k] = q[size_t(k) * v.all + e];
     }
     if constexpr (SGS) {
-        d.cp = v.pr > 0 ? v.mixCp[c] : 0.0;
+        d.cp = v.pr > 0 ? v.mixCp[e] : 0.0;
 #pragma unroll
-        for (int k = 0; k < NS; ++k) d.h[k] = needQ && v.sc > 0 ? v.spH[size_t(k) * v.all + c] : 0.0;
+        for (int k = 0; k < NS; ++k) d.h[k] = needQ && v.sc > 0 ? v.spH[size_t(k) * v.all + e] : 0.0;
     }
-    const ReactiveTransportPrimitive pr = v.primitive[c];
+}
+template <int NS, bool SGS = false>
+__device__ __forceinline__ void loadCell(const CartView& v, const double* __restrict__ q, size_t c, CellData& d,
+                                         bool needQ) {
+    loadShared<NS, SGS>(v, q, c, d, needQ);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) d.u[a] = v.in.u[a][c];
+    d.p = v.in.p[c]; d.T = v.in.T[c]; d.rho = v.in.rho[c]; d.c = v.in.c[c];
+    d.irho = v.in.irho[c]; d.ircv = v.in.ircv[c];
+}
+template <int NS, bool SGS = false>
+__device__ __forceinline__ void loadFixed(const CartView& v, const double* __restrict__ q,
+                                          const ReactiveTransportState* __restrict__ st, size_t fixed, CellData& d,
+                                          bool needQ) {
+    const size_t e = v.cells + fixed;
+    loadShared<NS, SGS>(v, q, e, d, needQ);
+    const ReactiveTransportPrimitive pr = v.primitive[e];
 #pragma unroll
     for (int a = 0; a < 3; ++a) d.u[a] = pr.u[a];
-    const ReactiveTransportState s = st[c];
-    d.p = s.p; d.T = s.T; d.rho = s.rho; d.cv = s.cv; d.c = s.sound;
+    const ReactiveTransportState s = st[e];
+    d.p = s.p; d.T = s.T; d.rho = s.rho; d.c = s.sound;
+    d.irho = 1 / s.rho; d.ircv = 1 / (s.rho * s.cv);
 }
 
 // Right state of a boundary face of kind 1 (slip: velocity and momentum
@@ -117,7 +172,7 @@ __device__ __forceinline__ void boundaryRight(const CartView& v, const double* _
                                               const ReactiveTransportFace& f, int axis, const CellData& L,
                                               CellData& R, bool needQ) {
     if (f.kind == 3) {
-        loadCell<NS, SGS>(v, q, st, v.cells + size_t(f.fixed), R, needQ);
+        loadFixed<NS, SGS>(v, q, st, size_t(f.fixed), R, needQ);
         return;
     }
     R = L;
@@ -152,11 +207,11 @@ __device__ __forceinline__ void twoSum(float& s, float& c, float x) {
 // its enthalpy flux, in the face graph's operation order
 // (src/reactiveTransport/reactiveTransportKernels.h:150-168, :440-477).
 template <int NS, class R, bool SGS = false>
-__device__ __forceinline__ void faceFluxCart(const CartView& v, int axis, double sgnD, double areaD, double distD,
+__device__ __forceinline__ void faceFluxCart(const CartView& v, int axis, double sgnD, double areaD, double invDistD,
                                              double wD, int kind, bool internal, const CellT<R>& L,
                                              const CellT<R>& Rt, const R* gL, const R* gR, R nutL, R nutR, R* F,
                                              bool& bad, bool& faceBad) {
-    const R sgn = R(sgnD), w = R(wD), dist = R(distD), area = R(areaD);
+    const R sgn = R(sgnD), w = R(wD), invDist = R(invDistD), area = R(areaD);
     const R unL = L.u[axis] * sgn, unR = Rt.u[axis] * sgn;
     const R aL = R(v.waveFactor) * L.c, aR = R(v.waveFactor) * Rt.c;
     const R left = rmin(R(0), rmin(unL - aL, unR - aR)), right = rmax(R(0), rmax(unL + aL, unR + aR));
@@ -211,7 +266,7 @@ __device__ __forceinline__ void faceFluxCart(const CartView& v, int axis, double
             R normal = R(0);
 #pragma unroll
             for (int d = 0; d < 3; ++d) normal += g[i * 3 + d] * nrm(d, axis, sgn);
-            const R target = (uR[i] - uL[i]) / (R(kind == 1 ? 2 : 1) * dist);
+            const R target = (uR[i] - uL[i]) * (R(kind == 1 ? .5 : 1.0) * invDist);
 #pragma unroll
             for (int d = 0; d < 3; ++d) g[i * 3 + d] += nrm(d, axis, sgn) * (target - normal);
         }
@@ -221,7 +276,7 @@ __device__ __forceinline__ void faceFluxCart(const CartView& v, int axis, double
         for (int i = 0; i < 3; ++i)
 #pragma unroll
             for (int d = 0; d < 3; ++d)
-                traction[i] += mu * (g[3 * i + d] + g[3 * d + i] - (i == d ? R(2) * div / R(3) : R(0)))
+                traction[i] += mu * (g[3 * i + d] + g[3 * d + i] - (i == d ? div * R(2.0 / 3.0) : R(0)))
                     * nrm(d, axis, sgn);
         if (kind == 1) {
             R dot = R(0);
@@ -233,7 +288,7 @@ __device__ __forceinline__ void faceFluxCart(const CartView& v, int axis, double
 #pragma unroll
         for (int d = 0; d < 3; ++d) energy -= traction[d] * (w * uL[d] + (R(1) - w) * uR[d]);
     }
-    if (v.conductivity > 0 && kind != 1) energy -= R(v.conductivity) * (Rt.T - L.T) / dist;
+    if (v.conductivity > 0 && kind != 1) energy -= R(v.conductivity) * (Rt.T - L.T) * invDist;
     R sgsJ[NS], sgsD = R(0), sgsSum = R(0), sgsCarrierFlux = R(0);
 #pragma unroll
     for (int k = 0; k < NS; ++k) sgsJ[k] = R(0);
@@ -241,11 +296,11 @@ __device__ __forceinline__ void faceFluxCart(const CartView& v, int axis, double
         if (v.pr > 0 && kind != 1) {
             const R rhoNut = w * L.rho * nutL + (R(1) - w) * Rt.rho * nutR;
             const R cp = w * L.cp + (R(1) - w) * Rt.cp;
-            energy -= rhoNut * cp / R(v.pr) * (Rt.T - L.T) / dist;
+            energy -= rhoNut * cp * R(v.invPr) * (Rt.T - L.T) * invDist;
         }
         if (v.sc > 0 && kind != 1) {
             const R rhoNut = w * L.rho * nutL + (R(1) - w) * Rt.rho * nutR;
-            sgsD = -rhoNut / R(v.sc) / dist;
+            sgsD = -rhoNut * R(v.invSc) * invDist;
             R largest = R(-1), yL[NS], yR[NS];
             int carrier = 0;
 #pragma unroll
@@ -338,7 +393,7 @@ __global__ void __launch_bounds__(256) cartGradients(CartView v, const ReactiveT
         int i, j, k;
         cellCoords(v, c, i, j, k);
         CellData C;
-        loadCell<NS>(v, nullptr, st, c, C, false);
+        loadCell<NS>(v, nullptr, c, C, false);
         R g[9] = {R(0), R(0), R(0), R(0), R(0), R(0), R(0), R(0), R(0)};
         const R iv = R(v.invV[c]);
 #pragma unroll
@@ -351,12 +406,12 @@ __global__ void __launch_bounds__(256) cartGradients(CartView v, const ReactiveT
             if (interior) {
                 // internal face: owner is the lower cell, normal +e_axis; this cell's
                 // incidence sign is +1 on its upper side (owner), -1 on its lower side
-                const ReactiveTransportPrimitive pn = v.primitive[neighbourOf(v, s, c)];
+                const size_t nb = neighbourOf(v, s, c);
                 const bool owner = s & 1;
 #pragma unroll
                 for (int a = 0; a < 3; ++a)
-                    uf[a] = owner ? R(.5) * R(C.u[a]) + (R(1) - R(.5)) * R(pn.u[a])
-                                  : R(.5) * R(pn.u[a]) + (R(1) - R(.5)) * R(C.u[a]);
+                    uf[a] = owner ? R(.5) * R(C.u[a]) + (R(1) - R(.5)) * R(v.in.u[a][nb])
+                                  : R(.5) * R(v.in.u[a][nb]) + (R(1) - R(.5)) * R(C.u[a]);
                 scale = R(owner ? 1.0 : -1.0) * R(v.area[axis]) * iv;
                 sgn = R(1);
             } else {
@@ -400,7 +455,7 @@ __device__ __forceinline__ void sideFlux(const CartView& v, const double* __rest
     if (interior) {
         const size_t nb = neighbourOf(v, s, c);
         CellData N;
-        loadCell<NS, SGS>(v, q, st, nb, N, true);
+        loadCell<NS, SGS>(v, q, nb, N, true);
         R gN[9] = {R(0), R(0), R(0), R(0), R(0), R(0), R(0), R(0), R(0)};
         if (viscous) {
 #pragma unroll
@@ -409,11 +464,11 @@ __device__ __forceinline__ void sideFlux(const CartView& v, const double* __rest
         const R nutN = v.wale ? nut[nb] : R(0);
         const CellT<R> cc = asCell<NS, R, SGS>(C), cn = asCell<NS, R, SGS>(N);
         if (s & 1) {  // this cell owns the face
-            faceFluxCart<NS, R, SGS>(v, axis, 1.0, v.area[axis], v.dist[axis], .5, 0, true, cc, cn, gC, gN, nutC,
+            faceFluxCart<NS, R, SGS>(v, axis, 1.0, v.area[axis], v.invDist[axis], .5, 0, true, cc, cn, gC, gN, nutC,
                                      nutN, F, bad, faceBad);
             sign = -1;
         } else {
-            faceFluxCart<NS, R, SGS>(v, axis, 1.0, v.area[axis], v.dist[axis], .5, 0, true, cn, cc, gN, gC, nutN,
+            faceFluxCart<NS, R, SGS>(v, axis, 1.0, v.area[axis], v.invDist[axis], .5, 0, true, cn, cc, gN, gC, nutN,
                                      nutC, F, bad, faceBad);
             sign = 1;
         }
@@ -422,7 +477,7 @@ __device__ __forceinline__ void sideFlux(const CartView& v, const double* __rest
         CellData Rt;
         boundaryRight<NS, SGS>(v, q, st, f, axis, C, Rt, true);
         // a boundary face's right-side WALE viscosity is the owner's
-        faceFluxCart<NS, R, SGS>(v, axis, (s & 1) ? 1.0 : -1.0, f.area, f.distance, f.ownerWeight, f.kind, false,
+        faceFluxCart<NS, R, SGS>(v, axis, (s & 1) ? 1.0 : -1.0, f.area, 1 / f.distance, f.ownerWeight, f.kind, false,
                                  asCell<NS, R, SGS>(C), asCell<NS, R, SGS>(Rt), gC, gC, nutC, nutC, F, bad, faceBad);
         sign = -1;
     }
@@ -449,7 +504,7 @@ __global__ void __launch_bounds__(128) cartRates(CartView v, const double* __res
         int i, j, k;
         cellCoords(v, c, i, j, k);
         CellData C;
-        loadCell<NS, SGS>(v, q, st, c, C, true);
+        loadCell<NS, SGS>(v, q, c, C, true);
         R gC[9] = {R(0), R(0), R(0), R(0), R(0), R(0), R(0), R(0), R(0)};
         if (viscous) {
 #pragma unroll
@@ -501,7 +556,7 @@ __global__ void __launch_bounds__(128) cartRates(CartView v, const double* __res
 // and FP32 faces with the compensated sums continued in the same order).
 // (defined with the CFL kernels below)
 template <bool SGS = false>
-__device__ __forceinline__ double faceSpeedCart(const CartView& v, int axis, double sgn, double dist, double w,
+__device__ __forceinline__ double faceSpeedCart(const CartView& v, int axis, double sgn, double invDist, double w,
                                                 int kind, const CellData& L, const CellData& R, double nutL,
                                                 double nutR);
 
@@ -569,7 +624,7 @@ __global__ void __launch_bounds__(128, RB200_FACE_MINBLOCKS) cartFaceFluxes(Cart
         }
         if (!any) continue;
         CellData C;
-        loadCell<NS, SGS>(v, q, st, c, C, true);
+        loadCell<NS, SGS>(v, q, c, C, true);
         R gC[9] = {R(0), R(0), R(0), R(0), R(0), R(0), R(0), R(0), R(0)};
         if (viscous) {
 #pragma unroll
@@ -585,7 +640,7 @@ __global__ void __launch_bounds__(128, RB200_FACE_MINBLOCKS) cartFaceFluxes(Cart
             const size_t nb = neighbourOf(v, s, c);
             if (!ownC && !(nb >= v.ownBegin && nb < v.ownEnd)) continue;
             CellData N;
-            loadCell<NS, SGS>(v, q, st, nb, N, true);
+            loadCell<NS, SGS>(v, q, nb, N, true);
             R gN[9] = {R(0), R(0), R(0), R(0), R(0), R(0), R(0), R(0), R(0)};
             if (viscous) {
 #pragma unroll
@@ -593,13 +648,13 @@ __global__ void __launch_bounds__(128, RB200_FACE_MINBLOCKS) cartFaceFluxes(Cart
             }
             const R nutN = v.wale ? nut[nb] : R(0);
             R F[NQ];
-            faceFluxCart<NS, R, SGS>(v, axis, 1.0, v.area[axis], v.dist[axis], .5, 0, true, cc,
+            faceFluxCart<NS, R, SGS>(v, axis, 1.0, v.area[axis], v.invDist[axis], .5, 0, true, cc,
                                      asCell<NS, R, SGS>(N), gC, gN, nutC, nutN, F, bad, faceBad);
 #pragma unroll
             for (int kk = 0; kk < NQ; ++kk) flux[(size_t(axis) * NQ + kk) * v.cells + c] = F[kk];
             if (cflPass)
                 v.faceFlux[splitSpeedOffset(NQ, v.cells) + size_t(axis) * v.cells + c] =
-                    faceSpeedCart<SGS>(v, axis, 1.0, v.dist[axis], .5, 0, C, N, double(nutC), double(nutN));
+                    faceSpeedCart<SGS>(v, axis, 1.0, v.invDist[axis], .5, 0, C, N, double(nutC), double(nutN));
         }
         if (bad) atomicOr(error, 1u);
         if (faceBad) atomicOr(error, 2u);
@@ -742,7 +797,7 @@ __global__ void __launch_bounds__(128) cartRatesBoxSides(CartView v, const doubl
         cellCoords(v, c, i, j, k);
         if (!(i == 0 || i + 1 == v.nx || j == 0 || j + 1 == v.ny || k == 0 || k + 1 == v.nz)) continue;
         CellData C;
-        loadCell<NS, SGS>(v, q, st, c, C, true);
+        loadCell<NS, SGS>(v, q, c, C, true);
         R gC[9] = {R(0), R(0), R(0), R(0), R(0), R(0), R(0), R(0), R(0)};
         if (viscous) {
 #pragma unroll
@@ -781,7 +836,7 @@ __global__ void __launch_bounds__(128) cartRatesBoxSides(CartView v, const doubl
                 const ReactiveTransportFace& f = sideFace(v, s, i, j, k);
                 CellData Rt;
                 boundaryRight<NS, SGS>(v, nullptr, st, f, axis, C, Rt, false);
-                const double sp = faceSpeedCart<SGS>(v, axis, (s & 1) ? 1.0 : -1.0, f.distance, f.ownerWeight,
+                const double sp = faceSpeedCart<SGS>(v, axis, (s & 1) ? 1.0 : -1.0, 1 / f.distance, f.ownerWeight,
                                                      f.kind, C, Rt, double(nutC), double(nutC));
                 if (!isfinite(sp) || sp < 0) badSpeed = true;
                 else denominator += f.area * sp;
@@ -842,7 +897,7 @@ __device__ __forceinline__ void stageTileCell(const CartView& v, const double* _
     using Lay = TileLayout<NS, SGS>;
     constexpr int S = Lay::SLOTS;
     CellData d;
-    loadCell<NS, SGS>(v, q, st, c, d, true);
+    loadCell<NS, SGS>(v, q, c, d, true);
     const CellT<R> t = asCell<NS, R, SGS>(d);
 #pragma unroll
     for (int k = 0; k < Lay::NQ; ++k) plane[(Lay::Q + k) * S + slot] = t.q[k];
@@ -874,7 +929,6 @@ __device__ __forceinline__ void tileCell(const R* plane, int slot, CellT<R>& t, 
     t.T = plane[Lay::T * S + slot];
     t.rho = plane[Lay::RHO * S + slot];
     t.c = plane[Lay::C * S + slot];
-    t.cv = R(0);
     if constexpr (SGS) {
         t.cp = plane[Lay::CP * S + slot];
 #pragma unroll
@@ -893,7 +947,7 @@ __device__ __forceinline__ void globalCell(const CartView& v, const double* __re
                                            const R* __restrict__ nut, size_t c, bool viscous, CellT<R>& t, R* g,
                                            R& nu) {
     CellData d;
-    loadCell<NS, SGS>(v, q, st, c, d, true);
+    loadCell<NS, SGS>(v, q, c, d, true);
     t = asCell<NS, R, SGS>(d);
 #pragma unroll
     for (int j = 0; j < 9; ++j) g[j] = viscous ? grad[size_t(j) * v.cells + c] : R(0);
@@ -935,7 +989,7 @@ __global__ void __launch_bounds__(kTileX * kTileY, RB200_TILE_MINBLOCKS) cartRat
         R gl[9], gh[9], nl, nh;
         globalCell<NS, R, SGS>(v, q, st, grad, nut, cellAt(gx, gy, z0 - 1), viscous, lo, gl, nl);
         globalCell<NS, R, SGS>(v, q, st, grad, nut, cellAt(gx, gy, z0), viscous, hi, gh, nh);
-        faceFluxCart<NS, R, SGS>(v, 2, 1.0, v.area[2], v.dist[2], .5, 0, true, lo, hi, gl, gh, nl, nh, down, bad,
+        faceFluxCart<NS, R, SGS>(v, 2, 1.0, v.area[2], v.invDist[2], .5, 0, true, lo, hi, gl, gh, nl, nh, down, bad,
                                  faceBad);
     }
     for (int z = z0; z < z1; ++z) {
@@ -977,7 +1031,7 @@ __global__ void __launch_bounds__(kTileX * kTileY, RB200_TILE_MINBLOCKS) cartRat
             tileCell<NS, R, SGS>(plane, (by + 1) * PX + bx + 1, Rt, gR, nR);
             R flux[NQ];
             const int axis = xFace ? 0 : 1;
-            faceFluxCart<NS, R, SGS>(v, axis, 1.0, v.area[axis], v.dist[axis], .5, 0, true, L, Rt, gL, gR, nL, nR,
+            faceFluxCart<NS, R, SGS>(v, axis, 1.0, v.area[axis], v.invDist[axis], .5, 0, true, L, Rt, gL, gR, nL, nR,
                                      flux, bad, faceBad);
 #pragma unroll
             for (int kk = 0; kk < NQ; ++kk) F[kk] = flux[kk];
@@ -993,7 +1047,7 @@ __global__ void __launch_bounds__(kTileX * kTileY, RB200_TILE_MINBLOCKS) cartRat
             R gl[9], gh[9], nl, nh;
             tileCell<NS, R, SGS>(plane, slot, lo, gl, nl);
             globalCell<NS, R, SGS>(v, q, st, grad, nut, cellAt(gx, gy, z + 1), viscous, hi, gh, nh);
-            faceFluxCart<NS, R, SGS>(v, 2, 1.0, v.area[2], v.dist[2], .5, 0, true, lo, hi, gl, gh, nl, nh, up, bad,
+            faceFluxCart<NS, R, SGS>(v, 2, 1.0, v.area[2], v.invDist[2], .5, 0, true, lo, hi, gl, gh, nl, nh, up, bad,
                                      faceBad);
         }
         __syncthreads();
@@ -1023,7 +1077,7 @@ __global__ void __launch_bounds__(kTileX * kTileY, RB200_TILE_MINBLOCKS) cartRat
             tileCell<NS, R, SGS>(plane, slot, me, gMe, nuMe);
             CellData C;
             const bool boundary = gx == 0 || gy == 0 || z == 0 || gx + 1 == v.nx || gy + 1 == v.ny || z + 1 == v.nz;
-            if (boundary) loadCell<NS, SGS>(v, q, st, c, C, true);
+            if (boundary) loadCell<NS, SGS>(v, q, c, C, true);
 #pragma unroll
             for (int side = 0; side < 6; ++side) {
                 if (hasNeighbour(v, side, gx, gy, z)) continue;
@@ -1032,7 +1086,7 @@ __global__ void __launch_bounds__(kTileX * kTileY, RB200_TILE_MINBLOCKS) cartRat
                 CellData Rd;
                 boundaryRight<NS, SGS>(v, q, st, f, axis, C, Rd, true);
                 R flux[NQ];
-                faceFluxCart<NS, R, SGS>(v, axis, (side & 1) ? 1.0 : -1.0, f.area, f.distance, f.ownerWeight, f.kind,
+                faceFluxCart<NS, R, SGS>(v, axis, (side & 1) ? 1.0 : -1.0, f.area, 1 / f.distance, f.ownerWeight, f.kind,
                                          false, me, asCell<NS, R, SGS>(Rd), gMe, gMe, nuMe, nuMe, flux, bad, faceBad);
                 add(flux, -1);
             }
@@ -1058,7 +1112,7 @@ __global__ void __launch_bounds__(kTileX * kTileY, RB200_TILE_MINBLOCKS) cartRat
 
 // Wave/diffusion speed of one face (faceSpeeds of the face graph); -1 when invalid.
 template <bool SGS>
-__device__ __forceinline__ double faceSpeedCart(const CartView& v, int axis, double sgn, double dist, double w,
+__device__ __forceinline__ double faceSpeedCart(const CartView& v, int axis, double sgn, double invDist, double w,
                                                 int kind, const CellData& L, const CellData& R, double nutL,
                                                 double nutR) {
     const double unL = L.u[axis] * sgn, unR = R.u[axis] * sgn;
@@ -1067,19 +1121,20 @@ __device__ __forceinline__ double faceSpeedCart(const CartView& v, int axis, dou
     const double invWave = 1 / (right - left);
     const double rhoNut = v.wale ? w * L.rho * nutL + (1 - w) * R.rho * nutR : 0;
     const double mu = v.viscosity + rhoNut;
-    const double D = 0.0 + dmax(dmax(4 * mu / (3 * L.rho), 4 * mu / (3 * R.rho)),
-                                dmax(v.conductivity / (L.rho * L.cv), v.conductivity / (R.rho * R.cv)));
+    const double mu43 = mu * (4.0 / 3.0);
+    const double D = 0.0 + dmax(dmax(mu43 * L.irho, mu43 * R.irho),
+                                dmax(v.conductivity * L.ircv, v.conductivity * R.ircv));
     double scalar = 0;
     if constexpr (SGS) {
         if (kind != 1) {
             if (v.pr > 0) {
-                const double k = rhoNut * (w * L.cp + (1 - w) * R.cp) / v.pr;
-                scalar = dmax(scalar, dmax(k / (L.rho * L.cv), k / (R.rho * R.cv)));
+                const double k = rhoNut * (w * L.cp + (1 - w) * R.cp) * v.invPr;
+                scalar = dmax(scalar, dmax(k * L.ircv, k * R.ircv));
             }
-            if (v.sc > 0) scalar = dmax(scalar, dmax(rhoNut / L.rho, rhoNut / R.rho) / v.sc);
+            if (v.sc > 0) scalar = dmax(scalar, dmax(rhoNut * L.irho, rhoNut * R.irho) * v.invSc);
         }
     }
-    double speed = dmax(fabs(unL) + aL, fabs(unR) + aR) + 2 * (D + scalar) / dist;
+    double speed = dmax(fabs(unL) + aL, fabs(unR) + aR) + 2 * (D + scalar) * invDist;
     if (!isfinite(unL) || !isfinite(unR) || !isfinite(speed) || !isfinite(invWave) || right <= left) speed = -1;
     return speed;
 }
@@ -1099,7 +1154,7 @@ __global__ void __launch_bounds__(256) cartSteps(CartView v, const ReactiveTrans
         int i, j, k;
         cellCoords(v, c, i, j, k);
         CellData C;
-        loadCell<NS, SGS>(v, nullptr, st, c, C, false);
+        loadCell<NS, SGS>(v, nullptr, c, C, false);
         const double nutC = v.wale ? double(nut[c]) : 0;
         double denominator = 0;
         bool bad = false, faceBad = false;
@@ -1113,16 +1168,16 @@ __global__ void __launch_bounds__(256) cartSteps(CartView v, const ReactiveTrans
             if (interior) {
                 const size_t nb = neighbourOf(v, s, c);
                 CellData N;
-                loadCell<NS, SGS>(v, nullptr, st, nb, N, false);
+                loadCell<NS, SGS>(v, nullptr, nb, N, false);
                 const double nutN = v.wale ? double(nut[nb]) : 0;
-                speed = (s & 1) ? faceSpeedCart<SGS>(v, axis, 1.0, v.dist[axis], .5, 0, C, N, nutC, nutN)
-                                : faceSpeedCart<SGS>(v, axis, 1.0, v.dist[axis], .5, 0, N, C, nutN, nutC);
+                speed = (s & 1) ? faceSpeedCart<SGS>(v, axis, 1.0, v.invDist[axis], .5, 0, C, N, nutC, nutN)
+                                : faceSpeedCart<SGS>(v, axis, 1.0, v.invDist[axis], .5, 0, N, C, nutN, nutC);
                 area = v.area[axis];
             } else {
                 const ReactiveTransportFace& f = sideFace(v, s, i, j, k);
                 CellData Rt;
                 boundaryRight<NS, SGS>(v, nullptr, st, f, axis, C, Rt, false);
-                speed = faceSpeedCart<SGS>(v, axis, (s & 1) ? 1.0 : -1.0, f.distance, f.ownerWeight, f.kind, C, Rt,
+                speed = faceSpeedCart<SGS>(v, axis, (s & 1) ? 1.0 : -1.0, 1 / f.distance, f.ownerWeight, f.kind, C, Rt,
                                            nutC, nutC);
                 area = f.area;
             }
@@ -1165,7 +1220,7 @@ __global__ void __launch_bounds__(256) cartLedger(CartView v, const double* __re
         const int axis = f.normal[0] != 0 ? 0 : (f.normal[1] != 0 ? 1 : 2);
         const double sgn = f.normal[axis] > 0 ? 1.0 : -1.0;
         CellData C, Rt;
-        loadCell<NS, SGS>(v, q, st, c, C, true);
+        loadCell<NS, SGS>(v, q, c, C, true);
         boundaryRight<NS, SGS>(v, q, st, f, axis, C, Rt, true);
         R g[9] = {R(0), R(0), R(0), R(0), R(0), R(0), R(0), R(0), R(0)};
         if (viscous) {
@@ -1174,7 +1229,7 @@ __global__ void __launch_bounds__(256) cartLedger(CartView v, const double* __re
         }
         const R nutC = v.wale ? nut[c] : R(0);
         R F[NS + 4];
-        faceFluxCart<NS, R, SGS>(v, axis, sgn, f.area, f.distance, f.ownerWeight, f.kind, false,
+        faceFluxCart<NS, R, SGS>(v, axis, sgn, f.area, 1 / f.distance, f.ownerWeight, f.kind, false,
                                  asCell<NS, R, SGS>(C), asCell<NS, R, SGS>(Rt), g, g, nutC, nutC, F, bad, faceBad);
 #pragma unroll
         for (int kk = 0; kk < NS + 4; ++kk) sum[kk] += double(F[kk]);
@@ -1224,7 +1279,7 @@ __global__ void __launch_bounds__(128) cartRateVjp(CartView v, const double* __r
         int i, j, k;
         cellCoords(v, c, i, j, k);
         CellData C;
-        loadCell<NS>(v, q, st, c, C, true);
+        loadCell<NS>(v, q, c, C, true);
         CellT<D> Cd = asCell<NS, D>(C);
         D gC[9], nutC(0.0);
 #pragma unroll
@@ -1263,7 +1318,7 @@ __global__ void __launch_bounds__(128) cartRateVjp(CartView v, const double* __r
             if (interior) {
                 const size_t nb = neighbourOf(v, s, c);
                 CellData Nc;
-                loadCell<NS>(v, q, st, nb, Nc, true);
+                loadCell<NS>(v, q, nb, Nc, true);
                 const CellT<D> Nd = asCell<NS, D>(Nc);
                 D gN[9], nutN(0.0);
 #pragma unroll
@@ -1271,13 +1326,13 @@ __global__ void __launch_bounds__(128) cartRateVjp(CartView v, const double* __r
                 if (v.wale) nutN = D(nut[nb]);
                 const double ivn = v.invV[nb];
                 if (s & 1) {  // c owns the face
-                    faceFluxCart<NS, D>(v, axis, 1.0, v.area[axis], v.dist[axis], .5, 0, true, Cd, Nd, gC, gN, nutC,
+                    faceFluxCart<NS, D>(v, axis, 1.0, v.area[axis], v.invDist[axis], .5, 0, true, Cd, Nd, gC, gN, nutC,
                                         nutN, F, bad, faceBad);
 #pragma unroll
                     for (int kk = 0; kk < NS + 4; ++kk)
                         W[kk] = w[size_t(kk) * v.cells + nb] * ivn - w[size_t(kk) * v.cells + c] * ivc;
                 } else {
-                    faceFluxCart<NS, D>(v, axis, 1.0, v.area[axis], v.dist[axis], .5, 0, true, Nd, Cd, gN, gC, nutN,
+                    faceFluxCart<NS, D>(v, axis, 1.0, v.area[axis], v.invDist[axis], .5, 0, true, Nd, Cd, gN, gC, nutN,
                                         nutC, F, bad, faceBad);
 #pragma unroll
                     for (int kk = 0; kk < NS + 4; ++kk)
@@ -1288,7 +1343,7 @@ __global__ void __launch_bounds__(128) cartRateVjp(CartView v, const double* __r
                 CellT<D> Rt;
                 if (f.kind == 3) {
                     CellData Fx;
-                    loadCell<NS>(v, q, st, v.cells + size_t(f.fixed), Fx, true);
+                    loadFixed<NS>(v, q, st, size_t(f.fixed), Fx, true);
                     Rt = asCell<NS, D>(Fx);
                 } else {
                     Rt = Cd;
@@ -1297,7 +1352,7 @@ __global__ void __launch_bounds__(128) cartRateVjp(CartView v, const double* __r
                         Rt.q[NS + axis] = Cd.q[NS + axis] - D(2.0) * Cd.q[NS + axis];
                     }
                 }
-                faceFluxCart<NS, D>(v, axis, (s & 1) ? 1.0 : -1.0, f.area, f.distance, f.ownerWeight, f.kind, false,
+                faceFluxCart<NS, D>(v, axis, (s & 1) ? 1.0 : -1.0, f.area, 1 / f.distance, f.ownerWeight, f.kind, false,
                                     Cd, Rt, gC, gC, nutC, nutC, F, bad, faceBad);
 #pragma unroll
                 for (int kk = 0; kk < NS + 4; ++kk) W[kk] = -w[size_t(kk) * v.cells + c] * ivc;
@@ -1384,7 +1439,7 @@ __global__ void __launch_bounds__(128) cartRateVjpInviscid(CartView v, const dou
         int i, j, k;
         cellCoords(v, c, i, j, k);
         CellData C;
-        loadCell<NS>(v, q, st, c, C, true);
+        loadCell<NS>(v, q, c, C, true);
         const double ivc = v.invV[c];
         double dq[NS + 4], du[3] = {0, 0, 0}, dp = 0, dc = 0, dT = 0, dRhoState = 0;
 #pragma unroll
@@ -1402,18 +1457,18 @@ __global__ void __launch_bounds__(128) cartRateVjpInviscid(CartView v, const dou
             if (interior != (n < 6)) continue;
             const int axis = s >> 1;
             CellData O;  // the other side
-            double Wa[NS + 4], sgn, area, wf, dist, gO[9], nutO = nutC;
+            double Wa[NS + 4], sgn, area, wf, invDist, gO[9], nutO = nutC;
             int kind = 0;
             bool cIsLeft = true;
             if (interior) {
                 const size_t nb = neighbourOf(v, s, c);
-                loadCell<NS>(v, q, st, nb, O, true);
+                loadCell<NS>(v, q, nb, O, true);
                 const double ivn = v.invV[nb];
                 cIsLeft = s & 1;
                 sgn = 1;
                 area = v.area[axis];
                 wf = .5;
-                dist = v.dist[axis];
+                invDist = v.invDist[axis];
                 if (viscous) {
 #pragma unroll
                     for (int t = 0; t < 9; ++t) gO[t] = grad[size_t(t) * v.cells + nb];
@@ -1430,7 +1485,7 @@ __global__ void __launch_bounds__(128) cartRateVjpInviscid(CartView v, const dou
                 sgn = (s & 1) ? 1.0 : -1.0;
                 area = f.area;
                 wf = f.ownerWeight;
-                dist = f.distance;
+                invDist = 1 / f.distance;
 #pragma unroll
                 for (int t = 0; t < 9; ++t) gO[t] = gC[t];
 #pragma unroll
@@ -1469,7 +1524,7 @@ __global__ void __launch_bounds__(128) cartRateVjpInviscid(CartView v, const dou
                 const double* gL = cIsLeft ? gC : gO;
                 const double* gR = cIsLeft ? gO : gC;
                 const double nutL = cIsLeft ? nutC : nutO, nutR = cIsLeft ? nutO : nutC;
-                const double kd = (kind == 1 ? 2 : 1) * dist;
+                const double ikd = (kind == 1 ? .5 : 1.0) * invDist;
                 double g[9];
 #pragma unroll
                 for (int t = 0; t < 9; ++t) g[t] = interior ? wf * gL[t] + (1 - wf) * gR[t] : gL[t];
@@ -1478,7 +1533,7 @@ __global__ void __launch_bounds__(128) cartRateVjpInviscid(CartView v, const dou
                     double normal = 0;
 #pragma unroll
                     for (int d = 0; d < 3; ++d) normal += g[a * 3 + d] * nv[d];
-                    const double target = (R.u[a] - L.u[a]) / kd;
+                    const double target = (R.u[a] - L.u[a]) * ikd;
 #pragma unroll
                     for (int d = 0; d < 3; ++d) g[a * 3 + d] += nv[d] * (target - normal);
                 }
@@ -1511,8 +1566,8 @@ __global__ void __launch_bounds__(128) cartRateVjpInviscid(CartView v, const dou
                     for (int d = 0; d < 3; ++d)
                         rn += mu * (av[a] * nv[d] + nv[a] * av[d] - (a == d ? 2.0 / 3.0 * an : 0.0)) * nv[d];
                     const double dbar = -Wa[NS + 3] * tau[a];
-                    duL[a] = wf * dbar - rn / kd;
-                    duR[a] = (1 - wf) * dbar + rn / kd;
+                    duL[a] = wf * dbar - rn * ikd;
+                    duR[a] = (1 - wf) * dbar + rn * ikd;
                     double t = -2.0 / 3.0 * div * nv[a];
 #pragma unroll
                     for (int d = 0; d < 3; ++d) t += (g[a * 3 + d] + g[d * 3 + a]) * nv[d];
@@ -1524,7 +1579,7 @@ __global__ void __launch_bounds__(128) cartRateVjpInviscid(CartView v, const dou
                 }
             }
             if (v.conductivity > 0 && kind != 1) {
-                dTL = Wa[NS + 3] * v.conductivity / dist;
+                dTL = Wa[NS + 3] * v.conductivity * invDist;
                 dTR = -dTL;
             }
             if (interior) {
@@ -1588,7 +1643,7 @@ __global__ void __launch_bounds__(128) cartViscousGradVjp(CartView v, const doub
         int i, j, k;
         cellCoords(v, c, i, j, k);
         CellData C;
-        loadCell<NS>(v, q, st, c, C, false);
+        loadCell<NS>(v, q, c, C, false);
         double gC[9];
 #pragma unroll
         for (int t = 0; t < 9; ++t) gC[t] = grad[size_t(t) * v.cells + c];
@@ -1602,19 +1657,19 @@ __global__ void __launch_bounds__(128) cartViscousGradVjp(CartView v, const doub
             if (interior != (n < 6)) continue;
             const int axis = s >> 1;
             CellData O;
-            double gO[9], nutO, W[4], sgn, wf, dist, area, weightC, dmu;
+            double gO[9], nutO, W[4], sgn, wf, invDist, area, weightC, dmu;
             int kind = 0;
             bool cLeft = true;
             if (interior) {
                 const size_t nbr = neighbourOf(v, s, c);
-                loadCell<NS>(v, q, st, nbr, O, false);
+                loadCell<NS>(v, q, nbr, O, false);
 #pragma unroll
                 for (int t = 0; t < 9; ++t) gO[t] = grad[size_t(t) * v.cells + nbr];
                 nutO = v.wale ? nut[nbr] : 0.0;
                 cLeft = s & 1;
                 sgn = 1;
                 wf = .5;
-                dist = v.dist[axis];
+                invDist = v.invDist[axis];
                 area = v.area[axis];
                 const double ivn = v.invV[nbr];
 #pragma unroll
@@ -1633,7 +1688,7 @@ __global__ void __launch_bounds__(128) cartViscousGradVjp(CartView v, const doub
                 kind = f.kind;
                 sgn = (s & 1) ? 1.0 : -1.0;
                 wf = f.ownerWeight;
-                dist = f.distance;
+                invDist = 1 / f.distance;
                 area = f.area;
 #pragma unroll
                 for (int t = 0; t < 4; ++t) W[t] = -w[size_t(NS + t) * v.cells + c] * ivc;
@@ -1657,7 +1712,7 @@ __global__ void __launch_bounds__(128) cartViscousGradVjp(CartView v, const doub
                 double normal = 0;
 #pragma unroll
                 for (int d = 0; d < 3; ++d) normal += g[a * 3 + d] * nv[d];
-                const double target = (R.u[a] - L.u[a]) / ((kind == 1 ? 2 : 1) * dist);
+                const double target = (R.u[a] - L.u[a]) * ((kind == 1 ? .5 : 1.0) * invDist);
 #pragma unroll
                 for (int d = 0; d < 3; ++d) g[a * 3 + d] += nv[d] * (target - normal);
             }

@@ -394,6 +394,20 @@ struct Transport {
     }
 
     // ---------------------------------------------------------------- kernels
+    // What the kernels of an entry read besides q and the states: on the structured
+    // box the cells' flux inputs, on the face graph their primitives.
+    void launchInputs(const double* qSoA, const ReactiveTransportState* state, cudaStream_t s) {
+        if (structured) {
+            cartInputs<<<gridFor(v.all, 256), 256, 0, s>>>(boxView(), qSoA, state, int(cfg.species), false);
+            launched();
+        } else launchPrimitives(qSoA, s);
+    }
+    // The same for the caller's primitives (in v.primitive) and states (stateDevice).
+    void launchInputsFromPrimitives() {
+        if (!structured) return;
+        cartInputs<<<gridFor(v.all, 256), 256, 0, stream>>>(boxView(), nullptr, stateDevice, int(cfg.species), true);
+        launched();
+    }
     void launchPrimitives(const double* qSoA, cudaStream_t s) {
         GraphView g = v;
         g.q = qSoA;
@@ -500,7 +514,7 @@ struct Transport {
     // -+e_axis. Any other face list, species diffusion, the mechanical
     // variables, or more than four species use the face graph.
     bool detectBox(const ReactiveTransportFace* faces, size_t nInternal, const double* invDevice,
-                   const ReactiveTransportPrimitive* primitive) {
+                   ReactiveTransportPrimitive* primitive) {
         if (cfg.mechanical || cfg.diffusivity != 0 || cfg.variables != cfg.species + 4 || cfg.species < 1
             || cfg.species > size_t(kCartMaxNs) || nInternal < 3 || cfg.cells < 8)
             return false;
@@ -555,13 +569,30 @@ struct Transport {
         }
         box.nx = int(nx); box.ny = int(ny); box.nz = int(nz);
         box.cells = cfg.cells; box.fixed = cfg.fixed; box.all = cfg.cells + cfg.fixed;
-        for (int a = 0; a < 3; ++a) { box.area[a] = area[a]; box.dist[a] = dist[a]; }
+        for (int a = 0; a < 3; ++a) {
+            box.area[a] = area[a];
+            box.dist[a] = dist[a];
+            box.invDist[a] = 1 / dist[a];
+        }
         box.invV = invDevice;
         box.face = v.face;
         for (int side = 0; side < 6; ++side) box.sideBase[side] = base[side];
         box.boundaryBase = nInternal;
         box.nBoundary = bnd;
         box.primitive = primitive;
+        // the flux inputs live in buffers the structured path leaves idle while its
+        // kernels run: the host bridge (variables >= 5 per cell, packed before and
+        // unpacked after them on the same stream) and the face graph's face speeds
+        // (at least three faces a cell here) and cell steps
+        double* bridge = staging;
+        for (double** array : {&box.in.u[0], &box.in.u[1], &box.in.u[2], &box.in.p, &box.in.T}) {
+            *array = bridge;
+            bridge += cfg.cells;
+        }
+        box.in.rho = v.faceSpeed;
+        box.in.c = v.faceSpeed + cfg.cells;
+        box.in.irho = v.faceSpeed + 2 * cfg.cells;
+        box.in.ircv = v.step;
         box.viscosity = cfg.viscosity; box.conductivity = cfg.conductivity; box.waveFactor = cfg.waveFactor;
         return true;
     }
@@ -583,6 +614,8 @@ struct Transport {
         b.sgs = v.sgs;
         b.pr = v.pr;
         b.sc = v.sc;
+        b.invPr = v.invPr;
+        b.invSc = v.invSc;
         b.mixCp = v.mixCp;
         b.spH = v.spH;
         // the split stage's face fluxes live in the face graph's workspace, which
@@ -829,7 +862,7 @@ struct Transport {
             gradBar = arena.get<double>(product(cfg.cells, 9));
             nutBarBuf = arena.get<double>(cfg.cells);
         }
-        launchPrimitives(q, s);
+        launchInputs(q, state, s);
         if (viscous) launchBoxGradientsT(state, v.grad, v.nut, s);
         bySpecies<RateVjpK>(boxView(), q, state, static_cast<const double*>(v.grad), static_cast<const double*>(v.nut),
                             w, qBar, stateBar, gradBar, nutBarBuf, viscous, s);
@@ -868,7 +901,7 @@ struct Transport {
             }
             slot = keep;
         };
-        launchPrimitives(q, s);
+        launchInputs(q, state, s);
         // candidates stay within each kernel's __launch_bounds__ (128 for the stage, 256 otherwise)
         pick(launch.gradients, {64u, 128u, 256u}, [&] {
             if (mixed) launchBoxGradientsT(state, gradF, nutF, s);
@@ -904,7 +937,7 @@ struct Transport {
             packInto(const_cast<double*>(v.gasH), gasH, cfg.cells, cfg.species, v.all, 0);
             profile.gasUploadBytes += 2 * cfg.cells * cfg.species * sizeof(double);
         }
-        launchPrimitives(q, stream);
+        launchInputs(q, stateDevice, stream);
         if (v.wale) buildWaleChecked();
         if (structured) {
             // the host-array entries on the structured box: FP64 HLL stencils, bitwise
@@ -1509,6 +1542,8 @@ struct Transport {
         }
         v.pr = options.turbulentPrandtl;
         v.sc = options.turbulentSchmidt;
+        v.invPr = v.pr > 0 ? 1 / v.pr : 0;
+        v.invSc = v.sc > 0 ? 1 / v.sc : 0;
         v.sgs = true;
         if (!structured) ensureGraphScalarWork();
         finish();
@@ -1604,6 +1639,7 @@ struct Transport {
     void uploadPrimitives(const ReactiveTransportPrimitive* primitive, const ReactiveTransportState* state) {
         require(primitive, "Null transport primitives");
         uploadState(state, primitive);
+        launchInputsFromPrimitives();
     }
 };
 

@@ -59,7 +59,7 @@ struct GraphView {
     // WALE scalar closure (turbulent Prandtl heat flux rho nu_t cp / Pr_t grad T,
     // turbulent Schmidt species mixing rho nu_t / Sc_t grad Y); 0 disables a term
     bool sgs = false;
-    double pr = 0, sc = 0;
+    double pr = 0, sc = 0, invPr = 0, invSc = 0;
     const double* mixCp = nullptr;                   // all, mixture cp
     const double* spH = nullptr;                     // SoA ns x all, effective species enthalpies
     double* sgsWork = nullptr;                       // SoA 3 x faces: diffusion, sumJ, carrier flux
@@ -180,18 +180,20 @@ __device__ __forceinline__ double faceSpeedOf(const GraphView& v, const Reactive
                                        + (1 - f.ownerWeight) * sr.rho * faceNut(v, f, true)
                                  : 0;
     const double mu = v.viscosity + rhoNut;
+    // the reciprocals the structured kernels keep per cell (the same operations)
+    const double iL = 1 / sl.rho, iR = 1 / sr.rho, icL = 1 / (sl.rho * sl.cv), icR = 1 / (sr.rho * sr.cv);
+    const double mu43 = mu * (4.0 / 3.0);
     const double D = v.diffusivity
-        + dmax(dmax(4 * mu / (3 * sl.rho), 4 * mu / (3 * sr.rho)),
-               dmax(v.conductivity / (sl.rho * sl.cv), v.conductivity / (sr.rho * sr.cv)));
+        + dmax(dmax(mu43 * iL, mu43 * iR), dmax(v.conductivity * icL, v.conductivity * icR));
     double scalar = 0;
     if (v.sgs && f.kind != 1) {
         if (v.pr > 0) {
-            const double k = rhoNut * (f.ownerWeight * v.mixCp[f.owner] + (1 - f.ownerWeight) * v.mixCp[r]) / v.pr;
-            scalar = dmax(scalar, dmax(k / (sl.rho * sl.cv), k / (sr.rho * sr.cv)));
+            const double k = rhoNut * (f.ownerWeight * v.mixCp[f.owner] + (1 - f.ownerWeight) * v.mixCp[r]) * v.invPr;
+            scalar = dmax(scalar, dmax(k * icL, k * icR));
         }
-        if (v.sc > 0) scalar = dmax(scalar, dmax(rhoNut / sl.rho, rhoNut / sr.rho) / v.sc);
+        if (v.sc > 0) scalar = dmax(scalar, dmax(rhoNut * iL, rhoNut * iR) * v.invSc);
     }
-    double speed = dmax(fabs(unL) + aL, fabs(unR) + aR) + 2 * (D + scalar) / f.distance;
+    double speed = dmax(fabs(unL) + aL, fabs(unR) + aR) + 2 * (D + scalar) * (1 / f.distance);
     if (!isfinite(unL) || !isfinite(unR) || !isfinite(speed) || !isfinite(invWave) || right <= left) speed = -1;
     return speed;
 }
@@ -478,7 +480,7 @@ __global__ void faceWork(GraphView v, bool speeds) {
         for (int d = 0; d < 3; ++d) { unL += ul[d] * f.normal[d]; unR += ur[d] * f.normal[d]; }
         const double aL = v.waveFactor * sl.sound, aR = v.waveFactor * sr.sound;
         const double left = dmin(0, dmin(unL - aL, unR - aR)), right = dmax(0, dmax(unL + aL, unR + aR));
-        const double invWave = 1 / (right - left);
+        const double invWave = 1 / (right - left), invDist = 1 / f.distance;
         double out[FW_FIELDS] = {};
         out[FW_VELOCITY] = (right * unL - left * unR) * invWave;
         out[FW_ADV_L] = right * (unL - left) * invWave;
@@ -518,7 +520,7 @@ __global__ void faceWork(GraphView v, bool speeds) {
             for (int i = 0; i < 3; ++i) {
                 double normal = 0;
                 for (int d = 0; d < 3; ++d) normal += g[i * 3 + d] * f.normal[d];
-                const double target = (ur[i] - ul[i]) / ((f.kind == 1 ? 2 : 1) * f.distance);
+                const double target = (ur[i] - ul[i]) * ((f.kind == 1 ? .5 : 1.0) * invDist);
                 for (int d = 0; d < 3; ++d) g[i * 3 + d] += f.normal[d] * (target - normal);
             }
             const double div = g[0] + g[4] + g[8];
@@ -526,7 +528,7 @@ __global__ void faceWork(GraphView v, bool speeds) {
                 + (v.wale ? w * sl.rho * faceNut(v, f, false) + (1 - w) * sr.rho * faceNut(v, f, true) : 0);
             for (int i = 0; i < 3; ++i)
                 for (int d = 0; d < 3; ++d)
-                    traction[i] += mu * (g[3 * i + d] + g[3 * d + i] - (i == d ? 2 * div / 3 : 0)) * f.normal[d];
+                    traction[i] += mu * (g[3 * i + d] + g[3 * d + i] - (i == d ? div * (2.0 / 3.0) : 0)) * f.normal[d];
             if (f.kind == 1) {
                 double dot = 0;
                 for (int d = 0; d < 3; ++d) dot += traction[d] * f.normal[d];
@@ -534,11 +536,11 @@ __global__ void faceWork(GraphView v, bool speeds) {
             }
             for (int d = 0; d < 3; ++d) energy -= traction[d] * (w * ul[d] + (1 - w) * ur[d]);
         }
-        if (v.conductivity > 0 && f.kind != 1) energy -= v.conductivity * (sr.T - sl.T) / f.distance;
+        if (v.conductivity > 0 && f.kind != 1) energy -= v.conductivity * (sr.T - sl.T) * invDist;
         if (v.sgs && v.pr > 0 && f.kind != 1) {
             const double rhoNut = w * sl.rho * faceNut(v, f, false) + (1 - w) * sr.rho * faceNut(v, f, true);
             const double cp = w * v.mixCp[l] + (1 - w) * v.mixCp[r];
-            energy -= rhoNut * cp / v.pr * (sr.T - sl.T) / f.distance;
+            energy -= rhoNut * cp * v.invPr * (sr.T - sl.T) * invDist;
         }
         int carrier = 0;
         if (v.diffusivity > 0 && sl.gasMass > 0 && sr.gasMass > 0 && f.kind != 1) {
@@ -569,7 +571,7 @@ __global__ void faceWork(GraphView v, bool speeds) {
         SgsFace sg;
         if (v.sgs && v.sc > 0 && f.kind != 1) {
             const double rhoNut = w * sl.rho * faceNut(v, f, false) + (1 - w) * sr.rho * faceNut(v, f, true);
-            sg.diffusion = -rhoNut / v.sc / f.distance;
+            sg.diffusion = -rhoNut * v.invSc * invDist;
             double largest = -1;
             for (size_t k = 0; k < v.ns; ++k) {
                 const double yl = v.q[k * v.all + l] / sl.rho, yr = v.q[k * v.all + r] / sr.rho;
