@@ -23,6 +23,8 @@
 #include "transport_kernels.cuh"
 #include "dual.cuh"
 
+#include <type_traits>
+
 namespace rb200 {
 
 constexpr int kCartMaxNs = 4;
@@ -206,7 +208,12 @@ __device__ __forceinline__ void twoSum(float& s, float& c, float x) {
 // (T_R - T_L) / d and the turbulent species mixing of total mass fractions with
 // its enthalpy flux, in the face graph's operation order
 // (src/reactiveTransport/reactiveTransportKernels.h:150-168, :440-477).
-template <int NS, class R, bool SGS = false>
+// AXIS >= 0: an interior face of that axis (normal +e_AXIS, ownerWeight .5, kind 0)
+// known at compile time. The products with zero normal components and the two
+// gradient components the face does not read then drop out, and .5 a + .5 b is
+// formed as .5 (a + b): for finite data every bit but the sign of a zero is the
+// general form's, with half its operations.
+template <int NS, class R, bool SGS = false, int AXIS = -1>
 __device__ __forceinline__ void faceFluxCart(const CartView& v, int axis, double sgnD, double areaD, double invDistD,
                                              double wD, int kind, bool internal, const CellT<R>& L,
                                              const CellT<R>& Rt, const R* gL, const R* gR, R nutL, R nutR, R* F,
@@ -255,7 +262,31 @@ __device__ __forceinline__ void faceFluxCart(const CartView& v, int axis, double
         }
     }
     R traction[3] = {R(0), R(0), R(0)}, energy = R(0);
-    if (v.viscosity > 0 || v.wale) {
+    if constexpr (AXIS >= 0) {
+        if (v.viscosity > 0 || v.wale) {
+            const R half = R(.5);
+            R g[9], onFace[3];
+#pragma unroll
+            for (int j = 0; j < 9; ++j) g[j] = half * (gL[j] + gR[j]);
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                const R normal = g[3 * i + AXIS], target = (Rt.u[i] - L.u[i]) * invDist;
+                onFace[i] = normal + (target - normal);
+            }
+#pragma unroll
+            for (int i = 0; i < 3; ++i) g[3 * i + AXIS] = onFace[i];
+            const R div = g[0] + g[4] + g[8];
+            const R mu = R(v.viscosity) + (v.wale ? half * (L.rho * nutL + Rt.rho * nutR) : R(0));
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                R t = g[3 * i + AXIS] + g[3 * AXIS + i];
+                if (i == AXIS) t -= div * R(2.0 / 3.0);
+                traction[i] = mu * t;
+            }
+#pragma unroll
+            for (int d = 0; d < 3; ++d) energy -= traction[d] * (half * (L.u[d] + Rt.u[d]));
+        }
+    } else if (v.viscosity > 0 || v.wale) {
         const R* uL = L.u;
         const R* uR = Rt.u;
         R g[9];
@@ -336,7 +367,9 @@ __device__ __forceinline__ void faceFluxCart(const CartView& v, int axis, double
 #pragma unroll
     for (int k = 0; k < NS + 4; ++k) {
         R flux = advL * L.q[k] + advR * Rt.q[k];
-        if (k >= NS && k < NS + 3) flux += pM * nrm(k - NS, axis, sgn);
+        if constexpr (AXIS >= 0) {
+            if (k == NS + AXIS) flux += pM;
+        } else if (k >= NS && k < NS + 3) flux += pM * nrm(k - NS, axis, sgn);
         if (k == NS + 3) flux += pE;
         if (k < NS) {
             // species diffusion: no molecular term on this path, the mixing flux when on
@@ -633,12 +666,11 @@ __global__ void __launch_bounds__(128, RB200_FACE_MINBLOCKS) cartFaceFluxes(Cart
         const R nutC = v.wale ? nut[c] : R(0);
         const CellT<R> cc = asCell<NS, R, SGS>(C);
         bool bad = false, faceBad = false;
-#pragma unroll 1
-        for (int axis = 0; axis < 3; ++axis) {
-            const int s = 2 * axis + 1;
-            if (!hasNeighbour(v, s, i, j, k)) continue;
+        auto upperFace = [&](auto ax) {
+            constexpr int axis = decltype(ax)::value, s = 2 * axis + 1;
+            if (!hasNeighbour(v, s, i, j, k)) return;
             const size_t nb = neighbourOf(v, s, c);
-            if (!ownC && !(nb >= v.ownBegin && nb < v.ownEnd)) continue;
+            if (!ownC && !(nb >= v.ownBegin && nb < v.ownEnd)) return;
             CellData N;
             loadCell<NS, SGS>(v, q, nb, N, true);
             R gN[9] = {R(0), R(0), R(0), R(0), R(0), R(0), R(0), R(0), R(0)};
@@ -648,14 +680,17 @@ __global__ void __launch_bounds__(128, RB200_FACE_MINBLOCKS) cartFaceFluxes(Cart
             }
             const R nutN = v.wale ? nut[nb] : R(0);
             R F[NQ];
-            faceFluxCart<NS, R, SGS>(v, axis, 1.0, v.area[axis], v.invDist[axis], .5, 0, true, cc,
-                                     asCell<NS, R, SGS>(N), gC, gN, nutC, nutN, F, bad, faceBad);
+            faceFluxCart<NS, R, SGS, axis>(v, axis, 1.0, v.area[axis], v.invDist[axis], .5, 0, true, cc,
+                                           asCell<NS, R, SGS>(N), gC, gN, nutC, nutN, F, bad, faceBad);
 #pragma unroll
             for (int kk = 0; kk < NQ; ++kk) flux[(size_t(axis) * NQ + kk) * v.cells + c] = F[kk];
             if (cflPass)
                 v.faceFlux[splitSpeedOffset(NQ, v.cells) + size_t(axis) * v.cells + c] =
                     faceSpeedCart<SGS>(v, axis, 1.0, v.invDist[axis], .5, 0, C, N, double(nutC), double(nutN));
-        }
+        };
+        upperFace(std::integral_constant<int, 0>{});
+        upperFace(std::integral_constant<int, 1>{});
+        upperFace(std::integral_constant<int, 2>{});
         if (bad) atomicOr(error, 1u);
         if (faceBad) atomicOr(error, 2u);
     }
