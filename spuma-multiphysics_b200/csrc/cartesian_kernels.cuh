@@ -418,49 +418,41 @@ __device__ __forceinline__ size_t neighbourOf(const CartView& v, int s, size_t c
 }
 
 // Green-Gauss gradient (and the WALE viscosity) of every cell, in arithmetic
-// type R (stored as R: 9 gradient components and nu_t per cell).
+// type R (stored as R: 9 gradient components and nu_t per cell). Bound by FP64
+// issue: a face adds to its own axis' three components only (the general form's
+// other products are with zero normal components and change no bit of finite
+// data), and the mean of the two cells' velocities is .5 (a + b).
 template <int NS, class R>
 __global__ void __launch_bounds__(256) cartGradients(CartView v, const ReactiveTransportState* __restrict__ st,
                                                      R* __restrict__ grad, R* __restrict__ nut, unsigned* error) {
     for (size_t c = blockIdx.x * size_t(blockDim.x) + threadIdx.x; c < v.cells; c += size_t(blockDim.x) * gridDim.x) {
         int i, j, k;
         cellCoords(v, c, i, j, k);
-        CellData C;
-        loadCell<NS>(v, nullptr, c, C, false);
-        R g[9] = {R(0), R(0), R(0), R(0), R(0), R(0), R(0), R(0), R(0)};
         const R iv = R(v.invV[c]);
+        R u[3], g[9] = {R(0), R(0), R(0), R(0), R(0), R(0), R(0), R(0), R(0)};
+#pragma unroll
+        for (int a = 0; a < 3; ++a) u[a] = R(v.in.u[a][c]);
 #pragma unroll
         for (int n = 0; n < 12; ++n) {
-            const int s = sideOf(n);
+            const int s = sideOf(n), axis = s >> 1;
             const bool interior = hasNeighbour(v, s, i, j, k);
             if (interior != (n < 6)) continue;
-            const int axis = s >> 1;
-            R uf[3], scale, sgn;
             if (interior) {
-                // internal face: owner is the lower cell, normal +e_axis; this cell's
-                // incidence sign is +1 on its upper side (owner), -1 on its lower side
+                // owner is the lower cell, normal +e_axis: incidence sign +1 on the upper side
                 const size_t nb = neighbourOf(v, s, c);
-                const bool owner = s & 1;
+                const R scale = R((s & 1) ? 1.0 : -1.0) * R(v.area[axis]) * iv;
 #pragma unroll
-                for (int a = 0; a < 3; ++a)
-                    uf[a] = owner ? R(.5) * R(C.u[a]) + (R(1) - R(.5)) * R(v.in.u[a][nb])
-                                  : R(.5) * R(v.in.u[a][nb]) + (R(1) - R(.5)) * R(C.u[a]);
-                scale = R(owner ? 1.0 : -1.0) * R(v.area[axis]) * iv;
-                sgn = R(1);
+                for (int a = 0; a < 3; ++a) g[3 * a + axis] += R(.5) * (u[a] + R(v.in.u[a][nb])) * scale;
             } else {
                 const ReactiveTransportFace& f = sideFace(v, s, i, j, k);
-                CellData Rt;
+                CellData C, Rt;
+                loadCell<NS>(v, nullptr, c, C, false);
                 boundaryRight<NS>(v, nullptr, st, f, axis, C, Rt, false);
-                const R w = R(f.ownerWeight);
+                const R w = R(f.ownerWeight), scale = R(f.area) * iv, sgn = (s & 1) ? R(1) : R(-1);
 #pragma unroll
-                for (int a = 0; a < 3; ++a) uf[a] = w * R(C.u[a]) + (R(1) - w) * R(Rt.u[a]);
-                scale = R(1.0) * R(f.area) * iv;
-                sgn = (s & 1) ? R(1) : R(-1);
+                for (int a = 0; a < 3; ++a)
+                    g[3 * a + axis] += (w * u[a] + (R(1) - w) * R(Rt.u[a])) * sgn * scale;
             }
-#pragma unroll
-            for (int a = 0; a < 3; ++a)
-#pragma unroll
-                for (int d = 0; d < 3; ++d) g[3 * a + d] += uf[a] * nrm(d, axis, sgn) * scale;
         }
 #pragma unroll
         for (int jj = 0; jj < 9; ++jj) grad[size_t(jj) * v.cells + c] = g[jj];
@@ -470,7 +462,7 @@ __global__ void __launch_bounds__(256) cartGradients(CartView v, const ReactiveT
             bool ok = isfinite(volume) && volume > R(0);
             if (ok) { delta = cbrt(volume); ok = isfinite(delta) && delta > R(0); }
             ok = ok && waleEddyViscosityT<R>(g, delta, R(v.cw), nu);
-            if (!ok || !isfinite(nu) || nu < R(0) || !isfinite(R(C.rho) * nu)) atomicOr(error, 1u);
+            if (!ok || !isfinite(nu) || nu < R(0) || !isfinite(R(v.in.rho[c]) * nu)) atomicOr(error, 1u);
             else nut[c] = nu;
         }
     }

@@ -28,9 +28,16 @@ __device__ inline bool waleEddyViscosityT(const R g[9], R delta, R cw, R& nut) {
         scale = fmax(scale, fabs(g[i]));
     }
     if (scale == R(0) || cw == R(0) || delta == R(0)) return true;
+    // one reciprocal for the nine components, unless a subnormal scale overflows it
+    const R inv = R(1) / scale;
     R h[9];
+    if (isfinite(inv)) {
 #pragma unroll
-    for (int i = 0; i < 9; ++i) h[i] = g[i] / scale;
+        for (int i = 0; i < 9; ++i) h[i] = g[i] * inv;
+    } else {
+#pragma unroll
+        for (int i = 0; i < 9; ++i) h[i] = g[i] / scale;
+    }
     R sq[9];
 #pragma unroll
     for (int i = 0; i < 3; ++i)
