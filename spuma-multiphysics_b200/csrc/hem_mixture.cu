@@ -33,8 +33,13 @@
 //     (:486-560, src/reactiveThermo/reactiveFlashSeeds.h:14-16).
 // Phase properties come from the mixture evaluator of pr_mixture.cuh (pinned to
 // the reference's evaluator). Every loop is bounded.
+// One copy of each evaluator routine, loops rolled: a warp's tasks are seldom at the same
+// instruction, so the searches are bound by instruction fetch (see mixture_residual.cuh).
+#define RB200_MIX_FN static __noinline__
+#define RB200_MIX_LOOP _Pragma("unroll 1")
 #include "hem_mixture.h"
 #include "pr_mixture.cuh"
+#include "mixture_residual.cuh"
 #include "common.cuh"
 
 #include <algorithm>
@@ -219,7 +224,7 @@ __device__ __noinline__ bool evaluate(MixCell& c, const double* mass, double p, 
 
 // Dense solve with full pivoting (pivot search column by column, rows inside
 // each column, first strict maximum) and the rank test pivot > largest * n * eps.
-__device__ bool solveDense(const double a0[4][4], const double* rhs, int n, double* x) {
+__device__ __noinline__ bool solveDense(const double a0[4][4], const double* rhs, int n, double* x) {
     double a[4][4], b[4], largest = 0;
     int column[4] = {0, 1, 2, 3};
     for (int i = 0; i < n; ++i) {
@@ -460,6 +465,7 @@ enum : int { kGasRecord = 0, kLiquidRecord = 1, kFullGasRecord = 2, kRecordKinds
 // the work list and its counters belong to the handle and are indexed by item.
 struct MixBatch {
     const ReactiveB200HemModel* model;
+    const MixTerms* terms;
     const double* q;
     const double* energy;
     size_t count;
@@ -692,7 +698,7 @@ struct MixTask {
 // per active set (liquids present) the five seeds, in the boundary recovery the
 // sixth and, with two liquids, their twelve unequal pairs; in the restart search
 // the five seeds at each restart temperature of the set's legal interval.
-__device__ bool nthTask(const MixCell& c, bool restarts, int index, MixTask& t) {
+__device__ __noinline__ bool nthTask(const MixCell& c, bool restarts, int index, MixTask& t) {
     const ReactiveB200HemModel& m = c.m;
     constexpr double seeds[5] = {-1, .5, .95, .1, .9999};
     constexpr double pairs[4] = {.1, .5, .95, .9999};
@@ -733,7 +739,7 @@ __device__ bool nthTask(const MixCell& c, bool restarts, int index, MixTask& t) 
 }
 
 // The Newton start of a task, false when it has none.
-__device__ bool taskStart(const MixCell& c, const MixTask& t, double* x, double& scale) {
+__device__ __noinline__ bool taskStart(const MixCell& c, const MixTask& t, double* x, double& scale) {
     const ReactiveB200HemModel& m = c.m;
     const double rho = density(c), gT = t.restartT >= 0 ? t.restartT : c.guess.T;
     scale = fmax(1e5 * rho, fmax(fabs(c.energy), rho * 2000 * fmax(gT, m.Tmin)));
@@ -785,8 +791,17 @@ struct MixBest {
 // its bits; a Newton step takes two rounds instead of seven or more evaluations
 // in a row. An accepted evaluation is the stability test's own point, so the test
 // reads its chemical potentials.
-__device__ __noinline__ void runTasks(MixCell& c, bool restarts, MixRecord* bestRecord, MixBest& best) {
+__device__ __noinline__ void runTasks(MixCell& c, const MixTerms& terms, bool restarts, MixRecord* bestRecord,
+                                      MixBest& best) {
     const ReactiveB200HemModel& m = c.m;
+    double q[kNs];
+    bool alone = terms.valid;  // the residual formed alone (mixture_residual.cuh)
+#pragma unroll
+    for (int k = 0; k < kNs; ++k) {
+        q[k] = c.q[k];
+        alone = alone && q[k] >= 0 && fin(q[k]);
+    }
+    const double gasOffset = c.color * c.jump, liquidOffset = (1 - c.color) * c.jump;
     const unsigned lane = threadIdx.x & 31u;
     const int width = m.nl == 1 ? 6 : 8, groups = 32 / width;
     const int g = int(lane) / width;
@@ -799,7 +814,7 @@ __device__ __noinline__ void runTasks(MixCell& c, bool restarts, MixRecord* best
     bool more = inGroup, converged = false, settled = false;
     MixTask t{{0, 0}, 0, 0, 0, 0};
     double x[4] = {}, f[4] = {}, step[4] = {}, column[4] = {}, scale = 1, previous = 0;
-    MixEval v, side;
+    MixEval v;
     for (;;) {
         // idle groups take the next tasks in order
         {
@@ -850,7 +865,17 @@ __device__ __noinline__ void runTasks(MixCell& c, bool restarts, MixRecord* best
             for (int i = 0; i < t.n; ++i) point = point && !rejectedCoordinate(c.adaptive, xe[i + 2]);
         }
         bool ok = false;
-        if (point) ok = activeResidual(c, t.active, t.n, xe, scale, fe, st == SIDES ? side : v);
+        bool general = point && !alone;
+        if (point && alone) {
+            const int code = mixtureResidual(terms, q, c.energy, c.adaptive, gasOffset, liquidOffset, m.pmin, m.pmax, m.Tmin,
+                                             m.Tmax, t.active, t.n, xe, scale, fe, c.n.phases);
+            ok = code == RESIDUAL_OK;
+            general = code == RESIDUAL_UNDECIDED;
+            if (!general) ++c.n.residuals;
+        }
+        if (__any_sync(0xffffffffu, general)) {
+            if (general) ok = activeResidual(c, t.active, t.n, xe, scale, fe, v);
+        }
         __syncwarp();
         bool finished = false, stable = false, evaluated = false;  // evaluated: (x, f) is a new iterate
         if (st == SIDES) {
@@ -963,13 +988,24 @@ __device__ __noinline__ void runTasks(MixCell& c, bool restarts, MixRecord* best
                 it = st == START ? 0 : it + 1;
                 evaluated = true;
                 finished = it >= 90;
+                converged = fabs(f[0]) <= m.vtol && fabs(f[1]) <= m.etol && maxAbs(f + 2, t.n) <= m.mutol;
+                if (converged && !finished) {
+                    // the candidate's state: its residual's evaluation in full
+                    bool whole = true;
+                    if (int(lane) == owner) {
+                        const Tally keep = c.n;
+                        double same[4] = {};
+                        whole = activeResidual(c, t.active, t.n, x, scale, same, v);
+                        c.n = keep;
+                    }
+                    finished = __ballot_sync(group, !whole) != 0;
+                }
             } else {
                 k += width;
                 finished = st == START || k >= kTrials;
             }
         }
         if (evaluated && !finished) {
-            converged = fabs(f[0]) <= m.vtol && fabs(f[1]) <= m.etol && maxAbs(f + 2, t.n) <= m.mutol;
             st = SIDES;
             settled = false;
             attempt = 0;
@@ -996,8 +1032,8 @@ __device__ __noinline__ void runTasks(MixCell& c, bool restarts, MixRecord* best
 // One search (the candidate list, then the restart temperatures when it found no
 // stable candidate) into *bestRecord (shared by the warp): the fixed-partition
 // candidates' records, then the tasks.
-__device__ __noinline__ bool searchWarp(MixCell& c, const MixRecord& gas, const MixRecord& liquid,
-                                        MixRecord* bestRecord) {
+__device__ __noinline__ bool searchWarp(MixCell& c, const MixTerms& terms, const MixRecord& gas,
+                                        const MixRecord& liquid, MixRecord* bestRecord) {
     const ReactiveB200HemModel& m = c.m;
     const unsigned lane = threadIdx.x & 31u;
     MixBest best{false, 0.0, 0};
@@ -1010,8 +1046,8 @@ __device__ __noinline__ bool searchWarp(MixCell& c, const MixRecord& gas, const 
     offer(liquid, -1);
     __syncwarp();
     const bool prune = m.stableGasPrune && prunable(m) && gas.status == kStable && gas.s.gasMass > 0 && !c.adaptive;
-    if (!prune && m.nl) runTasks(c, false, bestRecord, best);
-    if (!best.have && m.nl) runTasks(c, true, bestRecord, best);
+    if (!prune && m.nl) runTasks(c, terms, false, bestRecord, best);
+    if (!best.have && m.nl) runTasks(c, terms, true, bestRecord, best);
     return best.have;
 }
 
@@ -1023,9 +1059,18 @@ __device__ __noinline__ bool searchWarp(MixCell& c, const MixRecord& gas, const 
 // on a tie) kept. A frozen partition's result is its record. Results go to
 // out/success, or to outputs[cell] for the resident form; a failed cell gets its
 // seed.
-__global__ void __launch_bounds__(kSearchBlock, 3) mixtureSearch(MixBatch b) {
+//
+// Bound by instruction fetch (see mixture_residual.cuh), whose waits more warps hide:
+// 20,011 cells of the four-species gas take 51.9 ms at four blocks a multiprocessor
+// (128 registers), 48.3 at six and 42.3 at eight (64, 140 bytes spilled).
+__global__ void __launch_bounds__(kSearchBlock, 8) mixtureSearch(MixBatch b) {
     const ReactiveB200HemModel& m = *b.model;
     __shared__ MixRecord found[kSearchBlock / 32][2];
+    __shared__ MixTerms terms;
+    static_assert(sizeof(MixTerms) % sizeof(double) == 0, "copied by doubles");
+    for (unsigned i = threadIdx.x; i < sizeof(MixTerms) / sizeof(double); i += blockDim.x)
+        reinterpret_cast<double*>(&terms)[i] = reinterpret_cast<const double*>(b.terms)[i];
+    __syncthreads();
     MixRecord* best = found[threadIdx.x >> 5];
     const unsigned lane = threadIdx.x & 31u;
     Tally n;
@@ -1044,7 +1089,7 @@ __global__ void __launch_bounds__(kSearchBlock, 3) mixtureSearch(MixBatch b) {
             if (gas.status == kStable) result = &gas.s;
         } else {
             const MixRecord& liquid = b.record[kLiquidRecord][i];
-            const bool have = searchWarp(c, gas, liquid, best);
+            const bool have = searchWarp(c, terms, gas, liquid, best);
             if (have) result = &best[0].s;
             if (m.boundaryRecovery || b.capillary) {
                 bool again = !have;
@@ -1055,7 +1100,7 @@ __global__ void __launch_bounds__(kSearchBlock, 3) mixtureSearch(MixBatch b) {
                     }
                 if (again) {
                     c.adaptive = true;
-                    const bool other = searchWarp(c, b.record[kFullGasRecord] ? b.record[kFullGasRecord][i] : gas,
+                    const bool other = searchWarp(c, terms, b.record[kFullGasRecord] ? b.record[kFullGasRecord][i] : gas,
                                                   liquid, best + 1);
                     if (other && !(have && best[0].entropyD >= best[1].entropyD)) result = &best[1].s;
                 }
@@ -1169,6 +1214,7 @@ struct MixtureFlash {
     cudaStream_t stream = nullptr;
     std::vector<void*> blocks;
     ReactiveB200HemModel* model = nullptr;
+    MixTerms* terms = nullptr;
     double* q = nullptr;
     double* energy = nullptr;
     ReactiveThermoState* seed = nullptr;
@@ -1203,6 +1249,7 @@ MixtureFlash* mixtureCreate(const ReactiveB200HemModel& m, size_t capacity, int 
     f->ns = m.ns;
     check(cudaStreamCreateWithFlags(&f->stream, cudaStreamNonBlocking), "cudaStreamCreate");
     f->model = f->alloc<ReactiveB200HemModel>(1);
+    f->terms = f->alloc<MixTerms>(1);
     f->q = f->alloc<double>(capacity * size_t(m.ns));
     f->energy = f->alloc<double>(capacity);
     f->seed = f->alloc<ReactiveThermoState>(capacity);
@@ -1220,7 +1267,10 @@ MixtureFlash* mixtureCreate(const ReactiveB200HemModel& m, size_t capacity, int 
     f->newtonBlocks = unsigned(std::max(1, perSm) * std::max(1, sms));
     check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, mixtureSearch, kSearchBlock, 0), "occupancy");
     f->searchBlocks = unsigned(std::max(1, perSm) * std::max(1, sms));
+    MixTerms terms;
+    mixTerms(m, terms);
     check(cudaMemcpyAsync(f->model, &m, sizeof(m), cudaMemcpyHostToDevice, f->stream), "H2D model");
+    check(cudaMemcpyAsync(f->terms, &terms, sizeof(terms), cudaMemcpyHostToDevice, f->stream), "H2D terms");
     check(cudaStreamSynchronize(f->stream), "sync");
     return f.release();
 }
@@ -1234,6 +1284,7 @@ size_t mixtureDeviceBytes(const MixtureFlash* f) { return f ? f->bytes : 0; }
 static void launchRecovery(MixtureFlash* f, MixBatch b) {
     for (int i = 0; i < kRecordKinds; ++i) b.record[i] = f->record[i];
     b.model = f->model;
+    b.terms = f->terms;
     b.list = f->list;
     b.counters = f->counters;
     b.totals = f->totals;

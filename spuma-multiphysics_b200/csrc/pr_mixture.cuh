@@ -22,6 +22,15 @@
 #define RB200_HD
 #endif
 
+// Linkage of the evaluator's routines, and how its loops over species compile. A
+// kernel bound by instruction fetch defines them as calls and as rolled loops.
+#ifndef RB200_MIX_FN
+#define RB200_MIX_FN inline
+#endif
+#ifndef RB200_MIX_LOOP
+#define RB200_MIX_LOOP
+#endif
+
 namespace rb200 {
 namespace mix {
 
@@ -45,9 +54,10 @@ struct Props {
 RB200_HD inline bool finiteD(double x) { return x == x && fabs(x) <= DBL_MAX; }
 
 // Mole fractions and molar mass of the mass fractions Y (sum within 1e-12 of 1).
-RB200_HD inline int moles(const ReactiveB200Table& t, const double* Y, double* x, double& W) {
+RB200_HD RB200_MIX_FN int moles(const ReactiveB200Table& t, const double* Y, double* x, double& W) {
     if (t.ns < 1 || t.ns > kMaxNs) return BAD_TABLE;
     double sumY = 0, perW = 0;
+    RB200_MIX_LOOP
     for (int k = 0; k < t.ns; ++k) {
         if (!finiteD(Y[k]) || Y[k] < 0) return BAD_COMPOSITION;
         sumY += Y[k];
@@ -55,13 +65,14 @@ RB200_HD inline int moles(const ReactiveB200Table& t, const double* Y, double* x
     }
     if (!(perW > 0) || fabs(sumY - 1.0) > 1e-12) return BAD_COMPOSITION;
     W = 1.0 / perW;
+    RB200_MIX_LOOP
     for (int k = 0; k < t.ns; ++k) x[k] = Y[k] * W / t.species[k].molecularWeight;
     return OK;
 }
 
 // NASA7/9 cp/R, h/RT, s/R of species k at T (iT = 1/T, lT = ln T, shared by the
 // species of one evaluation).
-RB200_HD inline void nasa(const ReactiveB200Species& sp, double T, double iT, double lT, double& cpR, double& hRT,
+RB200_HD RB200_MIX_FN void nasa(const ReactiveB200Species& sp, double T, double iT, double lT, double& cpR, double& hRT,
                           double& sR) {
     int r = 0;
     for (int j = 1; j < sp.regionCount; ++j) {
@@ -92,9 +103,10 @@ struct Mixing {
     double q[kMaxNs];
 };
 
-RB200_HD inline int mixing(const ReactiveB200Table& t, double T, const double* x, Mixing& m) {
+RB200_HD RB200_MIX_FN int mixing(const ReactiveB200Table& t, double T, const double* x, Mixing& m) {
     double dq[kMaxNs], d2q[kMaxNs];
     m.a = m.b = m.aa = m.da = m.d2a = 0;
+    RB200_MIX_LOOP
     for (int i = 0; i < t.ns; ++i) {
         const ReactiveB200Species& sp = t.species[i];
         const double Tc = sp.a * kOmB / (sp.b * kOmA * kR);
@@ -107,7 +119,9 @@ RB200_HD inline int mixing(const ReactiveB200Table& t, double T, const double* x
         d2q[i] = sign * sp.kappa / (4.0 * Tc * Tc * root * root * root);
         m.b += x[i] * sp.b;
     }
+    RB200_MIX_LOOP
     for (int i = 0; i < t.ns; ++i)
+        RB200_MIX_LOOP
         for (int j = 0; j < t.ns; ++j) {
             const double w = x[i] * x[j] * t.aBinary[i][j];
             m.a += w;
@@ -129,6 +143,7 @@ struct PhaseLine {
     bool ready;
     RB200_HD bool holds(const ReactiveB200Table& t, const double* y) const {
         bool same = ready;
+        RB200_MIX_LOOP
         for (int k = 0; k < t.ns; ++k) same = same && x[k] == y[k];
         return same;
     }
@@ -144,7 +159,7 @@ RB200_HD inline double cubic(double V, double bn, double cn, double dn) { return
 
 // Roots of the PR cubic in V at (T, p) for mixture terms m (Cantera's signed root
 // count: 3, 2, +1 gas side, -1 liquid side).
-RB200_HD inline int roots(const Mixing& m, double T, double p, Roots& r) {
+RB200_HD RB200_MIX_FN int roots(const Mixing& m, double T, double p, Roots& r) {
     const double b = m.b, b2 = b * b, RTp = kR * T / p, aap = m.aa / p, bn = b - RTp;
     const double cn = -(2.0 * RTp * b - aap + 3.0 * b2), dn = b2 * RTp + b2 * b - aap * b;
     const double center = -bn / 3.0, delta2 = (bn * bn - 3.0 * cn) / 9.0;
@@ -193,6 +208,7 @@ RB200_HD inline int roots(const Mixing& m, double T, double p, Roots& r) {
         raw = 3;
     } else return NO_ROOT;
     if (!side)
+        RB200_MIX_LOOP
         for (int i = 0; i < raw; ++i)
             for (int it = 0; it < 12; ++it) {
                 const double d = (3.0 * v[i] + 2.0 * bn) * v[i] + cn;
@@ -232,7 +248,7 @@ RB200_HD inline int roots(const Mixing& m, double T, double p, Roots& r) {
 // The line's end at T_mid = Tc - 100 K (or Tc / 2): the mid density of the two
 // roots there, the pressure raised by 4% until the cubic has both roots above pc or
 // three roots (at most 100 cubic solves).
-RB200_HD inline int phaseLine(const ReactiveB200Table& t, const double* x, double W, double tc, double pc,
+RB200_HD RB200_MIX_FN int phaseLine(const ReactiveB200Table& t, const double* x, double W, double tc, double pc,
                               PhaseLine& line) {
     line.tmid = tc - 100.0 < 0 ? .5 * tc : tc - 100.0;
     const double tmid = line.tmid, ratio = tc / tmid;
@@ -282,7 +298,7 @@ RB200_HD inline int reportedPhase(const ReactiveB200Table& t, double T, const do
 // Properties at (T, rho); chem: the species chemical potentials. The composition
 // comes as its mole fractions x, molar mass W and mixing terms m at T; kept as in
 // reportedPhase. (See trho for mass fractions.)
-RB200_HD inline int trhoMixed(const ReactiveB200Table& t, double T, double rho, const double* x, double W,
+RB200_HD RB200_MIX_FN int trhoMixed(const ReactiveB200Table& t, double T, double rho, const double* x, double W,
                               const Mixing& m, bool chem, Props& s, PhaseLine* kept) {
     if (!finiteD(rho) || rho <= 0) return BAD_INPUT;
     const double b = m.b, V = W / rho;
@@ -299,6 +315,7 @@ RB200_HD inline int trhoMixed(const ReactiveB200Table& t, double T, double rho, 
     const double L = logRatio / (2.0 * kRt2 * b);
     const double iT = 1.0 / T, lT = log(T);
     double h0 = 0, s0 = 0, cp0 = 0, xlx = 0, hk[kMaxNs], sk[kMaxNs];
+    RB200_MIX_LOOP
     for (int k = 0; k < t.ns; ++k) {
         double cpR, hRT, sR;
         nasa(t.species[k], T, iT, lT, cpR, hRT, sR);
@@ -327,8 +344,10 @@ RB200_HD inline int trhoMixed(const ReactiveB200Table& t, double T, double rho, 
     s.sound = sqrt(sound2);
     if (chem) {
         const double lnZ = log(z), lnV = log(V / vmb);
+        RB200_MIX_LOOP
         for (int k = 0; k < t.ns; ++k) {
             double pp = 0;
+            RB200_MIX_LOOP
             for (int i = 0; i < t.ns; ++i) pp += x[i] * t.aBinary[k][i] * (m.q[i] * m.q[k]);
             const double bk = t.species[k].b, num = 2.0 * b * pp - m.aa * bk;
             s.mu[k] = RT * (hk[k] - sk[k]) + RT * log(fmax(1e-300, x[k])) + RT * lnP
@@ -344,7 +363,7 @@ RB200_HD inline int trhoMixed(const ReactiveB200Table& t, double T, double rho, 
     return OK;
 }
 
-RB200_HD inline int trho(const ReactiveB200Table& t, double T, double rho, const double* Y, bool chem, Props& s,
+RB200_HD RB200_MIX_FN int trho(const ReactiveB200Table& t, double T, double rho, const double* Y, bool chem, Props& s,
                          PhaseLine* kept = nullptr) {
     if (!finiteD(T) || !finiteD(rho) || T <= 0 || rho <= 0) return BAD_INPUT;
     double x[kMaxNs] = {}, W = 0;
@@ -374,15 +393,18 @@ RB200_HD inline int partialEnthalpies(const ReactiveB200Table& t, double T, cons
     const double L = logRatio / (2.0 * kRt2 * b);
     const double fac = T * m.da - m.aa, fac2 = V + T * s.dpdT / s.dpdV;
     double dq[kMaxNs];
+    RB200_MIX_LOOP
     for (int i = 0; i < t.ns; ++i) {
         const ReactiveB200Species& sp = t.species[i];
         const double Tc = sp.a * kOmB / (sp.b * kOmA * kR), root = sqrt(T / Tc);
         const double f = 1.0 + sp.kappa * (1.0 - root);
         dq[i] = -(f > 0 ? 1.0 : -1.0) * sp.kappa / (2.0 * Tc * root);
     }
+    RB200_MIX_LOOP
     for (int k = 0; k < t.ns; ++k) {
         // a*alpha's composition derivative and its temperature derivative
         double pp = 0, dpp = 0;
+        RB200_MIX_LOOP
         for (int i = 0; i < t.ns; ++i) {
             const double pair = t.aBinary[k][i] * m.q[k] * m.q[i];
             pp += x[i] * pair;
@@ -403,7 +425,7 @@ RB200_HD inline int partialEnthalpies(const ReactiveB200Table& t, double T, cons
 // Properties at (T, p, Y) on the chosen root (AUTO: the largest, as Cantera starts
 // gas-side), with the pressure postcondition |p(T, rho) - p| <= 1e-7 max(1, p)
 // and the reported phase consistent with a GAS / LIQUID choice.
-RB200_HD inline int tp(const ReactiveB200Table& t, double T, double p, const double* Y, int choice, bool chem,
+RB200_HD RB200_MIX_FN int tp(const ReactiveB200Table& t, double T, double p, const double* Y, int choice, bool chem,
                        Props& s, PhaseLine* kept = nullptr) {
     if (!finiteD(T) || !finiteD(p) || T <= 0 || p <= 0) return BAD_INPUT;
     double x[kMaxNs] = {}, W = 0;
