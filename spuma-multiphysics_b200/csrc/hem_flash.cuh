@@ -297,7 +297,7 @@ __device__ RB200_FLASH_FN bool evaluate(const HemConst& C, double q, double mass
 __device__ __forceinline__ double energyScale(const Eval& v, double q) { return fmax(1e5 * q, v.cpD * v.T); }
 
 // Full-pivot elimination for n <= 3 with the rank test pivot > largest*n*eps.
-__device__ RB200_FLASH_FN bool solveSmall(double a[3][3], double b[3], int n, double x[3]) {
+__device__ __forceinline__ bool solveSmallBody(double a[3][3], double b[3], int n, double x[3]) {
     int column[3] = {0, 1, 2};
     double largest = 0;
 #pragma unroll
@@ -359,6 +359,9 @@ __device__ RB200_FLASH_FN bool solveSmall(double a[3][3], double b[3], int n, do
         for (int c = 0; c < 3; ++c)
             if (i < n && column[i] == c) x[c] = z[i];
     return true;
+}
+__device__ RB200_FLASH_FN bool solveSmall(double a[3][3], double b[3], int n, double x[3]) {
+    return solveSmallBody(a, b, n, x);
 }
 
 // The gas-root check by the root solve: the cubic's roots at (g.t.T, p) into

@@ -30,21 +30,33 @@ struct TwoPhasePoint {
     double gasMass, liqMass, Vp, VT, Ep, ET, energy, cpD, volume;
 };
 
-// One root's terms at (T, p), false where the general evaluation rejects it.
+// polishRoot of two roots at once: their steps are independent chains, which one
+// thread's instructions then interleave. Each stops moving at its own last step.
+__device__ __forceinline__ void polishPair(double& x, double& y, double bn, double cn, double dn) {
+    bool moveX = true, moveY = true;
+    for (int n = 0; n < 12 && (moveX || moveY); ++n) {
+        const double fx = cubicAt(x, bn, cn, dn), dx = (3.0 * x + 2.0 * bn) * x + cn;
+        const double fy = cubicAt(y, bn, cn, dn), dy = (3.0 * y + 2.0 * bn) * y + cn;
+        const double sx = fx / dx, sy = fy / dy;
+        moveX = moveX && fabs(dx) > 1e-300;
+        moveY = moveY && fabs(dy) > 1e-300;
+        x -= moveX ? sx : 0.0;
+        y -= moveY ? sy : 0.0;
+        moveX = moveX && !(fabs(sx) <= 4e-15 * fmax(1.0, fabs(x)));
+        moveY = moveY && !(fabs(sy) <= 4e-15 * fmax(1.0, fabs(y)));
+    }
+}
+
+// One root's terms at (T, p), false where the general evaluation rejects it (the
+// terms of a rejected root are not read; no branch, so two roots' chains interleave).
 __device__ __forceinline__ bool phaseTerms(const PureSpecies& sp, double T, double RT, double aa, double da, double d2a,
                                            double cpR, double hRT, double p, double V, bool gas, PhaseTerms& o) {
     const double b = sp.b, vmb = V - b, den = V * V + sp.twoB * V - sp.bb;
-    if (!(vmb > 0) || !(den > 0)) return false;
     o.V = V;
     o.iv = 1.0 / vmb;
     o.id = 1.0 / den;
     const double pe = RT * o.iv - aa * o.id;
     const double dpdV = 2.0 * aa * (V + b) * (o.id * o.id) - RT * (o.iv * o.iv), dpdT = kGas * o.iv - da * o.id;
-    if (!(pe > 0) || !(dpdV < 0) || fabs(pe - p) > 1e-7 * fmax(1.0, p)) return false;
-    if (T >= sp.tcLine) {
-        if (!gas) return false;
-    } else if ((sp.W < (sp.rhoC + (T - sp.tcLine) * sp.lineSlope) * V) != gas)
-        return false;
     o.L = log((V + sp.covolumeHi) / (V + sp.covolumeLo)) * sp.invL;
     o.eM = RT * (hRT - 1.0) + o.L * (T * da - aa);
     o.hM = o.eM + pe * V;
@@ -52,7 +64,9 @@ __device__ __forceinline__ bool phaseTerms(const PureSpecies& sp, double T, doub
     o.vp = idp;
     o.vt = -dpdT * idp;
     o.cpM = cvM + T * dpdT * o.vt;
-    return cvM > 0 && fin(o.cpM) && fin(o.eM);
+    const bool side = T >= sp.tcLine ? gas : (sp.W < (sp.rhoC + (T - sp.tcLine) * sp.lineSlope) * V) == gas;
+    return vmb > 0 && den > 0 && pe > 0 && dpdV < 0 && !(fabs(pe - p) > 1e-7 * fmax(1.0, p)) && side && cvM > 0
+           && fin(o.cpM) && fin(o.eM);
 }
 
 // Evaluation of the residuals (and their ingredients) at x = (ln p, ln T, beta).
@@ -86,13 +100,13 @@ __device__ __forceinline__ bool twoPhasePoint(const HemConst& C, const PureSpeci
     double sn, cs;
     sincos(acos(fmin(1.0, fmax(-1.0, -.5 * qc / (delta * delta2)))) * kThird, &sn, &cs);
     const double dc = delta * cs, ds = 1.7320508075688772 * delta * sn;
-    const double hi = polishRoot(center + 2.0 * dc, bn, cn, dn);
-    double lo = polishRoot(center - dc - ds, bn, cn, dn);
+    double hi = center + 2.0 * dc, lo = center - dc - ds;
+    polishPair(hi, lo, bn, cn, dn);
     if (!(lo > b)) lo = polishRoot(center - dc + ds, bn, cn, dn);  // the liquid-like root of two
     if (!(lo > b) || !(hi > lo) || !fin(hi)) return false;
-    if (!phaseTerms(sp, T, RT, aa, da, d2a, cpR, hRT, p, hi, true, o.gas)
-        || !phaseTerms(sp, T, RT, aa, da, d2a, cpR, hRT, p, lo, false, o.liq))
-        return false;
+    const bool gasOk = phaseTerms(sp, T, RT, aa, da, d2a, cpR, hRT, p, hi, true, o.gas);
+    const bool liqOk = phaseTerms(sp, T, RT, aa, da, d2a, cpR, hRT, p, lo, false, o.liq);
+    if (!gasOk || !liqOk) return false;
     o.p = p;
     o.T = T;
     o.RT = RT;
@@ -189,7 +203,7 @@ __device__ __forceinline__ int twoPhaseAdvance(const HemConst& C, const PureSpec
     }
     if (fabs(o.f0) <= C.vtol && fabs(o.f1) <= C.etol && fabs(o.f2) <= C.mutol) return TP_CONVERGED;
     double J[3][3], rhs[3] = {-o.f0, -o.f1, -o.f2}, step[3] = {0, 0, 0};
-    if (!twoPhaseJacobian(sp, s, o, J, n) || !solveSmall(J, rhs, 3, step)) return TP_FAILED;
+    if (!twoPhaseJacobian(sp, s, o, J, n) || !solveSmallBody(J, rhs, 3, step)) return TP_FAILED;
     const double limiter = fmax(fmax(1., fmax(fabs(step[0]) / .7, fabs(step[1]) / .18)), fabs(step[2]) / .3);
     const double shorten = 1.0 / limiter;
     s.s0 = step[0] * shorten;
@@ -213,7 +227,7 @@ __device__ __forceinline__ bool twoPhaseState(const HemConst& C, const PureSpeci
                                               const TwoPhasePoint& o, ReactiveThermoState& st, double& entropyD,
                                               bool& stable, Counts& n) {
     double J[3][3], rhs[3] = {-1 / s.q, o.p / (s.q * s.scale), 0}, response[3] = {0, 0, 0};
-    if (!twoPhaseJacobian(sp, s, o, J, n) || !solveSmall(J, rhs, 3, response)) return false;
+    if (!twoPhaseJacobian(sp, s, o, J, n) || !solveSmallBody(J, rhs, 3, response)) return false;
     const double squared = o.p * response[0];
     if (!fin(squared) || squared <= 0) return false;
     const double T = o.T, q = s.q, ng = o.gasMass * sp.invW, nl = o.liqMass * sp.invW;
