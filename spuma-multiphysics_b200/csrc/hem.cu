@@ -142,13 +142,9 @@ __device__ __forceinline__ int nthSetBit(unsigned mask, int n) {
 // that passes the same acceptance test: the search ends on the same fraction with
 // the same evaluation (the same routine on the same inputs) as the serial search,
 // in fewer rounds of a lone lane's FP64 latency.
-__global__ void __launch_bounds__(kPassThreads, RB200_PASS_MINBLOCKS) passQueue(const HemConst* __restrict__ Cp,
-                                                          const CellInput* __restrict__ in, size_t count,
-                                                          const unsigned* __restrict__ list, int kindBase, int kinds,
-                                                          CandRecord* rec, unsigned* counters, int queueSlot,
-                                                          unsigned long long* totals) {
-    const HemConst& C = *Cp;
-    Counts n;
+__device__ __forceinline__ void queueLoop(const HemConst& C, const CellInput* __restrict__ in, size_t count,
+                                          const unsigned* __restrict__ list, int kindBase, int kinds, CandRecord* rec,
+                                          unsigned* counters, int queueSlot, Counts& n) {
     const unsigned cells = list ? counters[LIST] : unsigned(count);
     const unsigned total = unsigned(kinds) * cells;
     const MainRecords records{rec, count};
@@ -319,26 +315,24 @@ __global__ void __launch_bounds__(kPassThreads, RB200_PASS_MINBLOCKS) passQueue(
         }
         __syncwarp();
     }
+}
+__global__ void __launch_bounds__(kPassThreads, RB200_PASS_MINBLOCKS) passQueue(const HemConst* __restrict__ Cp,
+                                                          const CellInput* __restrict__ in, size_t count,
+                                                          const unsigned* __restrict__ list, int kindBase, int kinds,
+                                                          CandRecord* rec, unsigned* counters, int queueSlot,
+                                                          unsigned long long* totals) {
+    Counts n;
+    queueLoop(*Cp, in, count, list, kindBase, kinds, rec, counters, queueSlot, n);
     flushCounts(n, totals);
 }
 
 // The five two-phase candidates of every cell, or of list[0..counters[LIST]), of a
 // pure fluid: a persistent queue of (seed, cell) items, seed-major, whose lanes run
 // one solve each in registers and take the next item when it ends, so that all
-// lanes of a warp evaluate together whatever their solves' lengths. Bound by the
-// latency of the evaluations' FP64 chains.
-#ifndef RB200_TP_MINBLOCKS
-#define RB200_TP_MINBLOCKS 3
-#endif
-__global__ void __launch_bounds__(kPassThreads, RB200_TP_MINBLOCKS) passTwoPhase(const HemConst* __restrict__ Cp,
-                                                                                const __grid_constant__ PureSpecies sp,
-                                                                                const CellInput* __restrict__ in,
-                                                                                size_t count,
-                                                                                const unsigned* __restrict__ list,
-                                                                                CandRecord* rec, unsigned* counters,
-                                                                                unsigned long long* totals) {
-    const HemConst& C = *Cp;
-    Counts n;
+// lanes of a warp evaluate together whatever their solves' lengths.
+__device__ __forceinline__ void twoPhaseLoop(const HemConst& C, const PureSpecies& sp, const CellInput* __restrict__ in,
+                                             size_t count, const unsigned* __restrict__ list, CandRecord* rec,
+                                             unsigned* counters, Counts& n) {
     const unsigned cells = list ? counters[LIST] : unsigned(count), total = 5u * cells, lane = threadIdx.x & 31u;
     TwoPhaseSolve s;
     TwoPhasePoint o;
@@ -391,19 +385,6 @@ __global__ void __launch_bounds__(kPassThreads, RB200_TP_MINBLOCKS) passTwoPhase
         }
         __syncwarp();
     }
-    flushCounts(n, totals);
-}
-
-// The five two-phase candidates of the listed (or all) cells: in registers where one
-// species' tables serve both phases and the Jacobian is analytic, else through the
-// work queue.
-void launchSeeds(const HemConst& hostConst, const HemConst* cst, const CellInput* in, size_t count,
-                 const unsigned* cells, CandRecord* rec, unsigned* counters, unsigned long long* totals, int blocks,
-                 cudaStream_t s) {
-    if (hostConst.samePure && hostConst.analyticJacobian)
-        passTwoPhase<<<blocks, kPassThreads, 0, s>>>(cst, hostConst.gas, in, count, cells, rec, counters, totals);
-    else passQueue<<<blocks, kPassThreads, 0, s>>>(cst, in, count, cells, 2, 5, rec, counters, Q_B, totals);
-    check(cudaGetLastError(), "two-phase seeds");
 }
 
 __device__ __forceinline__ bool gasDecides(const HemConst& C, const CandRecord& gas) {
@@ -701,15 +682,10 @@ __global__ void __launch_bounds__(kGasThreads, RB200_GAS_MINBLOCKS) passGas(
 // machines restate (bit for bit the queue's candidates), selects as
 // selectCandidates does (the stable candidate of larger entropy, the all-gas one
 // on a tie) and writes the outputs; a cell with neither goes to the restart list.
-__global__ void __launch_bounds__(kPassThreads, RB200_PASS_MINBLOCKS) passSinglePhase(const HemConst* __restrict__ Cp,
-                                                                const CellInput* __restrict__ in,
-                                                                const unsigned* __restrict__ general,
-                                                                ReactiveThermoState* state,
-                                                                ReactiveTransportState* transport, int* success,
-                                                                unsigned* fallback, unsigned* counters,
-                                                                unsigned long long* totals) {
-    const HemConst& C = *Cp;
-    Counts n;
+__device__ __forceinline__ void singlePhaseLoop(const HemConst& C, const CellInput* __restrict__ in,
+                                                const unsigned* __restrict__ general, ReactiveThermoState* state,
+                                                ReactiveTransportState* transport, int* success, unsigned* fallback,
+                                                unsigned* counters, Counts& n) {
     const unsigned items = counters[GENERAL];
     for (size_t base = blockIdx.x * size_t(blockDim.x); base < items; base += size_t(blockDim.x) * gridDim.x) {
         const size_t item = base + threadIdx.x;
@@ -756,6 +732,50 @@ __global__ void __launch_bounds__(kPassThreads, RB200_PASS_MINBLOCKS) passSingle
         }
         appendTo(fallback, counters + FALLBACK, restart, c);
     }
+}
+__global__ void __launch_bounds__(kPassThreads, RB200_PASS_MINBLOCKS) passSinglePhase(const HemConst* __restrict__ Cp,
+                                                                const CellInput* __restrict__ in,
+                                                                const unsigned* __restrict__ general,
+                                                                ReactiveThermoState* state,
+                                                                ReactiveTransportState* transport, int* success,
+                                                                unsigned* fallback, unsigned* counters,
+                                                                unsigned long long* totals) {
+    Counts n;
+    singlePhaseLoop(*Cp, in, general, state, transport, success, fallback, counters, n);
+    flushCounts(n, totals);
+}
+
+// True where passSearch serves: one species' tables for both phases, analytic Jacobian.
+bool searchInRegisters(const HemConst& C) { return C.samePure && C.analyticJacobian; }
+
+// The candidates that passGas left, of a pure fluid with the analytic Jacobian, in
+// one launch: the listed single-phase cells, the one-phase candidates of the cells in
+// the dome, then all two-phase candidates. Each part is a loop over its own items
+// that a warp leaves when they run out; the few long solves are in the first two,
+// and the warps that hold one finish it while the others go on to the third, whose
+// items fill the device. As launches of their own the parts' tails add up: 1,000,000
+// cells, 60% saturated, spent 2.44 ms on a few hundred one-phase solves and 3.28 ms
+// on three million two-phase ones. `parts` (SEARCH_*): what to run.
+//
+// Bound by the latency of the evaluations' FP64 chains: one solve a lane, at the 168
+// registers that three blocks a multiprocessor leave (at four, spills: 65,537 cells
+// 14.2 ms against 10.5 ms).
+enum : int { SEARCH_GENERAL = 1, SEARCH_ONE_PHASE = 2, SEARCH_TWO_PHASE = 4 };
+__global__ void __launch_bounds__(kPassThreads, 3) passSearch(const HemConst* __restrict__ Cp,
+                                                             const __grid_constant__ PureSpecies sp, int parts,
+                                                             const CellInput* __restrict__ in, size_t count,
+                                                             const unsigned* __restrict__ list,
+                                                             const unsigned* __restrict__ general, CandRecord* rec,
+                                                             ReactiveThermoState* state,
+                                                             ReactiveTransportState* transport, int* success,
+                                                             unsigned* fallback, unsigned* counters,
+                                                             unsigned long long* totals) {
+    Counts n;
+    if (parts & SEARCH_GENERAL) singlePhaseLoop(*Cp, in, general, state, transport, success, fallback, counters, n);
+    __syncwarp();
+    if (parts & SEARCH_ONE_PHASE) queueLoop(*Cp, in, count, list, 0, 2, rec, counters, Q_A, n);
+    __syncwarp();
+    if (parts & SEARCH_TWO_PHASE) twoPhaseLoop(*Cp, sp, in, count, list, rec, counters, n);
     flushCounts(n, totals);
 }
 
@@ -1120,7 +1140,7 @@ struct HemDevice {
     ReactiveThermoState* dguess = nullptr;
     ReactiveThermoState* dout = nullptr;
     int* dsuccess = nullptr;
-    int passBlocks = 0;
+    int passBlocks = 0, searchBlocks = 0;
     int domeBuilt = 0;  // grid points of the two-phase bound (0: none for this model)
     size_t bytes = 0;
     std::vector<void*> blocks;
@@ -1185,6 +1205,17 @@ struct HemDevice {
         check(cudaMemsetAsync(counters, 0, NCOUNTERS * sizeof(unsigned), s), "memset counters");
         const unsigned* selectList = !hostConst.stableGasPrune && hostConst.domeN ? list : nullptr;
         const bool fused = cons && !hostConst.stableGasPrune && hostConst.domeN;
+        // passSearch where it applies, else the work queue
+        const bool fast = searchInRegisters(hostConst);
+        auto searchCandidates = [&](int parts, int kindBase, int kinds, const unsigned* cells) {
+            if (parts)
+                passSearch<<<searchBlocks, kPassThreads, 0, s>>>(cst, hostConst.gas, parts, in, count, cells, general, rec,
+                                                                 state, transport, success, fallback, counters, totals);
+            else
+                passQueue<<<passBlocks, kPassThreads, 0, s>>>(cst, in, count, cells, kindBase, kinds, rec, counters,
+                                                              kindBase ? Q_B : Q_A, totals);
+            check(cudaGetLastError(), "candidate search");
+        };
         if (cons && !fused) {
             inputsFromConserved<<<gridFor(count, 256), 256, 0, s>>>(cst, cons, stride, count, 1, seed, in);
             check(cudaGetLastError(), "inputs");
@@ -1195,7 +1226,7 @@ struct HemDevice {
             check(cudaGetLastError(), "passQueue");
             compactSeedCells<<<gridFor(count, 256), 256, 0, s>>>(cst, rec, count, list, counters);
             check(cudaGetLastError(), "compactSeedCells");
-            launchSeeds(hostConst, cst, in, count, list, rec, counters, totals, passBlocks, s);
+            searchCandidates(fast ? SEARCH_TWO_PHASE : 0, 2, 5, list);
         } else if (hostConst.domeN) {
             // single-phase cells one thread each (selected and written there), the
             // rest through the work queue and the selection below
@@ -1207,17 +1238,14 @@ struct HemDevice {
                 passGas<false><<<blocks, kGasThreads, 0, s>>>(gasPass, cst, in, nullptr, 0, nullptr, count, state,
                                                               transport, success, list, general, counters, totals);
             check(cudaGetLastError(), "passGas");
-            passSinglePhase<<<passBlocks, kPassThreads, 0, s>>>(cst, in, general, state, transport, success, fallback,
-                                                                counters, totals);
-            check(cudaGetLastError(), "passSinglePhase");
-            passQueue<<<passBlocks, kPassThreads, 0, s>>>(cst, in, count, list, 0, 2, rec, counters, Q_A, totals);
-            check(cudaGetLastError(), "passQueue");
-            launchSeeds(hostConst, cst, in, count, list, rec, counters, totals, passBlocks, s);
-        } else {
-            passQueue<<<passBlocks, kPassThreads, 0, s>>>(cst, in, count, nullptr, 0, 2, rec, counters, Q_A, totals);
-            check(cudaGetLastError(), "passQueue");
-            launchSeeds(hostConst, cst, in, count, nullptr, rec, counters, totals, passBlocks, s);
-        }
+            if (fast) searchCandidates(SEARCH_GENERAL | SEARCH_ONE_PHASE | SEARCH_TWO_PHASE, 0, 7, list);
+            else {
+                passSinglePhase<<<passBlocks, kPassThreads, 0, s>>>(cst, in, general, state, transport, success,
+                                                                    fallback, counters, totals);
+                check(cudaGetLastError(), "passSinglePhase");
+                searchCandidates(0, 0, 7, list);
+            }
+        } else searchCandidates(fast ? SEARCH_ONE_PHASE | SEARCH_TWO_PHASE : 0, 0, 7, nullptr);
         selectCandidates<<<gridFor(count, 256), 256, 0, s>>>(cst, rec, count, selectList, state, transport, success,
                                                              fallback, counters);
         check(cudaGetLastError(), "selectCandidates");
@@ -1373,6 +1401,8 @@ void* create(const void* raw, size_t bytes, size_t capacity, bool hostPath, char
         check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, passQueue, kPassThreads, 0), "occupancy");
         check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d->device), "attribute");
         d->passBlocks = std::max(1, perSm) * std::max(1, sms);
+        check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, passSearch, kPassThreads, 0), "occupancy");
+        d->searchBlocks = std::max(1, perSm) * std::max(1, sms);
         const HemConst& h = d->hostConst;
         d->gasPass = GasPass{h.gas, h.Tmin, h.Tmax, h.pmin, h.pmax, h.vtol, h.etol, h.gasTmin, h.gasTmax,
                              h.liquidFloor, h.liquidTmin, h.liquidTc, h.enforceBounds, h.scalarRecovery};
@@ -2108,14 +2138,20 @@ extern "C" int reactive_gpu_hem_run_static_v3(const void* model, size_t modelByt
         check(cudaMemsetAsync(totals, 0, NTOTALS * sizeof(unsigned long long), s), "clear totals");
         inputsFromConserved<<<gridFor(count, 256), 256, 0, s>>>(cst, conserved, stride, count, 1, seed, in);
         check(cudaGetLastError(), "inputs");
+        const bool fast = searchInRegisters(hostConst);
+        auto searchCandidates = [&](int parts, int kindBase, int kinds, const unsigned* cells) {
+            if (parts)
+                passSearch<<<blocks, kPassThreads, 0, s>>>(cst, hostConst.gas, parts, in, count, cells, nullptr, rec, state,
+                                                           transport, success, fallback, counters, totals);
+            else
+                passQueue<<<blocks, kPassThreads, 0, s>>>(cst, in, count, cells, kindBase, kinds, rec, counters,
+                                                          kindBase ? Q_B : Q_A, totals);
+        };
         if (hostConst.stableGasPrune) {
             passQueue<<<blocks, kPassThreads, 0, s>>>(cst, in, count, nullptr, 0, 2, rec, counters, Q_A, totals);
             compactSeedCells<<<gridFor(count, 256), 256, 0, s>>>(cst, rec, count, list, counters);
-            launchSeeds(hostConst, cst, in, count, list, rec, counters, totals, blocks, s);
-        } else {
-            passQueue<<<blocks, kPassThreads, 0, s>>>(cst, in, count, nullptr, 0, 2, rec, counters, Q_A, totals);
-            launchSeeds(hostConst, cst, in, count, nullptr, rec, counters, totals, blocks, s);
-        }
+            searchCandidates(fast ? SEARCH_TWO_PHASE : 0, 2, 5, list);
+        } else searchCandidates(fast ? SEARCH_ONE_PHASE | SEARCH_TWO_PHASE : 0, 0, 7, nullptr);
         check(cudaGetLastError(), "passQueue");
         selectCandidates<<<gridFor(count, 256), 256, 0, s>>>(cst, rec, count, nullptr, state, transport, success,
                                                              fallback, counters);
