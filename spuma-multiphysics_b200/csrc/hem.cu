@@ -438,7 +438,12 @@ struct GasPass {
 //                            is the liquid's; above it the reverse,
 //                rho, T      the reported phase is the other one, or the species'
 //                            or the liquid's range excludes the temperature,
-//                each by a margin of 1e-3 or more (1e-5 for the temperature ranges).
+//                p           it is out of range,
+//                each by a margin of 1e-3 or more (1e-5 for the temperature ranges; the
+//                pressure range three times what T' can wander: of a liquid stretched
+//                to a slightly negative pressure only that keeps its long solve out,
+//                and one such solve was 2.4 ms of a batch of any size).
+// The margins belong to tolerances of 1e-9; with larger ones nothing is skipped.
 // Nearer the critical temperature the spinodal's edge is left out by a wide margin
 // instead (|x| > .1: a T' on it would be 7% off, which takes cp/cv > 1e7 and a pair
 // of roots inside the near-repeated band), and saturation is not used. An isochore
@@ -449,7 +454,7 @@ struct GasPass {
 __device__ __forceinline__ int singlePhaseImpossible(const GasPass& G, const HemConst& C, double q, double e, double gT) {
     const PureSpecies& sp = G.gas;
     DensityTerms d;
-    if (!isfinite(e) || !densityTerms(sp, q, d)) return 0;
+    if (!(G.etol <= 1.01e-9 && G.vtol <= 1.01e-9) || !isfinite(e) || !densityTerms(sp, q, d)) return 0;
     GasProbe g;
     double T = clampd(gT, G.Tmin, G.Tmax);
     bool settled = false;
@@ -465,7 +470,9 @@ __device__ __forceinline__ int singlePhaseImpossible(const GasPass& G, const Hem
     const bool cold = T < .985 * sp.Tc;
     if (g.dpdV > (cold ? -1e-3 : .1) * scale) return SKIP_GAS | SKIP_LIQUID;
     if (!cold && !(g.dpdV < -.1 * scale)) return 0;
-    if (g.p < G.pmin - 1e-3 * thermal || g.p > G.pmax + 1e-3 * thermal) return SKIP_GAS | SKIP_LIQUID;
+    // T' is T to etol (1 + 10/|x|), and T dp/dT stays below three thermal pressures
+    const double margin = thermal * (1e-6 - 1e-7 * scale / g.dpdV);
+    if (g.p < G.pmin - margin || g.p > G.pmax + margin) return SKIP_GAS | SKIP_LIQUID;
     if (!(g.p > 0)) return 0;
     int skip = 0;
     if (T < .999 * sp.Tc) {
