@@ -506,13 +506,13 @@ __device__ __forceinline__ int singlePhaseImpossible(const GasPass& G, const Hem
 // temperatures, so its bits), decided without a root solve. False hands the cell
 // to the general pass.
 //
-// The bracket probe of a solve that moves (scalarGas widens the seed by `radius`
-// toward the residual's zero before its first Newton step) is checked for
-// acceptance only, by its mechanical half: its energy residual's sign is known,
-// since cv > 0 makes the residual rise with T, once the solution lies at least
-// half a radius inside the bracket (cv times half a radius is orders of magnitude
-// above the tolerance). Every other course (a step out of the bracket or past half
-// a radius, a rejected probe) goes to the general pass.
+// scalarGas widens the seed by doubled radii toward the residual's zero before its
+// first Newton step; its probes confine the steps and do not enter them. With cv > 0 the
+// residual rises with T, so the solution tells which probe ended the bracket: Newton
+// first, then each of those probes is checked for acceptance by its mechanical half
+// (5% of a radius from the solution, where cv is orders of magnitude above the
+// tolerance), and the steps must have stayed inside. Every other course (a step out of
+// the bracket, a rejected probe, a probe next to the solution) goes to the general pass.
 __device__ __forceinline__ bool gasCell(const GasPass& G, const HemConst& C, double q, double e, double gT,
                                         unsigned& phases, double* row) {
     const PureSpecies& sp = G.gas;
@@ -520,13 +520,14 @@ __device__ __forceinline__ bool gasCell(const GasPass& G, const HemConst& C, dou
     if (!isfinite(e) || !densityTerms(sp, q, d)) return false;
     GasProbe g;
     bool clear;
-    auto mechanics = [&](double T, GasProbe& at, bool& apart) {
+    auto mechanics = [&](double T, GasProbe& at) {
         return probeMechanics(sp, d, T, at) && at.p >= G.pmin && at.p <= G.pmax && T >= G.Tmin && T <= G.Tmax
-               && !(G.enforceBounds && (T < G.gasTmin || T > G.gasTmax)) && gasRootIsV0(sp, d, at, apart) == 1;
+               && !(G.enforceBounds && (T < G.gasTmin || T > G.gasTmax))
+               && (plainGasRoot(sp, d, at) || gasRootIsV0(sp, d, at, clear) == 1);
     };
     const double T0 = clampd(gT, G.Tmin, G.Tmax);
     ++phases;
-    if (!(T0 > 0) || !mechanics(T0, g, clear) || !probeEnergy(sp, d, g)) return false;
+    if (!(T0 > 0) || !mechanics(T0, g) || !probeEnergy(sp, d, g)) return false;
     double T = T0, F = fma(d.iV, g.eM, -e), cv = __dmul_rn(d.iV, g.cvM);
     const double cp0 = __dmul_rn(probeCp(g, 1.0 / g.dpdV), sp.invW);
     const double tolerance = G.etol * fmax(1e5 * q, q * cp0 * T);
@@ -539,8 +540,7 @@ __device__ __forceinline__ bool gasCell(const GasPass& G, const HemConst& C, dou
         if (!(upper - lower > .75 * radius)) return false;
         {
             GasProbe edge;
-            bool unused;
-            if (!mechanics(F > 0 ? lower : upper, edge, unused)) return false;
+            if (!mechanics(F > 0 ? lower : upper, edge)) return false;
         }
         while (fabs(F) > tolerance) {
             if (F > 0) upper = T; else lower = T;
@@ -548,13 +548,13 @@ __device__ __forceinline__ bool gasCell(const GasPass& G, const HemConst& C, dou
             if (!(next > lower && next < upper) || !(fabs(next - T0) <= .5 * radius) || ++it > 8) return false;
             T = next;
             ++phases;
-            if (!mechanics(T, g, clear) || !probeEnergy(sp, d, g)) return false;
+            if (!mechanics(T, g) || !probeEnergy(sp, d, g)) return false;
             F = fma(d.iV, g.eM, -e);
             cv = __dmul_rn(d.iV, g.cvM);
             if (!isfinite(F) || !isfinite(cv) || !(cv > 0)) return false;
         }
     }
-    if (!clear || !belowSaturation(C, g.p, T)) return false;
+    if (gasRootIsV0(sp, d, g, clear) != 1 || !clear || !belowSaturation(C, g.p, T)) return false;
     PhaseProps ph;
     ChemTerms chem;
     double sR;
@@ -567,8 +567,9 @@ __device__ __forceinline__ bool gasCell(const GasPass& G, const HemConst& C, dou
     row[0] = g.p;
     row[1] = T;
     row[2] = q;
-    row[3] = v.energy / q;
-    row[4] = v.entropyD / q;
+    const double specific = 1.0 / q;
+    row[3] = v.energy * specific;
+    row[4] = v.entropyD * specific;
     row[5] = row[6] = v.soundFrozen;
     row[7] = 0;
     row[8] = eres;
@@ -578,7 +579,7 @@ __device__ __forceinline__ bool gasCell(const GasPass& G, const HemConst& C, dou
     row[13] = q;
     row[14] = row[15] = row[16] = row[17] = 0;
     row[18] = q;
-    row[19] = v.cpD / q;
+    row[19] = v.cpD * specific;
     row[20] = v.cv;
     row[21] = __hiloint2double(it, 0);  // iterations, activeLiquids
     return true;
@@ -603,7 +604,7 @@ __device__ __forceinline__ bool gasCell(const GasPass& G, const HemConst& C, dou
 // states and touches no other cell's.
 constexpr int kGasThreads = 128, kStageRow = 23;  // 22 words a record and one of padding against bank conflicts
 #ifndef RB200_GAS_MINBLOCKS
-#define RB200_GAS_MINBLOCKS 5
+#define RB200_GAS_MINBLOCKS 6
 #endif
 template <bool FROM_CONSERVED>
 __global__ void __launch_bounds__(kGasThreads, RB200_GAS_MINBLOCKS) passGas(

@@ -72,7 +72,7 @@ enum : int { SKIP_TWO_PHASE = 1, SKIP_GAS = 2, SKIP_LIQUID = 4 };
 // line widened by the margins: the two-phase seeds would all fail.
 __device__ inline bool twoPhaseImpossible(const HemConst& C, double q, double e) {
     if (C.domeN < 4 || !(q > 0) || !isfinite(q) || !isfinite(e)) return false;
-    const double v = 1 / q, u = e / q;
+    const double v = 1.0 / q, u = e * v;
     if (v < C.domeVlo * (1 - C.domeMarginV) || v > C.domeVhi * (1 + C.domeMarginV)) return true;
     int j = int(floor((log(v) - C.domeLnV0) * C.domeInvStep));
     j = j < 1 ? 1 : (j > C.domeN - 3 ? C.domeN - 3 : j);
@@ -424,6 +424,18 @@ __device__ __forceinline__ int gasRootIsV0(const PureSpecies& sp, const DensityT
     return -1;
 }
 
+// True where gasRootIsV0 needs no root: V0 past 4b, more than the cubic's critical volume
+// (3.951b, whatever a), on a falling stretch of the isotherm is on its gas branch, so
+// V0 is the largest root; where it is the only one below Tc it is above the classification
+// centre (dp/dV < 0 at v = V/b bounds a, and with that bound V0 > centre reads
+// v^3 - 3v^2 - 3v - 3 > 0, whose root is the critical volume). The density on the gas side
+// of the reported-phase line. For points on the way to a solution: the accepted one is
+// checked by its roots (gasRootIsV0), for its liquid's sake too.
+__device__ __forceinline__ bool plainGasRoot(const PureSpecies& sp, const DensityTerms& d, const GasProbe& g) {
+    return d.V >= 4.0 * sp.b && g.dpdV <= -1e-3 * (g.RT * d.iv2)
+           && (g.T >= sp.tcLine || d.q < fma(__dsub_rn(g.T, sp.tcLine), sp.lineSlope, sp.rhoC) * (1 - 1e-9));
+}
+
 // Energy residual of the all-gas state at (T, rho) and the gas-root check: the
 // probe at (T, rho), then the gas root of the cubic at the resulting pressure must
 // be that density: decided by gasRootIsV0 where its margins allow, else by the
@@ -734,8 +746,9 @@ __device__ inline void stateFromEval(const Eval& v, double q, const CandidateOut
     s.p = v.p;
     s.T = v.T;
     s.rho = q;
-    s.e = v.energy / q;
-    s.entropy = v.entropyD / q;
+    const double specific = 1.0 / q;
+    s.e = v.energy * specific;
+    s.entropy = v.entropyD * specific;
     s.soundFrozen = v.soundFrozen;
     s.soundEquilibrium = o.soundEq;
     s.volumeResidual = o.vres;
@@ -750,7 +763,7 @@ __device__ inline void stateFromEval(const Eval& v, double q, const CandidateOut
     s.liquidMass[0] = v.liqMass;
     s.liquidMass[1] = 0;
     s.gasMass = v.gasMass;
-    s.cp = v.cpD / q;
+    s.cp = v.cpD * specific;
     s.cv = v.cv;
     s.activeLiquids = v.liqMass > 0 ? 1 : 0;
     s.iterations = o.iterations;

@@ -234,6 +234,7 @@ __device__ __forceinline__ bool twoPhaseState(const HemConst& C, const PureSpeci
     GasProbe probe;  // for the ideal gas' entropy
     probe.T = T;
     probe.iT = 1.0 / T;
+    probe.lnT = log(T);
     const double sR = probeEntropy(sp, probe), lg = log(o.RT * o.gas.iv * sp.invRefP);
     entropyD = ng * (kGas * (sR - lg) + o.gas.L * o.da) + nl * (kGas * (sR - (lg + o.lnIv)) + o.liq.L * o.da);
     Eval v{};

@@ -147,6 +147,7 @@ __device__ __forceinline__ bool densityTerms(const PureSpecies& sp, double q, De
 // (probeEnergy) cp/R and h/RT of the ideal gas, the molar energy and cv.
 struct GasProbe {
     double T, iT, RT, alphaRoot, aa, da, d2a, p, dpdV, dpdT, cpR, hRT, eM, cvM;
+    double lnT;  // where the polynomials read it
 };
 // The mechanical half of a probe, false at the cusp of |1 + kappa (1 - sqrt(T/Tc))|.
 __device__ __forceinline__ bool probeTerms(const PureSpecies& sp, const DensityTerms& d, double T, GasProbe& g) {
@@ -179,8 +180,9 @@ __device__ __forceinline__ bool probeEnergy(const PureSpecies& sp, const Density
     g.cpR = fma(T, fma(T, fma(T, fma(T, n.c4, n.c3), n.c2), n.c1), n.c0);
     g.hRT = fma(T, fma(T, fma(T, fma(T, n.h4, n.h3), n.h2), n.h1), fma(n.hc, iT, n.c0));
     if (n.m1 != 0 || n.m2 != 0) {
+        g.lnT = log(T);
         g.cpR = fma(fma(n.m2, iT, n.m1), iT, g.cpR);
-        g.hRT = fma(fma(n.m1, log(T), -__dmul_rn(n.m2, iT)), iT, g.hRT);
+        g.hRT = fma(fma(n.m1, g.lnT, -__dmul_rn(n.m2, iT)), iT, g.hRT);
     }
     g.eM = fma(g.RT, __dsub_rn(g.hRT, 1.0), __dmul_rn(d.L, fma(T, g.da, -g.aa)));
     g.cvM = fma(kGas, __dsub_rn(g.cpR, 1.0), __dmul_rn(__dmul_rn(d.L, T), g.d2a));
@@ -190,12 +192,13 @@ __device__ __forceinline__ bool probeEnergy(const PureSpecies& sp, const Density
 __device__ __forceinline__ double probeCp(const GasProbe& g, double idp) {
     return fma(-__dmul_rn(g.T, g.dpdT), __dmul_rn(g.dpdT, idp), g.cvM);
 }
-// The probe's s/R of the ideal gas (its logarithm only the accepted point needs).
+// The probe's s/R of the ideal gas (only the accepted point needs it).
 __device__ __forceinline__ double probeEntropy(const PureSpecies& sp, const GasProbe& g) {
     const NasaPowers& n = sp.powers[nasaRegion(sp, g.T)];
-    const double T = g.T;
-    double s = fma(T, fma(T, fma(T, fma(T, n.s4, n.s3), n.s2), n.c1), fma(n.c0, log(T), n.sc));
-    if (n.m1 != 0 || n.m2 != 0) s = fma(-fma(__dmul_rn(.5, n.m2), g.iT, n.m1), g.iT, s);
+    const bool low = n.m1 != 0 || n.m2 != 0;
+    const double T = g.T, lnT = low ? g.lnT : log(T);
+    double s = fma(T, fma(T, fma(T, fma(T, n.s4, n.s3), n.s2), n.c1), fma(n.c0, lnT, n.sc));
+    if (low) s = fma(-fma(__dmul_rn(.5, n.m2), g.iT, n.m1), g.iT, s);
     return s;
 }
 
