@@ -1445,6 +1445,291 @@ __device__ __forceinline__ HllBar hllReverse(double wf, double unL, double unR, 
     return b;
 }
 
+// gb += nb * d nu_t / d g of one cell (the WALE eddy viscosity of its gradient g, the
+// Nicoud-Ducros relation of wale.cuh:
+// nu_t = (Cw Delta)^2 |g|_max (Sd:Sd)^(3/2) / ((S:S)^(5/2) + (Sd:Sd)^(5/4))
+// with the invariants of g / |g|_max; zero where the forward gives zero), by a
+// reverse pass derived by hand.
+__device__ __forceinline__ void waleReverse(const CartView& v, double invV, const double* g, double nb, double* gb) {
+    // nu_t = (Cw Delta)^2 |g|_max ratio(g / |g|_max) and ratio is homogeneous of
+    // degree one, so d nu_t / d g = (Cw Delta)^2 d ratio / d h at h = g / |g|_max
+    // (the normalisation's own derivative cancels). With ratio = dd^(3/2) /
+    // (ss^(5/2) + dd^(5/4)), ss = S:S (S = sym h), dd = D:D (D = dev sym(h h)):
+    // d ss / d h = 2 S and d dd / d h = G h^T + h^T G with G = 2 D.
+    if (nb == 0) return;
+    double scale = 0;
+#pragma unroll
+    for (int t = 0; t < 9; ++t) scale = fmax(scale, ::fabs(g[t]));
+    const double delta = cbrt(1 / invV);
+    if (scale == 0 || v.cw == 0 || delta == 0) return;
+    double h[9];
+#pragma unroll
+    for (int t = 0; t < 9; ++t) h[t] = g[t] / scale;
+    double sq[9];
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+        for (int b = 0; b < 3; ++b) sq[3 * a + b] = h[3 * a] * h[b] + h[3 * a + 1] * h[3 + b] + h[3 * a + 2] * h[6 + b];
+    const double trace = sq[0] + sq[4] + sq[8];
+    double S[9], G[9], ss = 0, dd = 0;
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+        for (int b = 0; b < 3; ++b) {
+            const double sab = .5 * (h[3 * a + b] + h[3 * b + a]);
+            double dab = .5 * (sq[3 * a + b] + sq[3 * b + a]);
+            if (a == b) dab -= trace / 3.0;
+            S[3 * a + b] = sab;
+            G[3 * a + b] = 2 * dab;
+            ss += sab * sab;
+            dd += dab * dab;
+        }
+    if (!(dd > 0)) return;
+    const double rootD = sqrt(dd), quarter = sqrt(rootD), rootS = sqrt(ss);
+    const double numerator = dd * rootD, denominator = ss * ss * rootS + dd * quarter;
+    const double den2 = denominator * denominator;
+    const double rDd = (1.5 * rootD * denominator - numerator * 1.25 * quarter) / den2;
+    const double rSs = -numerator * 2.5 * ss * rootS / den2;
+    const double weight = nb * (v.cw * delta * v.cw * delta);
+#pragma unroll
+    for (int u = 0; u < 3; ++u)
+#pragma unroll
+        for (int z = 0; z < 3; ++z) {
+            double dDd = 0;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) dDd += G[3 * u + k] * h[3 * z + k] + G[3 * k + z] * h[3 * k + u];
+            gb[3 * u + z] += weight * (rDd * dDd + rSs * 2 * S[3 * u + z]);
+        }
+}
+
+// What a cell's faces add to its adjoints.
+template <int NS> struct CellBar {
+    double q[NS + 4], u[3], p, c, T, rho, g[9], nut;
+};
+
+// The interior face on side S of cell c (axis and orientation compile-time: the
+// normal is +e_axis and the face's left cell is c on an odd side): its part of
+// c's adjoints. wc: c's adjoint weights over its volume. VISCOUS: also the adjoints
+// of c's gradient and eddy viscosity.
+template <int NS, int S, bool VISCOUS>
+__device__ __forceinline__ void interiorFaceBar(const CartView& v, const double* __restrict__ q,
+                                                const double* __restrict__ grad, const double* __restrict__ nut,
+                                                const double* __restrict__ w, size_t nb, const CellData& C,
+                                                const double* gC, double nutC, const double* wc, CellBar<NS>& o) {
+    constexpr int AX = S >> 1;
+    constexpr bool LEFT = S & 1;
+    CellData O;
+    loadCell<NS>(v, q, nb, O, true);
+    const double ivn = v.invV[nb], area = v.area[AX];
+    double Wa[NS + 4], SC = 0, SO = 0;
+#pragma unroll
+    for (int kk = 0; kk < NS + 4; ++kk) {
+        const double wn = w[size_t(kk) * v.cells + nb] * ivn;
+        Wa[kk] = area * (LEFT ? wn - wc[kk] : wc[kk] - wn);
+        SC += Wa[kk] * C.q[kk];
+        SO += Wa[kk] * O.q[kk];
+    }
+    const double We = Wa[NS + 3];
+    if constexpr (LEFT) {
+        const HllBar b = hllReverse(v.waveFactor, C.u[AX], O.u[AX], C.c, O.c, C.p, O.p, SC, SO, Wa[NS + AX], We);
+#pragma unroll
+        for (int kk = 0; kk < NS + 4; ++kk) o.q[kk] += Wa[kk] * b.qL;
+        o.u[AX] += b.unL;
+        o.p += b.pL;
+        o.c += b.cL;
+    } else {
+        const HllBar b = hllReverse(v.waveFactor, O.u[AX], C.u[AX], O.c, C.c, O.p, C.p, SO, SC, Wa[NS + AX], We);
+#pragma unroll
+        for (int kk = 0; kk < NS + 4; ++kk) o.q[kk] += Wa[kk] * b.qR;
+        o.u[AX] += b.unR;
+        o.p += b.pR;
+        o.c += b.cR;
+    }
+    const double away = LEFT ? -v.invDist[AX] : v.invDist[AX];  // d(face difference)/d(c's value)
+    if constexpr (VISCOUS) {
+        // the forward's corrected face gradient: its column AX is the difference quotient
+        double g[9], t[3], av[3];
+        const double nutO = v.wale ? nut[nb] : 0.0;
+#pragma unroll
+        for (int k = 0; k < 9; ++k) g[k] = .5 * (gC[k] + grad[size_t(k) * v.cells + nb]);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) g[a * 3 + AX] = (C.u[a] - O.u[a]) * away;
+        const double div = g[0] + g[4] + g[8];
+        const double mu = v.viscosity + (v.wale ? .5 * (C.rho * nutC + O.rho * nutO) : 0.0);
+        double jmu = 0;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            t[a] = g[a * 3 + AX] + g[AX * 3 + a] - (a == AX ? 2.0 / 3.0 * div : 0.0);
+            av[a] = -(Wa[NS + a] + We * (.5 * (C.u[a] + O.u[a])));
+            jmu += av[a] * t[a];
+        }
+        const double an = av[AX];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            // dJ/dt = dJ/dG' n; dJ/du_bar = -W_E A tau
+            const double rn = mu * (a == AX ? 4.0 / 3.0 * an : av[a]);
+            o.u[a] += rn * away - .5 * (We * (mu * t[a]));
+        }
+        if (v.wale) {
+            o.rho += .5 * (jmu * nutC);
+            o.nut += .5 * (jmu * C.rho);
+        }
+        // dJ/dG = dJ/dG' (I - n n^T), half of it c's: row AX off the normal column, and
+        // the trace's two other diagonal entries
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            if (d == AX) continue;
+            o.g[AX * 3 + d] += .5 * (mu * av[d]);
+            o.g[d * 3 + d] -= .5 * (mu * (2.0 / 3.0 * an));
+        }
+    }
+    if (v.conductivity > 0) o.T -= We * v.conductivity * away;
+}
+
+// The box-side faces of cell c: their part of its adjoints (sides are few: a routine
+// of its own, on sums in memory, keeps the interior's in registers).
+template <int NS>
+__device__ __noinline__ void boundaryFaceBars(const CartView& v, const double* __restrict__ q,
+                                              const ReactiveTransportState* __restrict__ st, int i, int j, int k,
+                                              const CellData& C, const double* gC, double nutC, const double* wc,
+                                              bool viscous, CellBar<NS>& o) {
+#pragma unroll 1
+    for (int s = 0; s < 6; ++s) {
+        if (hasNeighbour(v, s, i, j, k)) continue;
+        const int axis = s >> 1;
+        CellData O;  // the other side
+        double Wa[NS + 4];
+        const ReactiveTransportFace& f = sideFace(v, s, i, j, k);
+        const int kind = f.kind;
+        boundaryRight<NS>(v, q, st, f, axis, C, O, true);
+        const double sgn = (s & 1) ? 1.0 : -1.0, area = f.area, wf = f.ownerWeight, invDist = 1 / f.distance;
+#pragma unroll
+        for (int kk = 0; kk < NS + 4; ++kk) Wa[kk] = -area * wc[kk];
+        const CellData& L = C;
+        const CellData& R = O;
+        double SL = 0, SR = 0;
+#pragma unroll
+        for (int kk = 0; kk < NS + 4; ++kk) { SL += Wa[kk] * L.q[kk]; SR += Wa[kk] * R.q[kk]; }
+        const HllBar b = hllReverse(v.waveFactor, L.u[axis] * sgn, R.u[axis] * sgn, L.c, R.c, L.p, R.p, SL, SR,
+                                    Wa[NS + axis] * sgn, Wa[NS + 3]);
+        // c's own side
+#pragma unroll
+        for (int kk = 0; kk < NS + 4; ++kk) o.q[kk] += Wa[kk] * b.qL;
+        o.u[axis] += b.unL * sgn;
+        o.p += b.pL;
+        o.c += b.cL;
+        // a boundary ghost made from c (extrapolate: itself; slip: axis momentum and velocity mirrored)
+        if (kind == 1 || kind == 2) {
+            const double mirror = kind == 1 ? -1.0 : 1.0;
+#pragma unroll
+            for (int kk = 0; kk < NS + 4; ++kk) o.q[kk] += Wa[kk] * b.qR * (kk == NS + axis ? mirror : 1.0);
+            o.u[axis] += b.unR * sgn * mirror;
+            o.p += b.pR;
+            o.c += b.cR;
+        }
+        if (!viscous && !(v.conductivity > 0 && kind != 1)) continue;
+        // viscous traction and conduction at fixed gradients and eddy viscosities
+        double gMu = 0, gAv[3] = {0, 0, 0}, gAn = 0, gJmu = 0;
+        double duL[3] = {0, 0, 0}, duR[3] = {0, 0, 0}, dTL = 0, dTR = 0, dRL = 0, dRR = 0;
+        double nv[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) nv[d] = d == axis ? sgn : 0.0;
+        if (viscous) {
+            const double ikd = (kind == 1 ? .5 : 1.0) * invDist;
+            double g[9];
+#pragma unroll
+            for (int t = 0; t < 9; ++t) g[t] = gC[t];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                double normal = 0;
+#pragma unroll
+                for (int d = 0; d < 3; ++d) normal += g[a * 3 + d] * nv[d];
+                const double target = (R.u[a] - L.u[a]) * ikd;
+#pragma unroll
+                for (int d = 0; d < 3; ++d) g[a * 3 + d] += nv[d] * (target - normal);
+            }
+            const double div = g[0] + g[4] + g[8];
+            const double mu = v.viscosity + (v.wale ? wf * L.rho * nutC + (1 - wf) * R.rho * nutC : 0.0);
+            double tau[3], tn = 0, av[3], an = 0;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                double t = -2.0 / 3.0 * div * nv[a];
+#pragma unroll
+                for (int d = 0; d < 3; ++d) t += (g[a * 3 + d] + g[d * 3 + a]) * nv[d];
+                tau[a] = mu * t;
+                tn += tau[a] * nv[a];
+                av[a] = -(Wa[NS + a] + Wa[NS + 3] * (wf * L.u[a] + (1 - wf) * R.u[a]));
+                an += av[a] * nv[a];
+            }
+            if (kind == 1) {
+#pragma unroll
+                for (int a = 0; a < 3; ++a) { tau[a] = tn * nv[a]; av[a] = an * nv[a]; }
+            }
+            an = 0;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) an += av[a] * nv[a];
+            double jmu = 0;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                // dJ/dt_a = (dJ/dG' n)_a; dJ/du_bar_a = -W_E A tau_a
+                double rn = 0;
+#pragma unroll
+                for (int d = 0; d < 3; ++d)
+                    rn += mu * (av[a] * nv[d] + nv[a] * av[d] - (a == d ? 2.0 / 3.0 * an : 0.0)) * nv[d];
+                const double dbar = -Wa[NS + 3] * tau[a];
+                duL[a] = wf * dbar - rn * ikd;
+                duR[a] = (1 - wf) * dbar + rn * ikd;
+                double t = -2.0 / 3.0 * div * nv[a];
+#pragma unroll
+                for (int d = 0; d < 3; ++d) t += (g[a * 3 + d] + g[d * 3 + a]) * nv[d];
+                jmu += av[a] * t;
+            }
+            gMu = mu;
+            gAn = an;
+            gJmu = jmu;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) gAv[a] = av[a];
+            if (v.wale) {
+                dRL = jmu * wf * nutC;
+                dRR = jmu * (1 - wf) * nutC;
+            }
+        }
+        if (v.conductivity > 0 && kind != 1) {
+            dTL = Wa[NS + 3] * v.conductivity * invDist;
+            dTR = -dTL;
+        }
+        if (viscous) {
+            // dJ/dG' then the correction's transpose (av, an: the traction's weights)
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                double row[3], rn = 0;
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    row[d] = gMu * (gAv[a] * nv[d] + nv[a] * gAv[d] - (a == d ? 2.0 / 3.0 * gAn : 0.0));
+                    rn += row[d] * nv[d];
+                }
+#pragma unroll
+                for (int d = 0; d < 3; ++d) o.g[a * 3 + d] += row[d] - rn * nv[d];
+            }
+            if (v.wale) o.nut += gJmu * (wf * L.rho + (1 - wf) * R.rho);
+        }
+        // the owner, and the ghost made from it (extrapolate: itself; slip: mirrored velocity)
+#pragma unroll
+        for (int a = 0; a < 3; ++a) o.u[a] += duL[a];
+        o.T += dTL;
+        o.rho += dRL;
+        if (kind == 1 || kind == 2) {
+            double rn = 0;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) rn += duR[a] * nv[a];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) o.u[a] += kind == 1 ? duR[a] - 2 * rn * nv[a] : duR[a];
+            o.T += dTR;
+            o.rho += dRR;
+        }
+    }
+}
+
 // (dL/dq)^T w and (dL/dstate)^T w of the HLL operator of the structured box at
 // fixed cell gradients and eddy viscosities (the part cartRateVjp<NS, 0> forms
 // in dual numbers), gather form, in registers: the HLL flux by hllReverse; the
@@ -1452,200 +1737,85 @@ __device__ __forceinline__ HllBar hllReverse(double wf, double unL, double unR, 
 // target (u_R - u_L) / d and the work's u_bar) and through rho in the WALE
 // viscosity; conduction through T. With dJ/dG' = mu (a n^T + n a^T - 2/3 (a.n) I)
 // (a = -(W_m + W_E u_bar) A, projected on n at a slip wall): dJ/dt = dJ/dG' n,
-// dJ/du_bar = -W_E A tau, dJ/dmu = a . tau / mu. The gradients' and eddy
-// viscosities' own adjoints are cartViscousGradVjp's.
-template <int NS>
-__global__ void __launch_bounds__(128) cartRateVjpInviscid(CartView v, const double* __restrict__ q,
-                                                           const ReactiveTransportState* __restrict__ st,
-                                                           const double* __restrict__ grad,
-                                                           const double* __restrict__ nut,
-                                                           const double* __restrict__ w, double* __restrict__ qBar,
-                                                           ReactiveTransportState* __restrict__ stateBar) {
-    const bool viscous = v.viscosity > 0 || v.wale;
+// dJ/du_bar = -W_E A tau, dJ/dmu = a . tau / mu. With VISCOUS also the adjoints of
+// the cell's gradient and eddy viscosity (cartViscousGradVjp's, which the HLLC form
+// still takes from there), the latter carried to the gradient at once.
+//
+// One pass over a cell's faces for all of it, each side an instance of its own: with a
+// run-time axis the sides' velocities, weights and sums lived in local memory, and the
+// gradients' adjoints read every neighbour a second time (96^3 viscous box: 350 + 200 +
+// 77 us in three kernels).
+#ifndef RB200_VJP_MIN
+#define RB200_VJP_MIN 3
+#endif
+template <int NS, bool VISCOUS>
+__global__ void __launch_bounds__(128, RB200_VJP_MIN) cartRateVjpHll(CartView v, const double* __restrict__ q,
+                                                      const ReactiveTransportState* __restrict__ st,
+                                                      const double* __restrict__ grad,
+                                                      const double* __restrict__ nut,
+                                                      const double* __restrict__ w, double* __restrict__ qBar,
+                                                      ReactiveTransportState* __restrict__ stateBar,
+                                                      double* __restrict__ gBar) {
     for (size_t c = blockIdx.x * size_t(blockDim.x) + threadIdx.x; c < v.cells; c += size_t(blockDim.x) * gridDim.x) {
         int i, j, k;
         cellCoords(v, c, i, j, k);
         CellData C;
         loadCell<NS>(v, q, c, C, true);
         const double ivc = v.invV[c];
-        double dq[NS + 4], du[3] = {0, 0, 0}, dp = 0, dc = 0, dT = 0, dRhoState = 0;
+        double wc[NS + 4], gC[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll
-        for (int kk = 0; kk < NS + 4; ++kk) dq[kk] = 0;
-        double gC[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-        if (viscous) {
+        for (int kk = 0; kk < NS + 4; ++kk) wc[kk] = w[size_t(kk) * v.cells + c] * ivc;
+        if constexpr (VISCOUS) {
 #pragma unroll
             for (int t = 0; t < 9; ++t) gC[t] = grad[size_t(t) * v.cells + c];
         }
         const double nutC = v.wale ? nut[c] : 0.0;
-#pragma unroll 1
-        for (int n = 0; n < 12; ++n) {
-            const int s = sideOf(n);
-            const bool interior = hasNeighbour(v, s, i, j, k);
-            if (interior != (n < 6)) continue;
-            const int axis = s >> 1;
-            CellData O;  // the other side
-            double Wa[NS + 4], sgn, area, wf, invDist, gO[9], nutO = nutC;
-            int kind = 0;
-            bool cIsLeft = true;
-            if (interior) {
-                const size_t nb = neighbourOf(v, s, c);
-                loadCell<NS>(v, q, nb, O, true);
-                const double ivn = v.invV[nb];
-                cIsLeft = s & 1;
-                sgn = 1;
-                area = v.area[axis];
-                wf = .5;
-                invDist = v.invDist[axis];
-                if (viscous) {
+        CellBar<NS> o{};
+        bool edge = false;
+        auto face = [&](auto side) {
+            constexpr int S = decltype(side)::value;
+            if (hasNeighbour(v, S, i, j, k))
+                interiorFaceBar<NS, S, VISCOUS>(v, q, grad, nut, w, neighbourOf(v, S, c), C, gC, nutC, wc, o);
+            else edge = true;
+        };
+        face(std::integral_constant<int, 4>{});
+        face(std::integral_constant<int, 2>{});
+        face(std::integral_constant<int, 0>{});
+        face(std::integral_constant<int, 1>{});
+        face(std::integral_constant<int, 3>{});
+        face(std::integral_constant<int, 5>{});
+        if (edge) {
+            CellBar<NS> sums = o;
+            const CellData cell = C;
+            double g[9], weights[NS + 4];
 #pragma unroll
-                    for (int t = 0; t < 9; ++t) gO[t] = grad[size_t(t) * v.cells + nb];
-                }
-                if (v.wale) nutO = nut[nb];
+            for (int t = 0; t < 9; ++t) g[t] = gC[t];
 #pragma unroll
-                for (int kk = 0; kk < NS + 4; ++kk)
-                    Wa[kk] = area * (cIsLeft ? w[size_t(kk) * v.cells + nb] * ivn - w[size_t(kk) * v.cells + c] * ivc
-                                             : w[size_t(kk) * v.cells + c] * ivc - w[size_t(kk) * v.cells + nb] * ivn);
-            } else {
-                const ReactiveTransportFace& f = sideFace(v, s, i, j, k);
-                kind = f.kind;
-                boundaryRight<NS>(v, q, st, f, axis, C, O, true);
-                sgn = (s & 1) ? 1.0 : -1.0;
-                area = f.area;
-                wf = f.ownerWeight;
-                invDist = 1 / f.distance;
-#pragma unroll
-                for (int t = 0; t < 9; ++t) gO[t] = gC[t];
-#pragma unroll
-                for (int kk = 0; kk < NS + 4; ++kk) Wa[kk] = -area * w[size_t(kk) * v.cells + c] * ivc;
-            }
-            const CellData& L = cIsLeft ? C : O;
-            const CellData& R = cIsLeft ? O : C;
-            double SL = 0, SR = 0;
-#pragma unroll
-            for (int kk = 0; kk < NS + 4; ++kk) { SL += Wa[kk] * L.q[kk]; SR += Wa[kk] * R.q[kk]; }
-            const HllBar b = hllReverse(v.waveFactor, L.u[axis] * sgn, R.u[axis] * sgn, L.c, R.c, L.p, R.p, SL, SR,
-                                        Wa[NS + axis] * sgn, Wa[NS + 3]);
-            // c's own side
-            const double qMul = cIsLeft ? b.qL : b.qR;
-#pragma unroll
-            for (int kk = 0; kk < NS + 4; ++kk) dq[kk] += Wa[kk] * qMul;
-            du[axis] += (cIsLeft ? b.unL : b.unR) * sgn;
-            dp += cIsLeft ? b.pL : b.pR;
-            dc += cIsLeft ? b.cL : b.cR;
-            // a boundary ghost made from c (extrapolate: itself; slip: axis momentum and velocity mirrored)
-            if (!interior && (kind == 1 || kind == 2)) {
-                const double mirror = kind == 1 ? -1.0 : 1.0;
-#pragma unroll
-                for (int kk = 0; kk < NS + 4; ++kk) dq[kk] += Wa[kk] * b.qR * (kk == NS + axis ? mirror : 1.0);
-                du[axis] += b.unR * sgn * mirror;
-                dp += b.pR;
-                dc += b.cR;
-            }
-            if (!viscous && !(v.conductivity > 0 && kind != 1)) continue;
-            // viscous traction and conduction at fixed gradients and eddy viscosities
-            double duL[3] = {0, 0, 0}, duR[3] = {0, 0, 0}, dTL = 0, dTR = 0, dRL = 0, dRR = 0;
-            double nv[3];
-#pragma unroll
-            for (int d = 0; d < 3; ++d) nv[d] = d == axis ? sgn : 0.0;
-            if (viscous) {
-                const double* gL = cIsLeft ? gC : gO;
-                const double* gR = cIsLeft ? gO : gC;
-                const double nutL = cIsLeft ? nutC : nutO, nutR = cIsLeft ? nutO : nutC;
-                const double ikd = (kind == 1 ? .5 : 1.0) * invDist;
-                double g[9];
-#pragma unroll
-                for (int t = 0; t < 9; ++t) g[t] = interior ? wf * gL[t] + (1 - wf) * gR[t] : gL[t];
-#pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    double normal = 0;
-#pragma unroll
-                    for (int d = 0; d < 3; ++d) normal += g[a * 3 + d] * nv[d];
-                    const double target = (R.u[a] - L.u[a]) * ikd;
-#pragma unroll
-                    for (int d = 0; d < 3; ++d) g[a * 3 + d] += nv[d] * (target - normal);
-                }
-                const double div = g[0] + g[4] + g[8];
-                const double mu = v.viscosity + (v.wale ? wf * L.rho * nutL + (1 - wf) * R.rho * nutR : 0.0);
-                double tau[3], tn = 0, av[3], an = 0;
-#pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    double t = -2.0 / 3.0 * div * nv[a];
-#pragma unroll
-                    for (int d = 0; d < 3; ++d) t += (g[a * 3 + d] + g[d * 3 + a]) * nv[d];
-                    tau[a] = mu * t;
-                    tn += tau[a] * nv[a];
-                    av[a] = -(Wa[NS + a] + Wa[NS + 3] * (wf * L.u[a] + (1 - wf) * R.u[a]));
-                    an += av[a] * nv[a];
-                }
-                if (kind == 1) {
-#pragma unroll
-                    for (int a = 0; a < 3; ++a) { tau[a] = tn * nv[a]; av[a] = an * nv[a]; }
-                }
-                an = 0;
-#pragma unroll
-                for (int a = 0; a < 3; ++a) an += av[a] * nv[a];
-                double jmu = 0;
-#pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    // dJ/dt_a = (dJ/dG' n)_a; dJ/du_bar_a = -W_E A tau_a
-                    double rn = 0;
-#pragma unroll
-                    for (int d = 0; d < 3; ++d)
-                        rn += mu * (av[a] * nv[d] + nv[a] * av[d] - (a == d ? 2.0 / 3.0 * an : 0.0)) * nv[d];
-                    const double dbar = -Wa[NS + 3] * tau[a];
-                    duL[a] = wf * dbar - rn * ikd;
-                    duR[a] = (1 - wf) * dbar + rn * ikd;
-                    double t = -2.0 / 3.0 * div * nv[a];
-#pragma unroll
-                    for (int d = 0; d < 3; ++d) t += (g[a * 3 + d] + g[d * 3 + a]) * nv[d];
-                    jmu += av[a] * t;
-                }
-                if (v.wale) {
-                    dRL = jmu * wf * nutL;
-                    dRR = jmu * (1 - wf) * nutR;
-                }
-            }
-            if (v.conductivity > 0 && kind != 1) {
-                dTL = Wa[NS + 3] * v.conductivity * invDist;
-                dTR = -dTL;
-            }
-            if (interior) {
-#pragma unroll
-                for (int a = 0; a < 3; ++a) du[a] += cIsLeft ? duL[a] : duR[a];
-                dT += cIsLeft ? dTL : dTR;
-                dRhoState += cIsLeft ? dRL : dRR;
-            } else {
-                // the owner, and the ghost made from it (extrapolate: itself; slip: mirrored velocity)
-#pragma unroll
-                for (int a = 0; a < 3; ++a) du[a] += duL[a];
-                dT += dTL;
-                dRhoState += dRL;
-                if (kind == 1 || kind == 2) {
-                    double rn = 0;
-#pragma unroll
-                    for (int a = 0; a < 3; ++a) rn += duR[a] * nv[a];
-#pragma unroll
-                    for (int a = 0; a < 3; ++a) du[a] += kind == 1 ? duR[a] - 2 * rn * nv[a] : duR[a];
-                    dT += dTR;
-                    dRhoState += dRR;
-                }
-            }
+            for (int kk = 0; kk < NS + 4; ++kk) weights[kk] = wc[kk];
+            boundaryFaceBars<NS>(v, q, st, i, j, k, cell, g, nutC, weights, VISCOUS, sums);
+            o = sums;
         }
         // u = m / rho with rho the sum of the species masses
-        double rho = 0;
+        double rho = 0, dRho = 0;
 #pragma unroll
         for (int kk = 0; kk < NS; ++kk) rho += C.q[kk];
-        double dRho = 0;
+        const double irho = 1 / rho;
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-            dq[NS + a] += du[a] / rho;
-            dRho -= du[a] * C.u[a] / rho;
+            const double m = o.u[a] * irho;
+            o.q[NS + a] += m;
+            dRho -= m * C.u[a];
         }
 #pragma unroll
-        for (int kk = 0; kk < NS; ++kk) dq[kk] += dRho;
+        for (int kk = 0; kk < NS; ++kk) o.q[kk] += dRho;
 #pragma unroll
-        for (int kk = 0; kk < NS + 4; ++kk) qBar[size_t(kk) * v.cells + c] = dq[kk];
-        stateBar[c] = ReactiveTransportState{dp, dT, dRhoState, 0.0, dc, 0.0, 0.0};
+        for (int kk = 0; kk < NS + 4; ++kk) qBar[size_t(kk) * v.cells + c] = o.q[kk];
+        stateBar[c] = ReactiveTransportState{o.p, o.T, o.rho, 0.0, o.c, 0.0, 0.0};
+        if constexpr (VISCOUS) {
+            if (v.wale) waleReverse(v, ivc, gC, o.nut, o.g);
+#pragma unroll
+            for (int t = 0; t < 9; ++t) gBar[size_t(t) * v.cells + c] = o.g[t];
+        }
     }
 }
 
@@ -1787,67 +1957,21 @@ __global__ void __launch_bounds__(128) cartViscousGradVjp(CartView v, const doub
     }
 }
 
-// gBar += nutBar * d nu_t / d g per cell (the WALE eddy viscosity of the cell's
-// gradient, the Nicoud-Ducros relation of wale.cuh:
-// nu_t = (Cw Delta)^2 |g|_max (Sd:Sd)^(3/2) / ((S:S)^(5/2) + (Sd:Sd)^(5/4))
-// with the invariants of g / |g|_max; zero where the forward gives zero), by a
-// reverse pass derived by hand.
+// gBar += nutBar * d nu_t / d g per cell.
 __global__ void cartWaleVjp(CartView v, const double* __restrict__ grad, const double* __restrict__ nutBar,
                             double* __restrict__ gBar) {
-    // nu_t = (Cw Delta)^2 |g|_max ratio(g / |g|_max) and ratio is homogeneous of
-    // degree one, so d nu_t / d g = (Cw Delta)^2 d ratio / d h at h = g / |g|_max
-    // (the normalisation's own derivative cancels). With ratio = dd^(3/2) /
-    // (ss^(5/2) + dd^(5/4)), ss = S:S (S = sym h), dd = D:D (D = dev sym(h h)):
-    // d ss / d h = 2 S and d dd / d h = G h^T + h^T G with G = 2 D.
     for (size_t c = blockIdx.x * size_t(blockDim.x) + threadIdx.x; c < v.cells; c += size_t(blockDim.x) * gridDim.x) {
         const double nb = nutBar[c];
         if (nb == 0) continue;
-        double g[9], scale = 0;
+        double g[9], gb[9];
 #pragma unroll
         for (int t = 0; t < 9; ++t) {
             g[t] = grad[size_t(t) * v.cells + c];
-            scale = fmax(scale, ::fabs(g[t]));
+            gb[t] = gBar[size_t(t) * v.cells + c];
         }
-        const double delta = cbrt(1 / v.invV[c]);
-        if (scale == 0 || v.cw == 0 || delta == 0) continue;
-        double h[9];
+        waleReverse(v, v.invV[c], g, nb, gb);
 #pragma unroll
-        for (int t = 0; t < 9; ++t) h[t] = g[t] / scale;
-        double sq[9];
-#pragma unroll
-        for (int a = 0; a < 3; ++a)
-#pragma unroll
-            for (int b = 0; b < 3; ++b) sq[3 * a + b] = h[3 * a] * h[b] + h[3 * a + 1] * h[3 + b] + h[3 * a + 2] * h[6 + b];
-        const double trace = sq[0] + sq[4] + sq[8];
-        double S[9], G[9], ss = 0, dd = 0;
-#pragma unroll
-        for (int a = 0; a < 3; ++a)
-#pragma unroll
-            for (int b = 0; b < 3; ++b) {
-                const double sab = .5 * (h[3 * a + b] + h[3 * b + a]);
-                double dab = .5 * (sq[3 * a + b] + sq[3 * b + a]);
-                if (a == b) dab -= trace / 3.0;
-                S[3 * a + b] = sab;
-                G[3 * a + b] = 2 * dab;
-                ss += sab * sab;
-                dd += dab * dab;
-            }
-        if (!(dd > 0)) continue;
-        const double rootD = sqrt(dd), quarter = sqrt(rootD), rootS = sqrt(ss);
-        const double numerator = dd * rootD, denominator = ss * ss * rootS + dd * quarter;
-        const double den2 = denominator * denominator;
-        const double rDd = (1.5 * rootD * denominator - numerator * 1.25 * quarter) / den2;
-        const double rSs = -numerator * 2.5 * ss * rootS / den2;
-        const double weight = nb * (v.cw * delta * v.cw * delta);
-#pragma unroll
-        for (int u = 0; u < 3; ++u)
-#pragma unroll
-            for (int w = 0; w < 3; ++w) {
-                double dDd = 0;
-#pragma unroll
-                for (int k = 0; k < 3; ++k) dDd += G[3 * u + k] * h[3 * w + k] + G[3 * k + w] * h[3 * k + u];
-                gBar[size_t(3 * u + w) * v.cells + c] += weight * (rDd * dDd + rSs * 2 * S[3 * u + w]);
-            }
+        for (int t = 0; t < 9; ++t) gBar[size_t(t) * v.cells + c] = gb[t];
     }
 }
 

@@ -836,16 +836,20 @@ struct Transport {
         static void run(const CartView& b, const double* q, const ReactiveTransportState* st, const double* grad,
                         const double* nut, const double* w, double* qBar, ReactiveTransportState* stateBar,
                         double* gBar, double* nutBar, bool viscous, cudaStream_t s) {
-            // the state-side derivatives: HLL by hand (with the viscous and conduction
-            // terms at fixed gradients), HLLC in dual numbers
-            if (b.scheme == 0)
-                cartRateVjpInviscid<NS><<<gridFor(b.cells, 128), 128, 0, s>>>(b, q, st, grad, nut, w, qBar, stateBar);
-            else
-                cartRateVjp<NS, 0><<<gridFor(b.cells, 128), 128, 0, s>>>(b, q, st, grad, nut, w, qBar, stateBar,
-                                                                        nullptr, nullptr);
+            // HLL by hand, the state side and the gradients' in one pass; HLLC's state side
+            // in dual numbers
+            const unsigned grid = gridFor(b.cells, 128);
+            if (b.scheme == 0) {
+                if (viscous)
+                    cartRateVjpHll<NS, true><<<grid, 128, 0, s>>>(b, q, st, grad, nut, w, qBar, stateBar, gBar);
+                else cartRateVjpHll<NS, false><<<grid, 128, 0, s>>>(b, q, st, grad, nut, w, qBar, stateBar, nullptr);
+            } else
+                cartRateVjp<NS, 0><<<grid, 128, 0, s>>>(b, q, st, grad, nut, w, qBar, stateBar, nullptr, nullptr);
             if (!viscous) return;
-            cartViscousGradVjp<NS><<<gridFor(b.cells, 128), 128, 0, s>>>(b, q, st, grad, nut, w, gBar, nutBar);
-            if (b.wale) cartWaleVjp<<<gridFor(b.cells, 128), 128, 0, s>>>(b, grad, nutBar, gBar);
+            if (b.scheme != 0) {
+                cartViscousGradVjp<NS><<<grid, 128, 0, s>>>(b, q, st, grad, nut, w, gBar, nutBar);
+                if (b.wale) cartWaleVjp<<<grid, 128, 0, s>>>(b, grad, nutBar, gBar);
+            }
             cartGradientVjp<NS><<<gridFor(b.cells, 256), 256, 0, s>>>(b, q, gBar, qBar);
         }
     };
