@@ -46,18 +46,16 @@ sys.path.insert(0, str(ROOT))
 
 METRIC = "Mcell-steps/s at 160³, plain FP64 vs mixed/batched; adjoint/forward time"
 UNIT = "Mcell-steps/s"
-# Per-unit figures of the dominant kernel (the flash: its one-thread-per-cell
-# single-phase pass, with the work queue for the cells the two-phase bound keeps),
-# each per PR phase evaluation (the device counter the flash reports; a gas
-# probe's root check decided without the root solve is not one), from ncu
-# captures of one recovery of the impingement flow at 80^3, steps 21-22: FP64
-# FLOPs = 2 DFMA + DADD + DMUL thread instructions, and DRAM read+write bytes
-# (more cells than resident threads, as at 160^3, so the pass's stack frames do
-# not stay in L2). Both include the single-phase pass's own formation of the
-# flash inputs from the conserved rows and the seeds.
-FLOPS_PER_PHASE_EVAL = 652.3
+# Per-unit figures of the dominant kernels (the flash: the gas pass, one thread a
+# cell in registers, and the search of the cells it leaves), each per PR phase
+# evaluation (the device counter the flash reports; a gas probe's root check decided
+# without the root solve is not one), from ncu captures of one recovery of the
+# impingement flow at 80^3, steps 21-22: FP64 FLOPs = 2 DFMA + DADD + DMUL thread
+# instructions, and DRAM read+write bytes. Both include the gas pass's own
+# formation of the flash inputs from the conserved rows and the seeds.
+FLOPS_PER_PHASE_EVAL = 393.8
 FLASH_BYTES_PER_CELL = 40 + 24 + 184 + 56
-DRAM_BYTES_PER_PHASE_EVAL = 196.7
+DRAM_BYTES_PER_PHASE_EVAL = 146.7
 VISCOSITY, CONDUCTIVITY, WALE_CW, DT = 1.821e-5, 0.02587, 0.325, 1e-8
 REFERENCE_SAMPLE = 40  # cube size of the reference CPU arm's bounded sample
 
@@ -381,9 +379,8 @@ def run_slab(args, rank, world):
     stats1 = pkg._abi.Stats()
     f.lib.reactive_transport_stats(f.transport, C.byref(stats1))
     # transport launches counted by the handle while capturing both half steps,
-    # plus five per flash (single-phase pass, queue, selection, restart queue,
-    # restart selection)
-    launches_per_step = int(stats1.kernelLaunches - stats0.kernelLaunches) + 2 * 5
+    # plus four per flash (gas pass, candidate search, selection, restarts)
+    launches_per_step = int(stats1.kernelLaunches - stats0.kernelLaunches) + 2 * 4
 
     def barrier():
         if world > 1:
@@ -475,8 +472,8 @@ def run_ours(args, rank, world):
         return max_over_ranks_(a.elapsed_time(b) / steps), clocks_
 
     # kernels launched per step: the kernel nodes of the step's launches captured
-    # once more (else the transport's call count plus five per flash:
-    # single-phase pass, queue, selection, restart queue, restart selection)
+    # once more (else the transport's call count plus four per flash: gas pass,
+    # candidate search, selection, restarts)
     stats0 = pkg._abi.Stats()
     lib.reactive_transport_stats(flow.transport, C.byref(stats0))
     flow.capture(DT)
@@ -608,7 +605,7 @@ def run_ours(args, rank, world):
                     "frac": achieved / fp64 if achieved else None,
                     "traffic": args.dram_bytes_per_phase_eval * flash_phase_evals,
                     "peak_source": "measured in this run (FP64 FMA-chain probe)",
-                    "kernel": "HEM flash, one recovery of all cells (passSinglePhase + passQueue + selection + "
+                    "kernel": "HEM flash, one recovery of all cells (passGas + passSearch + selection + "
                               "restarts): the first recovery of each timed step, re-run from the timed steps' "
                               "start state",
                     "traffic_note": "DRAM bytes per launch, ncu per-phase-evaluation figure x this launch's "

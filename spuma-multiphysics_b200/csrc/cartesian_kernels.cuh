@@ -101,7 +101,8 @@ template <int NS, class R, bool SGS = false> __device__ __forceinline__ CellT<R>
 // The stage kernels read a cell's inputs up to seven times: as SoA their loads
 // coalesce (the 56-byte states and 32-byte primitives cost a warp 70 and 16
 // wavefronts a cell where these cost two a field), and the two reciprocals
-// replace five divisions a face of the CFL speed.
+// replace five divisions a face of the CFL speed. HBM bound: 96 us at 160^3 (168 B a
+// cell).
 __global__ void __launch_bounds__(256) cartInputs(CartView v, const double* __restrict__ q,
                                                   const ReactiveTransportState* __restrict__ st, int ns,
                                                   bool fromPrimitive) {
@@ -421,7 +422,7 @@ __device__ __forceinline__ size_t neighbourOf(const CartView& v, int s, size_t c
 // type R (stored as R: 9 gradient components and nu_t per cell). Bound by FP64
 // issue: a face adds to its own axis' three components only (the general form's
 // other products are with zero normal components and change no bit of finite
-// data), and the mean of the two cells' velocities is .5 (a + b).
+// data), and the mean of the two cells' velocities is .5 (a + b). 178 us at 160^3.
 template <int NS, class R>
 __global__ void __launch_bounds__(256) cartGradients(CartView v, const ReactiveTransportState* __restrict__ st,
                                                      R* __restrict__ grad, R* __restrict__ nut, unsigned* error) {
@@ -623,7 +624,9 @@ __device__ __forceinline__ double cellStep(const CartView& v, size_t c, double d
 // evaluated once): the minimum over both kernels' block minima
 // (minimumReduce) is bitwise cartSteps'.
 // Four blocks of 128 per SM (at most 128 registers) measured 7% faster at
-// 160^3 than the compiler's own 151 registers at three.
+// 160^3 than the compiler's own 151 registers at three. Each axis is an instance
+// of its own (faceFluxCart's AXIS): with a run-time axis the velocities and gradients
+// lived in local memory, and the 160^3 step took 7.87 ms against 6.90.
 #ifndef RB200_FACE_MINBLOCKS
 #define RB200_FACE_MINBLOCKS 4
 #endif
@@ -1744,12 +1747,11 @@ __device__ __noinline__ void boundaryFaceBars(const CartView& v, const double* _
 // One pass over a cell's faces for all of it, each side an instance of its own: with a
 // run-time axis the sides' velocities, weights and sums lived in local memory, and the
 // gradients' adjoints read every neighbour a second time (96^3 viscous box: 350 + 200 +
-// 77 us in three kernels).
-#ifndef RB200_VJP_MIN
-#define RB200_VJP_MIN 3
-#endif
+// 77 us in three kernels, 353 us here; 64^3 two-species inviscid 98 -> 75 us). Bound
+// by FP64 latency; three blocks a multiprocessor (168 registers) measured 1% faster than
+// four.
 template <int NS, bool VISCOUS>
-__global__ void __launch_bounds__(128, RB200_VJP_MIN) cartRateVjpHll(CartView v, const double* __restrict__ q,
+__global__ void __launch_bounds__(128, 3) cartRateVjpHll(CartView v, const double* __restrict__ q,
                                                       const ReactiveTransportState* __restrict__ st,
                                                       const double* __restrict__ grad,
                                                       const double* __restrict__ nut,

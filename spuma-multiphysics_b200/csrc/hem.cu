@@ -596,18 +596,17 @@ __device__ __forceinline__ bool gasCell(const GasPass& G, const HemConst& C, dou
 // come from the constant bank), and the 176-byte records leave through a
 // per-warp shared-memory stage as full lines (a thread's own 22 stores would
 // touch 22 x 32 sectors a warp). The outputs are not read again by the flash:
-// streaming stores.
+// streaming stores. 160^3 cells: 848 us a call (the general pass took 2.5 ms for the
+// same cells); six blocks a multiprocessor (80 registers) measured 2% of the step
+// faster than five, seven (72, spills) no faster.
 //
 // FROM_CONSERVED: the inputs come from the SoA conserved rows and the seeds (as
 // inputsFromConserved forms them), else from `in`. `seed` may be `state` (an
 // in-place recovery): a warp reads its own cells' seeds before it writes their
 // states and touches no other cell's.
 constexpr int kGasThreads = 128, kStageRow = 23;  // 22 words a record and one of padding against bank conflicts
-#ifndef RB200_GAS_MINBLOCKS
-#define RB200_GAS_MINBLOCKS 6
-#endif
 template <bool FROM_CONSERVED>
-__global__ void __launch_bounds__(kGasThreads, RB200_GAS_MINBLOCKS) passGas(
+__global__ void __launch_bounds__(kGasThreads, 6) passGas(
     const __grid_constant__ GasPass G, const HemConst* __restrict__ Cp, CellInput* __restrict__ in,
     const double* __restrict__ cons, size_t stride, const ReactiveThermoState* seed, size_t count,
     ReactiveThermoState* state, ReactiveTransportState* transport, int* success, unsigned* list, unsigned* general,
@@ -837,7 +836,8 @@ __global__ void selectCandidates(const HemConst* __restrict__ Cp, const CandReco
 // seeds) side by side, and the first maximum of the entropy density in the serial
 // order (temperatures, then seeds: the lane order) is written; a cell without one
 // keeps its seed and fails. The solves of one cell are long serial Newton chains;
-// one thread running a temperature's five in turn had them five times as long.
+// one thread running a temperature's five in turn had them five times as long (65,537
+// cells from fixed seeds: 62.0 -> 30.9 ms a batch).
 __global__ void __launch_bounds__(kPassThreads, RB200_PASS_MINBLOCKS) passRestarts(const HemConst* __restrict__ Cp,
                                                              const CellInput* __restrict__ in,
                                                              const unsigned* __restrict__ fallback,

@@ -14,7 +14,9 @@
 // cv > 0 and dp/dV < 0) and are formed once, for the converged state. The middle
 // root of the cubic is not polished. That leaves 15 divisions and 3 logarithms of
 // 37 and 5, and the iteration's state in registers instead of the work queue's
-// lane record on the stack.
+// lane record on the stack: 1,000,000 cells, 60% saturated, take 3.3 ms for their
+// two-phase candidates (the 40^3 step went from 1.49 to 1.11 ms, 1.09 with both roots'
+// chains interleaved).
 #pragma once
 #include "hem_flash.cuh"
 

