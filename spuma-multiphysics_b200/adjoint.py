@@ -77,7 +77,9 @@ class IdealGasBox:
         self.T_guess = torch.full((self.cells,), float(T_guess), **f64)
         self.volume = torch.from_numpy(self._volume).to(self.device)
         self.success = torch.zeros(self.cells, dtype=torch.int32, device=self.device)
-        self.failures = torch.zeros((), dtype=torch.int64, device=self.device)  # closure failures since check()
+        # closure failures of each cell since check() (summed there: a reduction a closure
+        # costs as much as the closure's kernel on a small box)
+        self.failures = torch.zeros(self.cells, dtype=torch.int32, device=self.device)
         self.err = C.create_string_buffer(1024)
 
     # ------------------------------------------------------------- plumbing
@@ -108,7 +110,7 @@ class IdealGasBox:
         self._gas_check(self.lib.reactive_ideal_gas_run_device_v3(
             self.gas, q.data_ptr(), q.shape[1], self.cells, self.nv, self.T_guess.data_ptr(), T.data_ptr(),
             tr.data_ptr(), self.success.data_ptr(), s, self.err, len(self.err)))
-        self.failures += (self.success == 0).sum()
+        self.failures.sub_(self.success).add_(1)
         return T, tr
 
     def stage(self, q_in, q_out, tr, dt, stage):
@@ -148,16 +150,16 @@ class IdealGasBox:
         q_n, q_1, T_n, T_1, tr_n, tr_1 = saved
         lam = lam.contiguous()
         q_bar1, tr_bar1 = self.rate_vjp(q_1, tr_1, (.5 * dt) * lam)
-        q_bar1 += .5 * lam
+        q_bar1.add_(lam, alpha=.5)
         self.closure_vjp(q_1, T_1, tr_bar1, q_bar1)
         q_barn, tr_barn = self.rate_vjp(q_n, tr_n, dt * q_bar1)
-        q_barn += .5 * lam + q_bar1
+        q_barn.add_(lam, alpha=.5).add_(q_bar1)
         self.closure_vjp(q_n, T_n, tr_barn, q_barn)
         return q_barn
 
     def check(self):
         """Every closure since the last check converged (synchronises)."""
-        failed = int(self.failures.item())
+        failed = int(self.failures.sum().item())
         self.failures.zero_()
         if failed:
             raise AdjointError(f"ideal-gas closure failed in {failed} cells")
@@ -215,19 +217,6 @@ def rollout(box, q0, steps, dt, checkpoint_every=10):
 # The HEM step (pure-fluid PR flash, structured viscous/WALE transport)
 
 
-def _compact(states_u8, cells):
-    """Transport states (cells, 7) of thermo states (uint8 view of cells x 176 B):
-    p, T, rho, cv, frozen sound, gas mass, 0 (the reference's compact,
-    ReactiveFoam.C:419-420)."""
-    s = states_u8.view(torch.float64).view(cells, 22)
-    tr = torch.zeros((cells, 7), dtype=torch.float64, device=states_u8.device)
-    tr[:, 0:3] = s[:, 0:3]
-    tr[:, 3] = s[:, 20]
-    tr[:, 4] = s[:, 5]
-    tr[:, 5] = s[:, 18]
-    return tr
-
-
 class HemStep:
     """Functional SSPRK2 + HEM steps over a `flow.Flow`'s transport and HEM
     handles (FP64, structured path), and their adjoint:
@@ -243,7 +232,9 @@ class HemStep:
         self.lib = flow.lib
         self.cells, self.fixed, self.nv = flow.cells, flow.fixed, flow.nv
         self.fixed_tr = flow.tr[self.cells:].clone()
+        # since check(): the flash derivatives that failed, and each cell's flash failures
         self.failed = torch.zeros(1, dtype=torch.int32, device=flow.device)
+        self.failures = torch.zeros(self.cells, dtype=torch.int32, device=flow.device)
         self.err = C.create_string_buffer(1024)
         if flow.precision != "fp64":
             raise AdjointError("the adjoint differentiates the FP64 operator: use a precision='fp64' flow")
@@ -252,8 +243,20 @@ class HemStep:
         if rc:
             raise AdjointError(self.lib.reactive_transport_error(self.flow.transport).decode())
 
-    def _tr_all(self, tr_cells):
-        return torch.cat([tr_cells, self.fixed_tr], 0).contiguous()
+    def _compact(self, states_u8):
+        """Transport states (cells + fixed, 7) of thermo states (uint8 view of cells x 176 B):
+        p, T, rho, cv, frozen sound, gas mass, 0 (the reference's compact,
+        ReactiveFoam.C:419-420), and the fixed states."""
+        s = states_u8.view(torch.float64).view(self.cells, 22)
+        tr = torch.empty((self.cells + self.fixed, 7), dtype=torch.float64, device=states_u8.device)
+        own = tr[:self.cells]
+        own[:, 0:3] = s[:, 0:3]
+        own[:, 3] = s[:, 20]
+        own[:, 4] = s[:, 5]
+        own[:, 5] = s[:, 18]
+        own[:, 6] = 0
+        tr[self.cells:] = self.fixed_tr
+        return tr
 
     def _flash(self, q, seed):
         f = self.flow
@@ -262,7 +265,7 @@ class HemStep:
         tr = torch.empty((self.cells + self.fixed, 7), dtype=torch.float64, device=f.device)
         tr[self.cells:] = self.fixed_tr
         f.hem.run_device(q, q.shape[1], self.cells, self.nv, seed, out, tr, f.success, s)
-        self.failed += (f.success == 0).sum().to(torch.int32)
+        self.failures.sub_(f.success).add_(1)
         return out, tr
 
     def _stage(self, q_in, q_out, tr, dt, stage):
@@ -279,7 +282,7 @@ class HemStep:
 
     def forward_step(self, q_n, s_n, dt):
         q_n = q_n.contiguous()
-        tr_n = self._tr_all(_compact(s_n, self.cells))
+        tr_n = self._compact(s_n)
         q_1 = q_n.clone()
         self._stage(q_n, q_1, tr_n, dt, 0)
         s_1, tr_1 = self._flash(q_1, s_n)
@@ -311,18 +314,19 @@ class HemStep:
         q_n, s_n, tr_n, q_1, s_1, tr_1 = saved
         lam = lam.contiguous()
         q_bar1, tr_bar1 = self.rate_vjp(q_1, tr_1, (.5 * dt) * lam)
-        q_bar1 += .5 * lam
+        q_bar1.add_(lam, alpha=.5)
         self.hem_vjp(q_1, s_1, tr_bar1, q_bar1)
         q_barn, tr_barn = self.rate_vjp(q_n, tr_n, dt * q_bar1)
-        q_barn += .5 * lam + q_bar1
+        q_barn.add_(lam, alpha=.5).add_(q_bar1)
         self.hem_vjp(q_n, s_n, tr_barn, q_barn)
         return q_barn
 
     def check(self):
         """Every flash and every flash derivative since the last check succeeded,
         and the transport status word is clear (synchronises)."""
-        n = int(self.failed.item())
+        n = int(self.failed.item()) + int(self.failures.sum().item())
         self.failed.zero_()
+        self.failures.zero_()
         status = C.c_uint()
         self._check(self.lib.reactive_transport_status_v3(self.flow.transport, C.byref(status), 1,
                                                           torch.cuda.current_stream().cuda_stream))
