@@ -787,10 +787,17 @@ struct MixBest {
 // only one does; the boundary recovery's coordinates step at least one ulp and
 // weight the two sides by their actual steps), or `width` consecutive fractions of
 // the line search, of which the first acceptable one is taken. The points, their
-// order and the accepted ones are those of a serial search, so the results are
-// its bits; a Newton step takes two rounds instead of seven or more evaluations
-// in a row. An accepted evaluation is the stability test's own point, so the test
-// reads its chemical potentials.
+// order and the rule that accepts them are a serial search's; a Newton step takes
+// two rounds instead of seven or more evaluations in a row. A point's residual is
+// formed alone (mixture_residual.cuh) or, where that decides nothing, taken from the
+// general evaluation, which differ by rounding.
+//
+// A point whose residual is within the tolerances is evaluated in full by its owner:
+// the candidate's state, its reported residuals and the stability test (the chemical
+// potentials of that same point) all come from this one evaluation, and the candidate
+// has converged when its residual is within the tolerances too, else the Newton goes on
+// from it. It stays in the owner's `v` while the last Jacobian is formed, so
+// side points have a `side` of their own.
 __device__ __noinline__ void runTasks(MixCell& c, const MixTerms& terms, bool restarts, MixRecord* bestRecord,
                                       MixBest& best) {
     const ReactiveB200HemModel& m = c.m;
@@ -814,7 +821,7 @@ __device__ __noinline__ void runTasks(MixCell& c, const MixTerms& terms, bool re
     bool more = inGroup, converged = false, settled = false;
     MixTask t{{0, 0}, 0, 0, 0, 0};
     double x[4] = {}, f[4] = {}, step[4] = {}, column[4] = {}, scale = 1, previous = 0;
-    MixEval v;
+    MixEval v, side;
     for (;;) {
         // idle groups take the next tasks in order
         {
@@ -874,7 +881,7 @@ __device__ __noinline__ void runTasks(MixCell& c, const MixTerms& terms, bool re
             if (!general) ++c.n.residuals;
         }
         if (__any_sync(0xffffffffu, general)) {
-            if (general) ok = activeResidual(c, t.active, t.n, xe, scale, fe, v);
+            if (general) ok = activeResidual(c, t.active, t.n, xe, scale, fe, st == SIDES ? side : v);
         }
         __syncwarp();
         bool finished = false, stable = false, evaluated = false;  // evaluated: (x, f) is a new iterate
@@ -988,17 +995,21 @@ __device__ __noinline__ void runTasks(MixCell& c, const MixTerms& terms, bool re
                 it = st == START ? 0 : it + 1;
                 evaluated = true;
                 finished = it >= 90;
-                converged = fabs(f[0]) <= m.vtol && fabs(f[1]) <= m.etol && maxAbs(f + 2, t.n) <= m.mutol;
+                auto within = [&] {
+                    return fabs(f[0]) <= m.vtol && fabs(f[1]) <= m.etol && maxAbs(f + 2, t.n) <= m.mutol;
+                };
+                converged = within();
                 if (converged && !finished) {
-                    // the candidate's state: its residual's evaluation in full
                     bool whole = true;
                     if (int(lane) == owner) {
                         const Tally keep = c.n;
-                        double same[4] = {};
-                        whole = activeResidual(c, t.active, t.n, x, scale, same, v);
+                        whole = activeResidual(c, t.active, t.n, x, scale, f, v);
                         c.n = keep;
                     }
                     finished = __ballot_sync(group, !whole) != 0;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) f[i] = __shfl_sync(group, f[i], owner);
+                    converged = within();
                 }
             } else {
                 k += width;
