@@ -201,7 +201,10 @@ int reactive_transport_capillary_resident_commit_v1(void* transport, ReactiveThe
  * src/reactiveTransport/reactiveTransport.cpp:1773-1789, which round-trips q
  * through the host between RK stages). Conserved arrays are SoA,
  * q[k*(cells+fixed)+c], with the fixed-state tail filled by
- * reactive_transport_fill_fixed_v3. */
+ * reactive_transport_fill_fixed_v3. The entries that compute share the handle's work
+ * arrays: order them, host and device entries alike, so that one is in flight at a
+ * time. upload_conserved, download_conserved and replace_stage_state_v1, which only
+ * move the handle's own conserved variables, may run beside a device entry. */
 int reactive_transport_layout_v3(void* transport, size_t* cells, size_t* fixed, size_t* variables,
     size_t* species);
 int reactive_transport_fill_fixed_v3(void* transport, double* q, ReactiveTransportState* state, void* stream);

@@ -43,7 +43,7 @@ struct CartView {
     struct Inputs {
         double *u[3], *p, *T, *rho, *c, *irho, *ircv;
     } in;
-    ReactiveTransportPrimitive* primitive;  // cells + fixed
+    ReactiveTransportPrimitive* primitive;  // the fixed states' from entry `cells` on (the cells' hold `in`)
     double viscosity, conductivity, waveFactor;
     bool wale;
     double cw;
@@ -97,7 +97,8 @@ template <int NS, class R, bool SGS = false> __device__ __forceinline__ CellT<R>
 }
 
 // The cells' flux inputs (CartView::Inputs) from the conserved rows and the
-// states, with fromPrimitive the velocities from the caller's primitives instead.
+// states; given: the velocities from the caller's cell primitives instead (the fixed
+// states' stay).
 // The stage kernels read a cell's inputs up to seven times: as SoA their loads
 // coalesce (the 56-byte states and 32-byte primitives cost a warp 70 and 16
 // wavefronts a cell where these cost two a field), and the two reciprocals
@@ -105,10 +106,11 @@ template <int NS, class R, bool SGS = false> __device__ __forceinline__ CellT<R>
 // cell).
 __global__ void __launch_bounds__(256) cartInputs(CartView v, const double* __restrict__ q,
                                                   const ReactiveTransportState* __restrict__ st, int ns,
-                                                  bool fromPrimitive) {
+                                                  const ReactiveTransportPrimitive* __restrict__ given) {
     for (size_t c = blockIdx.x * size_t(blockDim.x) + threadIdx.x; c < v.all; c += size_t(blockDim.x) * gridDim.x) {
+        if (given && c >= v.cells) continue;
         ReactiveTransportPrimitive p{};
-        if (fromPrimitive) p = v.primitive[c];
+        if (given) p = given[c];
         else {
             for (int k = 0; k < ns; ++k) p.rho += q[size_t(k) * v.all + c];
             for (int d = 0; d < 3; ++d) p.u[d] = q[size_t(ns + d) * v.all + c] / p.rho;

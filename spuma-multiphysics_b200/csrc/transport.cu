@@ -374,11 +374,11 @@ struct Transport {
         upload(stateDevice, states, cfg.cells);
         profile.stateUploadBytes += cfg.cells * sizeof(ReactiveTransportState);
         if (primitive) {
-            upload(v.primitive, primitive, cfg.cells);
+            upload(primitiveUpload(), primitive, cfg.cells);
             profile.primitiveUploadBytes += cfg.cells * sizeof(ReactiveTransportPrimitive);
         }
         check(cudaMemsetAsync(invalid, 0xff, 2 * sizeof(unsigned long long), stream), "memset");
-        validateUploads<<<gridFor(cfg.cells, 256), 256, 0, stream>>>(stateDevice, primitive ? v.primitive : nullptr,
+        validateUploads<<<gridFor(cfg.cells, 256), 256, 0, stream>>>(stateDevice, primitive ? primitiveUpload() : nullptr,
                                                                     cfg.cells, invalid);
         launched();
         unsigned long long first[2];
@@ -398,14 +398,20 @@ struct Transport {
     // box the cells' flux inputs, on the face graph their primitives.
     void launchInputs(const double* qSoA, const ReactiveTransportState* state, cudaStream_t s) {
         if (structured) {
-            cartInputs<<<gridFor(v.all, 256), 256, 0, s>>>(boxView(), qSoA, state, int(cfg.species), false);
+            cartInputs<<<gridFor(v.all, 256), 256, 0, s>>>(boxView(), qSoA, state, int(cfg.species), nullptr);
             launched();
         } else launchPrimitives(qSoA, s);
     }
-    // The same for the caller's primitives (in v.primitive) and states (stateDevice).
+    // Where the caller's cell primitives are uploaded to: on the structured box their
+    // array holds the flux inputs, so they pass through the host bridge.
+    ReactiveTransportPrimitive* primitiveUpload() const {
+        return structured ? reinterpret_cast<ReactiveTransportPrimitive*>(staging) : v.primitive;
+    }
+    // The flux inputs from the caller's primitives and states (stateDevice).
     void launchInputsFromPrimitives() {
         if (!structured) return;
-        cartInputs<<<gridFor(v.all, 256), 256, 0, stream>>>(boxView(), nullptr, stateDevice, int(cfg.species), true);
+        cartInputs<<<gridFor(v.all, 256), 256, 0, stream>>>(boxView(), nullptr, stateDevice, int(cfg.species),
+                                                            primitiveUpload());
         launched();
     }
     void launchPrimitives(const double* qSoA, cudaStream_t s) {
@@ -580,15 +586,19 @@ struct Transport {
         box.boundaryBase = nInternal;
         box.nBoundary = bnd;
         box.primitive = primitive;
-        // the flux inputs live in buffers the structured path leaves idle while its
-        // kernels run: the host bridge (variables >= 5 per cell, packed before and
-        // unpacked after them on the same stream) and the face graph's face speeds
-        // (at least three faces a cell here) and cell steps
-        double* bridge = staging;
-        for (double** array : {&box.in.u[0], &box.in.u[1], &box.in.u[2], &box.in.p, &box.in.T}) {
-            *array = bridge;
-            bridge += cfg.cells;
+        // the flux inputs live in arrays of the face graph that only its kernels use:
+        // the cells' primitives (32 bytes each; the fixed states' stay), its carrier
+        // species (an int a face, at least three faces a cell here), face speeds and
+        // cell steps. Not in the host bridge: an entry that only moves conserved
+        // variables fills that on the handle's stream, whatever a device entry has in
+        // flight on the caller's.
+        static_assert(sizeof(ReactiveTransportPrimitive) == 4 * sizeof(double), "four arrays a cell");
+        double* idle = reinterpret_cast<double*>(primitive);
+        for (double** array : {&box.in.u[0], &box.in.u[1], &box.in.u[2], &box.in.p}) {
+            *array = idle;
+            idle += cfg.cells;
         }
+        box.in.T = reinterpret_cast<double*>(v.carrier);
         box.in.rho = v.faceSpeed;
         box.in.c = v.faceSpeed + cfg.cells;
         box.in.irho = v.faceSpeed + 2 * cfg.cells;
