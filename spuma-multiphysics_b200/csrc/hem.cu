@@ -1147,7 +1147,8 @@ struct HemDevice {
     ReactiveThermoState* dguess = nullptr;
     ReactiveThermoState* dout = nullptr;
     int* dsuccess = nullptr;
-    int passBlocks = 0, searchBlocks = 0;
+    int passBlocks = 0, searchBlocks = 0, restartBlocks = 0;
+    int passLimit = 1, searchLimit = 1;  // resident blocks a multiprocessor of passQueue and passSearch
     int domeBuilt = 0;  // grid points of the two-phase bound (0: none for this model)
     size_t bytes = 0;
     std::vector<void*> blocks;
@@ -1256,8 +1257,8 @@ struct HemDevice {
         selectCandidates<<<gridFor(count, 256), 256, 0, s>>>(cst, rec, count, selectList, state, transport, success,
                                                              fallback, counters);
         check(cudaGetLastError(), "selectCandidates");
-        passRestarts<<<passBlocks, kPassThreads, 0, s>>>(cst, in, fallback, seed, state, transport, success, counters,
-                                                         totals);
+        passRestarts<<<restartBlocks, kPassThreads, 0, s>>>(cst, in, fallback, seed, state, transport, success, counters,
+                                                            totals);
         check(cudaGetLastError(), "passRestarts");
     }
 };
@@ -1407,9 +1408,11 @@ void* create(const void* raw, size_t bytes, size_t capacity, bool hostPath, char
         int perSm = 0, sms = 0;
         check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, passQueue, kPassThreads, 0), "occupancy");
         check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d->device), "attribute");
-        d->passBlocks = std::max(1, perSm) * std::max(1, sms);
+        d->passLimit = std::max(1, perSm);
+        d->passBlocks = d->restartBlocks = d->passLimit * std::max(1, sms);
         check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, passSearch, kPassThreads, 0), "occupancy");
-        d->searchBlocks = std::max(1, perSm) * std::max(1, sms);
+        d->searchLimit = std::max(1, perSm);
+        d->searchBlocks = d->searchLimit * std::max(1, sms);
         const HemConst& h = d->hostConst;
         d->gasPass = GasPass{h.gas, h.Tmin, h.Tmax, h.pmin, h.pmax, h.vtol, h.etol, h.gasTmin, h.gasTmax,
                              h.liquidFloor, h.liquidTmin, h.liquidTc, h.enforceBounds, h.scalarRecovery};
@@ -1987,29 +1990,44 @@ int reactive_gpu_hem_autotune_v3(void* raw, const double* conserved, size_t stri
         rb200::require(count <= d.capacity, "CUDA HEM batch exceeds capacity");
         rb200::check(cudaSetDevice(d.device), "cudaSetDevice");
         auto s = static_cast<cudaStream_t>(stream);
-        int perSm = 0, sms = 0;
-        rb200::check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, rb200::passQueue, rb200::kPassThreads, 0),
-                     "occupancy");
+        int sms = 0;
         rb200::check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d.device), "attribute");
         d.ensureHostPath();  // scratch outputs of the timed runs
         cudaEvent_t a, b;
         rb200::check(cudaEventCreate(&a), "event");
         rb200::check(cudaEventCreate(&b), "event");
-        float best = 1e30f;
-        int keep = std::max(1, perSm);
-        for (int k = 1; k <= std::max(1, perSm); ++k) {
-            d.passBlocks = k * sms;
-            for (int r = 0; r < 2; ++r) {  // the first run warms up
+        // the launches that search this model's candidates: passSearch, the work queue, or
+        // (stableGasPrune) the queue and then passSearch; the restart search keeps its grid,
+        // since a batch to tune on seldom has cells that reach it
+        const bool fast = rb200::searchInRegisters(d.hostConst);
+        const int limit = fast && !d.hostConst.stableGasPrune ? d.searchLimit : std::max(d.passLimit, d.searchLimit);
+        auto use = [&](int k) {
+            d.passBlocks = std::min(k, d.passLimit) * std::max(1, sms);
+            d.searchBlocks = std::min(k, d.searchLimit) * std::max(1, sms);
+        };
+        auto fastest = [&](int k) {
+            use(k);
+            float best = 1e30f;
+            for (int r = 0; r < 4; ++r) {  // the first run warms up
                 rb200::check(cudaEventRecord(a, s), "event");
                 d.launchSearch(count, seed, d.dout, nullptr, d.dsuccess, s, conserved, stride);
                 rb200::check(cudaEventRecord(b, s), "event");
                 rb200::check(cudaEventSynchronize(b), "event");
+                float ms = 0;
+                rb200::check(cudaEventElapsedTime(&ms, a, b), "event");
+                if (r) best = std::min(best, ms);
             }
-            float ms = 0;
-            rb200::check(cudaEventElapsedTime(&ms, a, b), "event");
+            return best;
+        };
+        // fewer blocks than the limit only where they gain more than repeated runs of one
+        // shape differ (2%): a batch that leaves the search little to do says nothing about one that does not
+        int keep = limit;
+        float best = .98f * fastest(limit);
+        for (int k = limit - 1; k >= 1; --k) {
+            const float ms = fastest(k);
             if (ms < best) { best = ms; keep = k; }
         }
-        d.passBlocks = keep * sms;
+        use(keep);
         cudaEventDestroy(a);
         cudaEventDestroy(b);
         if (blocksPerSm) *blocksPerSm = keep;
