@@ -1004,12 +1004,12 @@ __device__ __noinline__ void runTasks(MixCell& c, const MixTerms& terms, bool re
                     bool whole = true;
                     if (int(lane) == owner) {
                         const Tally keep = c.n;
-                        whole = activeResidual(c, t.active, t.n, x, scale, f, v);
+                        whole = activeResidual(c, t.active, t.n, x, scale, fe, v);
                         c.n = keep;
                     }
                     finished = __ballot_sync(group, !whole) != 0;
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) f[i] = __shfl_sync(group, f[i], owner);
+                    for (int i = 0; i < 4; ++i) f[i] = __shfl_sync(group, fe[i], owner);
                     converged = within();
                 }
             } else {
