@@ -32,7 +32,7 @@ constexpr int kCartMaxNs = 4;
 struct CartView {
     int nx, ny, nz;
     size_t cells, fixed, all;
-    double area[3], dist[3], invDist[3];  // internal faces per axis (ownerWeight 0.5)
+    double area[3], invDist[3];   // internal faces per axis: area, 1/distance (ownerWeight 0.5)
     const double* invV;
     const ReactiveTransportFace* face;
     size_t sideBase[6];           // -x,+x,-y,+y,-z,+z: first face of the side block
@@ -634,7 +634,6 @@ __device__ __forceinline__ double cellStep(const CartView& v, size_t c, double d
 #endif
 template <int NS, class R, bool SGS = false>
 __global__ void __launch_bounds__(128, RB200_FACE_MINBLOCKS) cartFaceFluxes(CartView v, const double* __restrict__ q,
-                                                      const ReactiveTransportState* __restrict__ st,
                                                       const R* __restrict__ grad, const R* __restrict__ nut,
                                                       unsigned* error, bool cflPass) {
     constexpr int NQ = NS + 4;
@@ -923,7 +922,6 @@ template <int NS, bool SGS> struct TileLayout {
 // eddy viscosity, into shared-memory slot `slot`.
 template <int NS, class R, bool SGS>
 __device__ __forceinline__ void stageTileCell(const CartView& v, const double* __restrict__ q,
-                                              const ReactiveTransportState* __restrict__ st,
                                               const R* __restrict__ grad, const R* __restrict__ nut, size_t c,
                                               R* plane, int slot, bool viscous) {
     using Lay = TileLayout<NS, SGS>;
@@ -975,9 +973,8 @@ __device__ __forceinline__ void tileCell(const R* plane, int slot, CellT<R>& t, 
 // next plane, and the plane below a chunk's first).
 template <int NS, class R, bool SGS>
 __device__ __forceinline__ void globalCell(const CartView& v, const double* __restrict__ q,
-                                           const ReactiveTransportState* __restrict__ st, const R* __restrict__ grad,
-                                           const R* __restrict__ nut, size_t c, bool viscous, CellT<R>& t, R* g,
-                                           R& nu) {
+                                           const R* __restrict__ grad, const R* __restrict__ nut, size_t c,
+                                           bool viscous, CellT<R>& t, R* g, R& nu) {
     CellData d;
     loadCell<NS, SGS>(v, q, c, d, true);
     t = asCell<NS, R, SGS>(d);
@@ -1019,8 +1016,8 @@ __global__ void __launch_bounds__(kTileX * kTileY, RB200_TILE_MINBLOCKS) cartRat
     if (inside && z0 > 0 && z0 < z1 && (own(gx, gy, z0 - 1) || own(gx, gy, z0))) {
         CellT<R> lo, hi;
         R gl[9], gh[9], nl, nh;
-        globalCell<NS, R, SGS>(v, q, st, grad, nut, cellAt(gx, gy, z0 - 1), viscous, lo, gl, nl);
-        globalCell<NS, R, SGS>(v, q, st, grad, nut, cellAt(gx, gy, z0), viscous, hi, gh, nh);
+        globalCell<NS, R, SGS>(v, q, grad, nut, cellAt(gx, gy, z0 - 1), viscous, lo, gl, nl);
+        globalCell<NS, R, SGS>(v, q, grad, nut, cellAt(gx, gy, z0), viscous, hi, gh, nh);
         faceFluxCart<NS, R, SGS>(v, 2, 1.0, v.area[2], v.invDist[2], .5, 0, true, lo, hi, gl, gh, nl, nh, down, bad,
                                  faceBad);
     }
@@ -1028,7 +1025,7 @@ __global__ void __launch_bounds__(kTileX * kTileY, RB200_TILE_MINBLOCKS) cartRat
         __syncthreads();  // the previous plane's readers are done
         // stage the plane: the tile's own slots, then the halo ring
         if (inside)
-            stageTileCell<NS, R, SGS>(v, q, st, grad, nut, cellAt(gx, gy, z), plane, (ty + 1) * PX + tx + 1,
+            stageTileCell<NS, R, SGS>(v, q, grad, nut, cellAt(gx, gy, z), plane, (ty + 1) * PX + tx + 1,
                                       viscous);
         constexpr int ring = 2 * kTileX + 2 * kTileY;
         for (int h = tid; h < ring; h += kTileX * kTileY) {
@@ -1039,7 +1036,7 @@ __global__ void __launch_bounds__(kTileX * kTileY, RB200_TILE_MINBLOCKS) cartRat
             else { lx = kTileX; ly = h - 2 * kTileX - kTileY; }
             const int x = x0 + lx, y = y0 + ly;
             if (x >= 0 && y >= 0 && x < v.nx && y < v.ny)
-                stageTileCell<NS, R, SGS>(v, q, st, grad, nut, cellAt(x, y, z), plane, (ly + 1) * PX + lx + 1,
+                stageTileCell<NS, R, SGS>(v, q, grad, nut, cellAt(x, y, z), plane, (ly + 1) * PX + lx + 1,
                                           viscous);
         }
         __syncthreads();
@@ -1078,7 +1075,7 @@ __global__ void __launch_bounds__(kTileX * kTileY, RB200_TILE_MINBLOCKS) cartRat
             CellT<R> lo, hi;
             R gl[9], gh[9], nl, nh;
             tileCell<NS, R, SGS>(plane, slot, lo, gl, nl);
-            globalCell<NS, R, SGS>(v, q, st, grad, nut, cellAt(gx, gy, z + 1), viscous, hi, gh, nh);
+            globalCell<NS, R, SGS>(v, q, grad, nut, cellAt(gx, gy, z + 1), viscous, hi, gh, nh);
             faceFluxCart<NS, R, SGS>(v, 2, 1.0, v.area[2], v.invDist[2], .5, 0, true, lo, hi, gl, gh, nl, nh, up, bad,
                                      faceBad);
         }

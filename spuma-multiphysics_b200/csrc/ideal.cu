@@ -239,6 +239,7 @@ std::string speciesFromTable(const ReactiveB200Species& s, PureSpecies& sp) {
             if (!std::isfinite(g.coefficient[j])) return "Invalid ideal-gas NASA coefficient";
         sp.polynomial[r] = g.polynomial;
         sp.regionMin[r] = g.minimumTemperature;
+        for (int j = 0; j < 9; ++j) sp.coeff[r][j] = g.coefficient[j];
         sp.powers[r] = nasaPowers(g.polynomial, g.coefficient);
     }
     sp.regionMaxLast = s.regions[s.regionCount - 1].maximumTemperature;

@@ -577,7 +577,6 @@ struct Transport {
         box.cells = cfg.cells; box.fixed = cfg.fixed; box.all = cfg.cells + cfg.fixed;
         for (int a = 0; a < 3; ++a) {
             box.area[a] = area[a];
-            box.dist[a] = dist[a];
             box.invDist[a] = 1 / dist[a];
         }
         box.invV = invDevice;
@@ -670,8 +669,8 @@ struct Transport {
                           double maximumStep, double* result, cudaStream_t s) {
             const bool cflPass = cfl > 0;
             const unsigned grid = gridFor(b.cells, 128), cellGrid = gridFor(b.cells, 256);
-            if (b.sgs) cartFaceFluxes<NS, R, true><<<grid, 128, 0, s>>>(b, q, st, grad, nut, error, cflPass);
-            else cartFaceFluxes<NS, R><<<grid, 128, 0, s>>>(b, q, st, grad, nut, error, cflPass);
+            if (b.sgs) cartFaceFluxes<NS, R, true><<<grid, 128, 0, s>>>(b, q, grad, nut, error, cflPass);
+            else cartFaceFluxes<NS, R><<<grid, 128, 0, s>>>(b, q, grad, nut, error, cflPass);
             cartRatesFromFaces<NS, R><<<cellGrid, 256, 0, s>>>(b, q, out, stride, mode, dt, cfl, maximumStep);
             const bool shell = b.nx >= 3 && b.ny >= 3 && b.nz >= 3;
             const size_t sides = shell ? 2 * size_t(b.nx) * b.ny
