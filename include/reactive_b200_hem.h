@@ -116,8 +116,9 @@ int reactive_gpu_hem_two_phase_bound_v3(void* hem, int request, int* active, cha
  * 5), adds to conservedBar (SoA, stride barStride) the adjoint of the
  * transport-state outputs {p, T, rho, cv, frozen sound, gas mass} given in
  * transportBar, by the implicit function theorem on the converged candidate's
- * residual (two-phase (ln p, ln T, beta) or a single-phase (ln p, ln T)
- * partition). Cells whose derivative could not be formed add nothing and
+ * residual: two-phase (ln p, ln T, beta); single-phase the energy at the cell's density,
+ * in T, with its derivatives written out (the (ln p, ln T) partition where that
+ * phase does not exist at (T, rho)). Cells whose derivative could not be formed add nothing and
  * increment *failed (device counter, may be NULL). Asynchronous on `stream`. */
 int reactive_gpu_hem_vjp_device_v3(void* hem, const double* conserved, size_t stride, size_t count,
     size_t variables, const ReactiveThermoState* state, const ReactiveTransportState* transportBar,

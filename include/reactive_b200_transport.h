@@ -244,7 +244,7 @@ int reactive_transport_structured_v3(void* transport, int request, int* active);
  * (src/reactiveInterface/reactiveBalancedCapillary.h:55-142), falling back to
  * the HLL coefficients when the star speed leaves the wave fan. A face whose
  * HLLC state cannot be formed sets bit 1 of the status word. Selecting the face
- * graph returns to HLL; the rate VJP covers HLL only. *active (may be NULL)
+ * graph returns to HLL. *active (may be NULL)
  * receives the scheme. */
 int reactive_transport_flux_v3(void* transport, int request, int* active);
 /* Arithmetic of the structured path (no reference counterpart; the reference
@@ -282,8 +282,8 @@ int reactive_transport_owned_cells_v3(void* transport, uint64_t begin, uint64_t 
 int reactive_transport_rate_vjp_v3(void* transport, const double* q, const ReactiveTransportState* state,
     const double* w, double* qBar, ReactiveTransportState* stateBar, void* stream);
 /* Launch-shape autotuner of the structured path (no reference counterpart).
- * Times the candidates of the stage kernel (0: the shared-memory tiled form; or
- * the per-cell form with 64, 96 (the default), 128 threads a block), gradient
+ * Times the candidates of the stage kernel (0: the shared-memory tiled form; 1: the
+ * split stage, the default; or the per-cell form with 64, 96, 128 threads a block), gradient
  * (64, 128, 256) and CFL (64, 128, 256) kernels on this handle's problem (q and
  * state as stage_device_v3 takes them; neither is modified) and keeps the
  * fastest for later launches; results do not depend on the choice. Synchronous;

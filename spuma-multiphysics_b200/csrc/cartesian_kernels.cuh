@@ -5,20 +5,22 @@
 // normals +x, +y, +z; boundary faces on the six box sides), the operator is
 // evaluated by cell stencils instead of a face graph: no face-work array and no
 // CSR incidence are read. One kernel forms the Green-Gauss velocity gradient and
-// the WALE viscosity of a cell from its six neighbours; a second computes the six
-// face fluxes of a cell (HLL, viscous/WALE traction, conduction), sums them and
-// applies the SSPRK2 update, so the flux of an internal face is computed by both
-// of its cells instead of being stored and re-read. Boundary sides keep their own
+// the WALE viscosity of a cell from its six neighbours. The stage then either computes
+// the six face fluxes of a cell (HLL, viscous/WALE traction, conduction), sums them
+// and applies the SSPRK2 update (cartRates, cartRatesTile: the flux of an internal face
+// is computed by both of its cells), or (the default) in a pass over the faces and one
+// over the cells (cartFaceFluxes, cartRatesFromFaces). Boundary sides keep their own
 // face records (kind, fixed index, weight, distance, area); in the canonical
 // ordering the boundary faces of each box side form one contiguous block.
 //
 // The face physics is that of transport_kernels.cuh
 // (src/reactiveTransport/reactiveTransportKernels.h:290-560). With an
-// axis-aligned unit normal every projection reduces to one component; the
-// terms a face graph multiplies by a zero normal component are still formed
-// and added here (they are signed zeros for finite data), and a cell's faces are
-// summed in its face-graph incidence order, so for finite data both paths give
-// bitwise identical stage results.
+// axis-aligned unit normal every projection reduces to one component. The terms
+// a face graph multiplies by a zero normal component are signed zeros for finite
+// data: they are left out where the axis is known at compile time (faceFluxCart's
+// AXIS, cartGradients) and formed elsewhere. A cell's faces are summed in its
+// face-graph incidence order. So for finite data both paths give bitwise identical
+// stage results.
 #pragma once
 #include "transport_kernels.cuh"
 #include "dual.cuh"

@@ -2,17 +2,24 @@
 //
 // Launch sequence per batch (all on one stream, no host synchronisation, no
 // allocation; capturable in a CUDA graph):
-//   1 inputs     per cell: (rho, e, seed p/T/liquid mass); with the two-phase bound
-//                passGas also decides the cells that are plainly gas, and
-//                passSinglePhase the others outside the bound
-//   2 queue      persistent lane-level work queue over (candidate, cell) items:
-//                all seven candidates of every cell; with the model's
-//                stableGasPrune option, the all-gas/all-liquid items first, then
-//   3 compact    the cells the all-gas candidate does not decide, and
-//   4 queue      their five two-phase seeds
-//   5 select     first maximum entropy among stable candidates, in reference
+//   1 inputs     per cell: (rho, e, seed p/T/liquid mass). With the two-phase bound
+//                passGas forms them; it decides the cells that are plainly gas and
+//                lists the others: those inside the bound, and the general
+//                single-phase ones
+//   2 search     passSearch (one species' tables, analytic Jacobian), three loops over
+//                on-device counters: the listed single-phase cells; the all-gas and
+//                all-liquid candidates of the cells inside the bound (without it, of
+//                every cell) through the lane-level work queue; their five
+//                two-phase candidates in registers. Other models: passSinglePhase
+//                (with the bound) and passQueue, the work queue over all seven
+//                candidates
+//     prune      with the model's stableGasPrune option instead: passQueue over every
+//                cell's all-gas/all-liquid candidates, compactSeedCells (the cells
+//                that the all-gas one does not decide), then their five two-phase
+//                candidates by passSearch or passQueue
+//   3 select     first maximum entropy among stable candidates, in reference
 //                order; cells without one are queued for the restart search
-//   6 pass C     a warp per queued cell: 4 restart temperatures x 5 seeds on its
+//   4 restarts   a warp per queued cell: 4 restart temperatures x 5 seeds on its
 //                lanes, the first best written; cells still without one fail
 // Candidate records live in HBM (192 B each); every loop in the solvers is
 // bounded and no thread waits on another, so every launch terminates.
@@ -588,8 +595,8 @@ __device__ __forceinline__ bool gasCell(const GasPass& G, const HemConst& C, dou
 // First pass of a search with the two-phase bound: one thread per cell. A cell
 // outside the bound whose density also excludes the all-liquid partition has only
 // its all-gas candidate; where gasCell decides it, its outputs are written here.
-// Cells inside the bound are listed for the work queue, the others for the general
-// single-phase pass, with their inputs stored.
+// Cells inside the bound are listed for the candidate search, the others for the
+// general single-phase cells' part of it, with their inputs stored.
 //
 // Bound by FP64 latency and issue: the solve runs in registers (no stack: the
 // routines it shares with the general solvers are inlined, the species' constants
@@ -1204,7 +1211,7 @@ struct HemDevice {
         check(cudaMemsetAsync(counters, 0, NCOUNTERS * sizeof(unsigned), s), "memset counters");
         launchPlainFlash(cst, in, count, seed, state, transport, success, counters, totals, s);
     }
-    // Launches steps 2-6 for `count` prepared inputs, or, given the SoA conserved
+    // Launches steps 2-4 for `count` prepared inputs, or, given the SoA conserved
     // rows of a pure fluid (cons, stride), forms the inputs first: inside passGas
     // when the two-phase bound is on, else with inputsFromConserved.
     void launchSearch(size_t count, const ReactiveThermoState* seed, ReactiveThermoState* state,

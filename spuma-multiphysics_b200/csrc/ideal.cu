@@ -97,9 +97,14 @@ __device__ bool bracketedT(const IdealConst& G, const double* q, const double* q
 // are the steps the bracketed Newton takes. So the Newton runs first, and only a
 // step that left that bracket (or [Tmin, Tmax], or an iterate with cv <= 0)
 // goes back to the bracketed form. At the usual few per cent off the seed that
-// leaves four evaluations of seven to ten (64^3 two-species box: 24 us a call). The accepted iterate takes the Newton
-// step of the residual it was accepted with (within the tolerance, 4e-14 of T, no
-// further evaluation), so T is the solution to round-off and a smooth function of q.
+// leaves four evaluations of seven to ten (64^3 two-species box: 24 us a call).
+//
+// The accepted iterate takes the Newton step of the residual it was accepted with, at
+// no further evaluation. Acceptance is |F| <= .25 tol max(1e5 rho, rho cp T), so that step
+// is at most .25 tol max(1e5, cp T) / cv (at IdealGasBox's tol of 1e-13: 4e-14 of T where
+// cp T is above 1e5), and by the Newton's quadratic convergence it leaves an error of the
+// order of its own relative size squared: T is the solution to round-off, and a smooth
+// function of q, for tol below 1e-8, and better than tol for any.
 template <int NS>
 __global__ void __launch_bounds__(128) idealClosure(const IdealConst* __restrict__ Gp, const double* __restrict__ q,
                                                     size_t stride, size_t count, const double* Tseed, double* Tout,

@@ -772,7 +772,7 @@ struct Transport {
         }
     }
     // gradientsReady: the gradients and eddy viscosities of `state` (and the
-    // primitives of qIn) were formed by the preceding launches on this stream.
+    // flux inputs of qIn) were formed by the preceding launches on this stream.
     template <class R>
     void launchBoxStageT(const double* qIn, double* qOut, const ReactiveTransportState* state, double dt, int stage,
                          double* rate, R* grad, R* nut, cudaStream_t s, bool gradientsReady = false) {
