@@ -845,6 +845,82 @@ __global__ void selectCandidates(const HemConst* __restrict__ Cp, const CandReco
 // keeps its seed and fails. The solves of one cell are long serial Newton chains;
 // one thread running a temperature's five in turn had them five times as long (65,537
 // cells from fixed seeds: 62.0 -> 30.9 ms a batch).
+//
+// The lanes step through one flat loop, an evaluation a round each, that they leave
+// together (RestartSolve: twoPhaseSolve's iterates): calls of twoPhaseSolve side by side
+// part at its nested loops and run one lane after the other (60,000 cells of which
+// 17,000 have no answer: 36 to 38 ms so, 7.5 to 13.3 ms in the flat loop; a thread running
+// a temperature's five solves in turn took 12.5 to 26 ms).
+struct RestartSolve {
+    double x0, x1, x2, s0, s1, s2, scale, previous, fraction;
+    int it, k;
+    bool first;
+};
+__device__ __forceinline__ void restartStart(const HemConst& C, const CellInput& in, double seed, double restartT,
+                                             RestartSolve& s) {
+    s.scale = fmax(1e5 * in.q, fmax(fabs(in.e), in.q * 2000 * fmax(restartT, C.Tmin)));
+    s.x0 = log(clampd(in.gp, C.pmin, C.pmax));
+    s.x1 = log(clampd(restartT, C.Tmin, C.Tmax));
+    s.x2 = seed < 0 ? clampd(in.gml / in.q, 1e-8, 1 - 1e-8) : seed;
+    s.s0 = s.s1 = s.s2 = s.previous = 0;
+    s.fraction = 1;
+    s.it = s.k = 0;
+    s.first = true;
+}
+// The next fraction whose beta is in [0, 1) (a rejected one costs no evaluation), false past the last.
+__device__ __forceinline__ bool restartTrial(RestartSolve& s, Counts& n) {
+    for (; s.k < 30; ++s.k, s.fraction *= .5) {
+        const double beta = s.x2 + s.fraction * s.s2;
+        if (beta >= 0 && beta < 1) return true;
+        ++n.residuals;
+    }
+    return false;
+}
+// Takes the residuals f (ok) of the current trial, evaluated into v, and sets the next
+// trial (0), or ends the solve: converged with its sound speed (1) or failed (-1).
+__device__ __forceinline__ int restartAdvance(const HemConst& C, const CellInput& in, RestartSolve& s, bool ok, double f[3],
+                                              const Eval& v, CandidateOut& o, Counts& n) {
+    const double largest = fmax(fabs(f[0]), fmax(fabs(f[1]), fabs(f[2])));
+    if (s.first) {
+        if (!ok) return -1;
+        s.first = false;
+    } else {
+        if (!(ok && largest < s.previous * (1 - 1e-4 * s.fraction))) {
+            ++s.k;
+            s.fraction *= .5;
+            return restartTrial(s, n) ? 0 : -1;
+        }
+        s.x0 += s.fraction * s.s0;
+        s.x1 += s.fraction * s.s1;
+        s.x2 += s.fraction * s.s2;
+        if (++s.it >= 90) return -1;
+    }
+    const double x[3] = {s.x0, s.x1, s.x2};
+    double J[3][3];
+    const bool converged = fabs(f[0]) <= C.vtol && fabs(f[1]) <= C.etol && fabs(f[2]) <= C.mutol;
+    if (!jacobian(C, in, x, s.scale, f, v, J, n)) return -1;
+    double rhs[3] = {-f[0], -f[1], -f[2]}, step[3] = {0, 0, 0};
+    if (converged) {
+        rhs[0] = -1 / in.q;
+        rhs[1] = v.p / (in.q * s.scale);
+        rhs[2] = 0;
+    }
+    if (!solveSmall(J, rhs, 3, step)) return -1;
+    if (converged) {
+        const double squared = v.p * step[0];
+        if (!fin(squared) || squared <= 0) return -1;
+        o = CandidateOut{fabs(f[0]), fabs(f[1]), fabs(f[2]), sqrt(squared), s.it};
+        return o.soundEq <= v.soundFrozen * (1 + 2e-3) ? 1 : -1;
+    }
+    const double limiter = fmax(fmax(1., fmax(fabs(step[0]) / .7, fabs(step[1]) / .18)), fabs(step[2]) / .3);
+    s.s0 = step[0] / limiter;
+    s.s1 = step[1] / limiter;
+    s.s2 = step[2] / limiter;
+    s.previous = largest;
+    s.k = 0;
+    s.fraction = 1;
+    return restartTrial(s, n) ? 0 : -1;
+}
 __global__ void __launch_bounds__(kPassThreads, RB200_PASS_MINBLOCKS) passRestarts(const HemConst* __restrict__ Cp,
                                                              const CellInput* __restrict__ in,
                                                              const unsigned* __restrict__ fallback,
@@ -866,17 +942,35 @@ __global__ void __launch_bounds__(kPassThreads, RB200_PASS_MINBLOCKS) passRestar
         const CellInput x = in[c];
         Eval v;
         CandidateOut o{};
-        bool have = false;
+        RestartSolve s;
+        bool have = false, active = false;
         if (lane < solves) {
             if (x.skip & SKIP_TWO_PHASE) {  // no restart seed can converge either
                 ++n.candidates;
                 ++n.failures;
             } else if (upper > lower) {
-                have = twoPhaseSolve(C, x, kSeeds[lane % 5], lower + (upper - lower) * kRestart[lane / 5], v, o, n)
-                       && stableAt(C, x.q, v.liqMass, v.p, v.T, n);
-                if (have) ++n.stable; else ++n.failures;
+                ++n.candidates;
+                restartStart(C, x, kSeeds[lane % 5], lower + (upper - lower) * kRestart[lane / 5], s);
+                active = true;
             }
         }
+        const bool solved = active;
+        while (__any_sync(0xffffffffu, active)) {
+            double f[3] = {0, 0, 0};
+            bool ok = false;
+            if (active)
+                ok = twoPhaseResidual(C, x, s.x0 + s.fraction * s.s0, s.x1 + s.fraction * s.s1, s.x2 + s.fraction * s.s2,
+                                      s.scale, f, v, n);
+            __syncwarp();
+            if (active) {
+                const int code = restartAdvance(C, x, s, ok, f, v, o, n);
+                active = code == 0;
+                have = code > 0;
+            }
+            __syncwarp();
+        }
+        have = have && stableAt(C, x.q, v.liqMass, v.p, v.T, n);
+        if (have) ++n.stable; else if (solved) ++n.failures;
         __syncwarp();
         double best = have ? v.entropyD : -HUGE_VAL;
         for (int s = 16; s; s >>= 1) best = fmax(best, __shfl_xor_sync(0xffffffffu, best, s));
