@@ -561,7 +561,9 @@ __device__ __forceinline__ bool gasCell(const GasPass& G, const HemConst& C, dou
             if (!isfinite(F) || !isfinite(cv) || !(cv > 0)) return false;
         }
     }
-    if (gasRootIsV0(sp, d, g, clear) != 1 || !clear || !belowSaturation(C, g.p, T)) return false;
+    if (gasRootIsV0(sp, d, g, clear) != 1) return false;
+    // stable without a liquid: the liquid's range ends below T, or the saturation table says so
+    if (!(T >= G.liquidTc * (1 - 1e-10)) && (!clear || !belowSaturation(C, g.p, T))) return false;
     PhaseProps ph;
     ChemTerms chem;
     double sR;
@@ -594,7 +596,10 @@ __device__ __forceinline__ bool gasCell(const GasPass& G, const HemConst& C, dou
 
 // First pass of a search with the two-phase bound: one thread per cell. A cell
 // outside the bound whose density also excludes the all-liquid partition has only
-// its all-gas candidate; where gasCell decides it, its outputs are written here.
+// its all-gas candidate; where gasCell decides it, its outputs are written here. Gas
+// hotter than the liquid's range is decided too: left to the general pass after its
+// attempt here, 400,000 cells between 320 and 1,200 K took 370 us a batch, 330 before
+// this pass was split off, 120 so.
 // Cells inside the bound are listed for the candidate search, the others for the
 // general single-phase cells' part of it, with their inputs stored.
 //

@@ -8,7 +8,7 @@ import pytest
 from oracle import oracle
 from spuma_multiphysics_b200 import _abi as A, cases, thermo_data as td
 from spuma_multiphysics_b200.eos import PureFluid
-from spuma_multiphysics_b200.thermo_data import N2O
+from spuma_multiphysics_b200.thermo_data import N2O, N2O_FLASH
 import flash_cases as F
 from test_two_phase_bound_gpu import assert_same, both
 
@@ -42,6 +42,22 @@ def test_gas_cells_equal_the_queue_bitwise_and_the_oracle(shift):
     # both stop at an energy residual of 1e-9 of max(1e5 rho, rho cp T), which cp/cv < 1.5
     # here and the pressure's T-slope turn into less than 1e-8 of p and T
     assert s["p_rel"] <= 1e-8 and s["T_rel"] <= 1e-8, s
+
+
+# about the liquid range's end, above which no liquid is evaluated, and up to past the
+# critical pressure there
+@pytest.mark.parametrize("shift", [0.0, 4e-3, -4e-3])
+def test_cells_at_the_end_of_the_liquid_range(shift):
+    n, rng = 3000, np.random.default_rng(9)
+    end = N2O_FLASH["liquidTc"] * (1 - 1e-10)
+    step = np.resize([0.0, 1e-15, -1e-15, 1e-12, -1e-12, 1e-9, -1e-9, 1e-6, -1e-6, 1e-3, -1e-3, .1], n)
+    T, p = end * (1 + step), np.exp(rng.uniform(np.log(1e5), np.log(1.2e7), n))
+    props = PureFluid(N2O).tp(T, p, root="gas")
+    guess = np.zeros(n, dtype=A.THERMO_DTYPE)
+    guess["p"], guess["T"], guess["rho"] = p, T * (1 + shift), props["rho"]
+    on, off = both(np.ascontiguousarray(props["rho"]), np.ascontiguousarray(props["rho"] * props["e"]), guess)
+    assert_same(on, off)
+    assert on[2].mean() > .9
 
 
 # one thread, a warp's edges, a block's edges, and a mix of gas, dome and liquid
