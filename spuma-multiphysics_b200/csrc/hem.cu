@@ -700,18 +700,19 @@ __global__ void __launch_bounds__(kGasThreads, 6) passGas(
 // cell solves them through the same out-of-line solvers the work queue's state
 // machines restate (bit for bit the queue's candidates), selects as
 // selectCandidates does (the stable candidate of larger entropy, the all-gas one
-// on a tie) and writes the outputs; a cell with neither goes to the restart list.
+// on a tie) and writes the outputs. A cell with neither fails here: the restarts are
+// two-phase too (through the restart list, a warp a cell, 84,000 such cells of 400,000
+// took 198 us; their writes here take 60).
 __device__ __forceinline__ void singlePhaseLoop(const HemConst& C, const CellInput* __restrict__ in,
-                                                const unsigned* __restrict__ general, ReactiveThermoState* state,
-                                                ReactiveTransportState* transport, int* success, unsigned* fallback,
-                                                unsigned* counters, Counts& n) {
+                                                const unsigned* __restrict__ general, const ReactiveThermoState* seed,
+                                                ReactiveThermoState* state, ReactiveTransportState* transport,
+                                                int* success, unsigned* counters, Counts& n) {
     const unsigned items = counters[GENERAL];
     for (size_t base = blockIdx.x * size_t(blockDim.x); base < items; base += size_t(blockDim.x) * gridDim.x) {
         const size_t item = base + threadIdx.x;
-        bool restart = false;
-        unsigned c = 0;
+        bool failed = false;
         if (item < items) {
-            c = general[item];
+            const unsigned c = general[item];
             const CellInput x = in[c];
             double bestEntropy = 0;
             bool have = false;
@@ -743,24 +744,26 @@ __device__ __forceinline__ void singlePhaseLoop(const HemConst& C, const CellInp
                     writeOutputs(st, c, state, transport);
                 }
             }
-            n.candidates += 5;  // the two-phase seeds, failed without their solves
-            n.failures += 5;
-            if (have) {
-                if (success) __stcs(success + c, 1);
-            } else restart = true;
+            failed = !have;
+            // the two-phase seeds, and the restarts' twenty, failed without their solves
+            n.candidates += failed ? 25 : 5;
+            n.failures += failed ? 25 : 5;
+            if (success) __stcs(success + c, have ? 1 : 0);
+            if (failed && seed) writeOutputs(seed[c], c, state, transport);
         }
-        appendTo(fallback, counters + FALLBACK, restart, c);
+        const unsigned losses = __ballot_sync(0xffffffffu, failed);
+        if (losses && (threadIdx.x & 31) == 0) atomicAdd(counters + FAILED, unsigned(__popc(losses)));
     }
 }
 __global__ void __launch_bounds__(kPassThreads, RB200_PASS_MINBLOCKS) passSinglePhase(const HemConst* __restrict__ Cp,
                                                                 const CellInput* __restrict__ in,
                                                                 const unsigned* __restrict__ general,
+                                                                const ReactiveThermoState* seed,
                                                                 ReactiveThermoState* state,
                                                                 ReactiveTransportState* transport, int* success,
-                                                                unsigned* fallback, unsigned* counters,
-                                                                unsigned long long* totals) {
+                                                                unsigned* counters, unsigned long long* totals) {
     Counts n;
-    singlePhaseLoop(*Cp, in, general, state, transport, success, fallback, counters, n);
+    singlePhaseLoop(*Cp, in, general, seed, state, transport, success, counters, n);
     flushCounts(n, totals);
 }
 
@@ -785,12 +788,12 @@ __global__ void __launch_bounds__(kPassThreads, 3) passSearch(const HemConst* __
                                                              const CellInput* __restrict__ in, size_t count,
                                                              const unsigned* __restrict__ list,
                                                              const unsigned* __restrict__ general, CandRecord* rec,
+                                                             const ReactiveThermoState* seed,
                                                              ReactiveThermoState* state,
                                                              ReactiveTransportState* transport, int* success,
-                                                             unsigned* fallback, unsigned* counters,
-                                                             unsigned long long* totals) {
+                                                             unsigned* counters, unsigned long long* totals) {
     Counts n;
-    if (parts & SEARCH_GENERAL) singlePhaseLoop(*Cp, in, general, state, transport, success, fallback, counters, n);
+    if (parts & SEARCH_GENERAL) singlePhaseLoop(*Cp, in, general, seed, state, transport, success, counters, n);
     __syncwarp();
     if (parts & SEARCH_ONE_PHASE) queueLoop(*Cp, in, count, list, 0, 2, rec, counters, Q_A, n);
     __syncwarp();
@@ -1324,7 +1327,7 @@ struct HemDevice {
         auto searchCandidates = [&](int parts, int kindBase, int kinds, const unsigned* cells) {
             if (parts)
                 passSearch<<<searchBlocks, kPassThreads, 0, s>>>(cst, hostConst.gas, parts, in, count, cells, general, rec,
-                                                                 state, transport, success, fallback, counters, totals);
+                                                                 seed, state, transport, success, counters, totals);
             else
                 passQueue<<<passBlocks, kPassThreads, 0, s>>>(cst, in, count, cells, kindBase, kinds, rec, counters,
                                                               kindBase ? Q_B : Q_A, totals);
@@ -1354,8 +1357,8 @@ struct HemDevice {
             check(cudaGetLastError(), "passGas");
             if (fast) searchCandidates(SEARCH_GENERAL | SEARCH_ONE_PHASE | SEARCH_TWO_PHASE, 0, 7, list);
             else {
-                passSinglePhase<<<passBlocks, kPassThreads, 0, s>>>(cst, in, general, state, transport, success,
-                                                                    fallback, counters, totals);
+                passSinglePhase<<<passBlocks, kPassThreads, 0, s>>>(cst, in, general, seed, state, transport, success,
+                                                                    counters, totals);
                 check(cudaGetLastError(), "passSinglePhase");
                 searchCandidates(0, 0, 7, list);
             }
@@ -2272,8 +2275,8 @@ extern "C" int reactive_gpu_hem_run_static_v3(const void* model, size_t modelByt
         const bool fast = searchInRegisters(hostConst);
         auto searchCandidates = [&](int parts, int kindBase, int kinds, const unsigned* cells) {
             if (parts)
-                passSearch<<<blocks, kPassThreads, 0, s>>>(cst, hostConst.gas, parts, in, count, cells, nullptr, rec, state,
-                                                           transport, success, fallback, counters, totals);
+                passSearch<<<blocks, kPassThreads, 0, s>>>(cst, hostConst.gas, parts, in, count, cells, nullptr, rec, seed,
+                                                           state, transport, success, counters, totals);
             else
                 passQueue<<<blocks, kPassThreads, 0, s>>>(cst, in, count, cells, kindBase, kinds, rec, counters,
                                                           kindBase ? Q_B : Q_A, totals);
